@@ -119,6 +119,7 @@ struct srs_sim {
   float2* d_adjp_bs = nullptr;  // plain engine: (bsl, sum a + kb) with the domain flags
   // total Ca (built on first use)
   MassArgs mass{};
+  int mass_blocks = 0;
   // adjoint work buffers, kept between calls (name -> allocation)
   std::vector<std::pair<void*, size_t>> adj_bufs;
 };
@@ -1862,6 +1863,92 @@ int srs_batch_run_simulation(srs_batch* b, srs_run_output* outs) {
 }
 
 
+}  // extern "C"
+
+namespace {
+
+int sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n;
+}
+
+// f(0) .. f(n - 1), dealt in turn to at most `most` host threads (the caller
+// among them).
+template <class F>
+void host_parallel(int n, int most, F&& f) {
+  const int nt = std::max(1, std::min({n, most, (int)std::thread::hardware_concurrency()}));
+  auto work = [&](int t) {
+    for (int i = t; i < n; i += nt) f(i);
+  };
+  std::vector<std::thread> pool;
+  for (int t = 1; t < nt; ++t) pool.emplace_back(work, t);
+  work(0);
+  for (auto& th : pool) th.join();
+}
+
+// The line scan's weights by sample on the device: the untiled form reads
+// them, and the adjoint's ticks (which upload them when they first run).
+int linescan_csr(srs_sim* s) {
+  LinescanArgs& a = s->ls;
+  if (a.ptr) return SRS_OK;
+  int32_t* dp;
+  SRS_TRY(dev_upload(s, (int32_t**)&a.col, s->ls_col_h.data(), s->ls_col_h.size()));
+  SRS_TRY(dev_upload(s, (double**)&a.w, s->ls_w_h.data(), s->ls_w_h.size()));
+  SRS_TRY(dev_upload(s, &dp, s->ls_ptr_h.data(), s->ls_ptr_h.size()));
+  a.ptr = dp;
+  return SRS_OK;
+}
+
+// The tiled form of the line scan's weights (LinescanArgs): for every group
+// of eight samples, by chunk of engine elements, the elements that any of
+// the eight weighs, with their eight weights and which of them count.
+int linescan_tiles(srs_sim* s, const std::vector<int32_t>& ptr, const std::vector<int32_t>& col,
+                   const std::vector<double>& w) {
+  LinescanArgs& a = s->ls;
+  a.tptr = nullptr;
+  const int ns = a.n_samples, groups = (ns + 7) / 8;
+  const int chunks = (a.n_state + LINESCAN_CHUNK - 1) / LINESCAN_CHUNK;
+  std::vector<int32_t> tptr;
+  std::vector<uint32_t> tent;
+  std::vector<double> tw;
+  tptr.reserve((size_t)groups * (chunks + 1));
+  std::vector<int32_t> at(a.n_state);  // entry of an element in this group
+  for (int g = 0; g < groups; ++g) {
+    const int i0 = 8 * g, i1 = std::min(ns, i0 + 8);
+    std::fill(at.begin(), at.end(), -1);
+    for (int q = ptr[i0]; q < ptr[i1]; ++q) at[col[q]] = 0;
+    for (int e = 0; e < a.n_state; ++e) {
+      if (e % LINESCAN_CHUNK == 0) tptr.push_back((int32_t)tent.size());
+      if (at[e] < 0) continue;
+      at[e] = (int32_t)tent.size();
+      tent.push_back((uint32_t)(e % LINESCAN_CHUNK));
+    }
+    tptr.push_back((int32_t)tent.size());
+    tw.resize(tent.size() * 8, 0.0);
+    for (int i = i0; i < i1; ++i)
+      for (int q = ptr[i]; q < ptr[i + 1]; ++q) {
+        const int32_t k = at[col[q]];
+        tw[(size_t)k * 8 + (i - i0)] = w[q];
+        tent[k] |= 1u << (24 + (i - i0));
+      }
+  }
+  a.n_chunk = chunks;
+  a.splits = linescan_splits(ns, a.n_state, s->R, sm_count());
+  int32_t* dp;
+  SRS_TRY(dev_upload(s, &dp, tptr.data(), tptr.size()));
+  SRS_TRY(dev_upload(s, (uint32_t**)&a.tent, tent.data(), tent.size()));
+  SRS_TRY(dev_upload(s, (double**)&a.tw, tw.data(), tw.size()));
+  SRS_TRY(dev_alloc(s, &a.part, (size_t)a.splits * s->R * ns));
+  a.tptr = dp;
+  return SRS_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
   if (!s || !d || d->res <= 0 || d->r_thresh <= 0) return fail(SRS_ERR_INPUT, "bad line-scan description");
   // linescan/main.cpp:160-190: line position and PSF widths by scan axis
@@ -1940,17 +2027,20 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
   s->ls_rest.assign(ns, 0.0);
   std::vector<double> S6;
   initial_states(m, s->p, &S6);
-  for (int i = 0; i < ns; ++i) {
+  // samples are independent: their rows are built by up to eight host threads
+  // and joined in order
+  std::vector<std::vector<int32_t>> cols(ns);
+  std::vector<std::vector<double>> ws(ns);
+  auto sample = [&](int i) {
     double c[3];
     center(i, c);
-    ptr[i] = (int32_t)col.size();
     double rest = 0.0;
     for (int j = 0; j < m.N; ++j) {
       double rx = cx[j] - c[0], ry = cy[j] - c[1], rz = cz[j] - c[2];
       if (rx * rx + ry * ry + rz * rz < d->r_thresh) {
         double wj = vol[j] * pdf(rx, ry, rz);
-        col.push_back(s->eng_of_ref[j]);
-        w.push_back(wj);
+        cols[i].push_back(s->eng_of_ref[j]);
+        ws[i].push_back(wj);
         rest += wj * S6[SP_DYE * (size_t)m.N + j];
       }
     }
@@ -1961,6 +2051,12 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
     }
     pad[i] = pd;
     s->ls_rest[i] = pd + rest;
+  };
+  host_parallel(ns, (size_t)ns * (m.N + px.size()) < 100000 ? 1 : 8, sample);
+  for (int i = 0; i < ns; ++i) {
+    ptr[i] = (int32_t)col.size();
+    col.insert(col.end(), cols[i].begin(), cols[i].end());
+    w.insert(w.end(), ws[i].begin(), ws[i].end());
   }
   ptr[ns] = (int32_t)col.size();
   s->ls_ptr_h = ptr;
@@ -1971,9 +2067,8 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
   LinescanArgs& a = s->ls;
   a.n_samples = ns;
   a.n_state = (int32_t)eng_count(s);
-  SRS_TRY(dev_upload(s, (int32_t**)&a.ptr, ptr.data(), ptr.size()));
-  SRS_TRY(dev_upload(s, (int32_t**)&a.col, col.data(), col.size()));
-  SRS_TRY(dev_upload(s, (double**)&a.w, w.data(), w.size()));
+  a.ptr = nullptr;  // uploaded by linescan_csr
+  a.tptr = nullptr;
   SRS_TRY(dev_upload(s, (double**)&a.pad, pad.data(), pad.size()));
   if (s->d.precision != SRS_FP64) {
     std::vector<double> rd(eng_count(s), 0.0);
@@ -1985,12 +2080,18 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
   }
   SRS_TRY(dev_alloc(s, &s->d_ls_out, (size_t)s->R * ns));
   a.out = s->d_ls_out;
+  if (s->R >= LINESCAN_TILE_R && (size_t)s->R * ns < (size_t)INT32_MAX) {
+    SRS_TRY(linescan_tiles(s, ptr, col, w));
+  } else {
+    a.tptr = nullptr;
+    SRS_TRY(linescan_csr(s));
+  }
   if (n_samples) *n_samples = ns;
   return SRS_OK;
 }
 
 int srs_linescan(srs_sim* s, double* out, double* rest) {
-  if (!s || !s->ls.ptr) return fail(SRS_ERR_STATE, "call srs_linescan_setup first");
+  if (!s || (!s->ls.ptr && !s->ls.tptr)) return fail(SRS_ERR_STATE, "call srs_linescan_setup first");
   LinescanArgs a = s->ls;
   if (s->d.precision == SRS_FP64) {
     a.S64 = s->d_S[0];
@@ -2000,7 +2101,7 @@ int srs_linescan(srs_sim* s, double* out, double* rest) {
     a.CMq = s->d_CMq;
   }
   if (launch_linescan(a, s->R, s->st)) return fail(SRS_ERR_CUDA, "line-scan launch failed");
-  s->launches++;
+  s->launches += a.tptr ? 2 : 1;
   if (out)
     SRS_CUDA(cudaMemcpyAsync(out, s->d_ls_out, sizeof(double) * s->R * a.n_samples,
                              cudaMemcpyDeviceToHost, s->st));
@@ -2336,9 +2437,10 @@ extern "C" {
 
 int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
   if (!s || !d || !out || !out->loss || !out->grad || !d->f0) return fail(SRS_ERR_INPUT, "null argument");
-  if (!s->ls.ptr) return fail(SRS_ERR_STATE, "call srs_linescan_setup first");
+  if (!s->ls.ptr && !s->ls.tptr) return fail(SRS_ERR_STATE, "call srs_linescan_setup first");
   AdjPlan pl;
   SRS_TRY(adjoint_plan(s, d, &pl));  // also checks the descriptor
+  SRS_TRY(linescan_csr(s));
   const bool plain = s->d.engine != SRS_ENGINE_RESIDENT;
   const int R = s->R, NR = s->NR, NL = s->NL, W = NR + 2 * NL + 1, te = d->tick_every;
   const size_t NE = eng_count(s);
@@ -2832,9 +2934,9 @@ int srs_adjoint_plan(srs_sim* s, const srs_adjoint_desc* d, int* segment_steps, 
 
 int srs_sim_total_ca(srs_sim* s, double* out) {
   if (!s || !out) return fail(SRS_ERR_INPUT, "null argument");
-  MassArgs& a = s->mass;
   const size_t NE = eng_count(s);
-  if (!a.v0) {
+  if (!s->mass.v0) {
+    MassArgs a{};  // kept when every buffer is there
     const double* Rr = s->p.reals;
     std::vector<double> v0(NE, 0.0), bhi(NE, 0.0), blo(NE, 0.0), rest4(4 * NE, 0.0), rimm(NE, 0.0);
     std::vector<uint8_t> jsr(NE, 0);
@@ -2863,9 +2965,12 @@ int srs_sim_total_ca(srs_sim* s, double* out) {
     SRS_TRY(dev_upload(s, (double**)&a.blo, blo.data(), blo.size()));
     SRS_TRY(dev_upload(s, (double**)&a.rest4, rest4.data(), rest4.size()));
     SRS_TRY(dev_upload(s, (double**)&a.rest_imm, rimm.data(), rimm.size()));
+    s->mass_blocks = total_ca_blocks(a.n_state, s->R, sm_count());
+    SRS_TRY(dev_alloc(s, &a.part, (size_t)2 * s->R * s->mass_blocks));
     SRS_TRY(dev_alloc(s, &a.out, (size_t)2 * s->R));
+    s->mass = a;
   }
-  MassArgs m = a;
+  MassArgs m = s->mass;
   if (s->d.precision == SRS_FP64) {
     m.S64 = s->d_S[0];
   } else {
@@ -2877,8 +2982,8 @@ int srs_sim_total_ca(srs_sim* s, double* out) {
     m.CIq = s->d_CIq;
   }
   SRS_CUDA(cudaStreamSynchronize(s->st));
-  if (launch_total_ca(m, s->R, s->st)) return fail(SRS_ERR_CUDA, "total-Ca launch failed");
-  s->launches++;
+  if (launch_total_ca(m, s->R, s->mass_blocks, s->st)) return fail(SRS_ERR_CUDA, "total-Ca launch failed");
+  s->launches += 2;
   SRS_CUDA(cudaMemcpyAsync(out, m.out, sizeof(double) * 2 * s->R, cudaMemcpyDeviceToHost, s->st));
   SRS_CUDA(cudaStreamSynchronize(s->st));
   return SRS_OK;
