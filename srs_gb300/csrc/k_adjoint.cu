@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int n_ch = rank == 0 ? n_ch0 : 0;  // channel elements: forward partition 0
   const size_t NE = (size_t)C * Pc;
-  const AdjRec* geo = a.geo + (size_t)rank * Pc;
+  const float4 *geo_a = a.geo_a + (size_t)rank * Pc, *geo_b = a.geo_b + (size_t)rank * Pc;
   const uint32_t mask = (1u << a.off_bits) - 1u;
   const uint32_t ch_mask = (1u << a.ch_off_bits) - 1u;  // channel codes: forward layout
   // element ranges of this CTA: forward partitions rank*msub .. + msub - 1,
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
       const double* coef = tick_coef(a, a.s0 + len, r);
       for_all([&](int i) {
         const float4 L = a.lam[roff + i];
-        const float4 gb = __ldg(reinterpret_cast<const float4*>(geo + i) + 1);
+        const float4 gb = __ldg(geo_b + i);
         const bool jsr = (__float_as_uint(gb.w) >> 31) != 0;
         const float c = (jsr ? k.c0j : k.c0) + xu[i].x;
         const float inj = tick_injection(a, coef, (int)(rank * Pc + i));
@@ -277,10 +277,9 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
       float cp;
     };
     auto preload = [&](int i, const StepPtr& sp, int t) {
-      const float4* gp = reinterpret_cast<const float4*>(geo + i);
       Pre q;
-      q.at = __ldg(gp);
-      q.gb = __ldg(gp + 1);
+      q.at = __ldg(geo_a + i);
+      q.gb = __ldg(geo_b + i);
       q.x = sp.tu[i];
       q.ig = sp.tig[i];
       q.cp = t > 1 ? sp.cprev[i].x : 0.0f;

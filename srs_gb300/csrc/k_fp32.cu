@@ -269,10 +269,10 @@ size_t resident_smem_bytes(int P, int NR, int NL, int n_chtet, int n_entries) {
   b += (size_t)(NR + 2 * NL + NR) * sizeof(int32_t);  // ryr, lcc, lccv, lattice counts
   b += (size_t)(2 * NR + 2 * NL) * sizeof(uint32_t);  // channel element offsets, LCC rest
   b = (b + 7) & ~(size_t)7;
-  b += (size_t)(NR + NL) * sizeof(double);
+  b += (size_t)(NR + NL) * (sizeof(double) + sizeof(float));
   b += (size_t)(n_chtet + 1) * sizeof(int32_t);
   b = (b + 15) & ~(size_t)15;
-  b += (size_t)n_entries * sizeof(ChanEntry32);
+  b += (size_t)n_entries * sizeof(float2);
   return b;
 }
 

@@ -24,6 +24,8 @@ namespace srs {
 //   aligned), then the channel block (used by rank 0).
 struct ResidentSmemTail {
   RealCtl ctl;
+  srs_gate_consts gc[2];  // of Protocol, by potential
+  int64_t next_ev;        // next step with protocol work
   uint32_t base[2][16];  // cluster addresses of buf[b] in CTA rank q
   int32_t bad;
   // Termination flag published by rank 0's warp 0 in step s into slot s & 3
@@ -55,6 +57,10 @@ struct ChanSmem {
   const uint32_t* js;   // [NR] RyR JSR element
   const uint32_t* lc;   // [NL] LCC element
   const float* lrest;   // [NL] resting Ca of the LCC element
+  int32_t *ryr, *lcc, *lccv, *nb;  // [NR], [NL], [NL], [NR]
+  double* res;                     // [NR + NL]
+  float* flux;                     // [NR + NL] flux of the coming step of every channel
+  const srs_gate_consts* gc;       // [2] gating constants by potential
 };
 
 struct ResidentCa {
@@ -79,66 +85,98 @@ struct ResidentCa {
   }
 };
 
-// Gating of every channel after time step ctl.step by one warp
-// (UpdateChannelGating, cpu/RunSimulation.cpp:656-674).  `src` holds the
-// state after that step; every channel element is local (partition 0).
 // Named barrier of the channel group (the first `n` threads of the CTA).
 __device__ __forceinline__ void group_sync(int n) {
   if (n > 32) asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
   else __syncwarp();
 }
 
-// Gating of every channel after time step ctl.step by the channel group of
-// partition 0 (UpdateChannelGating, cpu/RunSimulation.cpp:656-674): group
-// lane gl takes RyR gl, then LCC gl - NR, so with 64 lanes every channel of
-// a dyad is gated in one round.  `src` holds the state after that step;
-// every channel element is local (partition 0).
-static __device__ void resident_gate(const ResidentArgs& a, RealCtl& ctl, const float4* src,
-                              int32_t* s_ryr, int32_t* s_lcc, int32_t* s_lccv, double* s_res,
-                              int32_t* s_nb, const ChanSmem& cs, int gl, int ng) {
+// Flux of a channel in the next step from the state after this one
+// (UpdateRyRFlux / UpdateLCCFlux, cpu/RunSimulation.cpp:127-164).  Computed
+// once per channel by the lane that gates it: the channel elements then only
+// sum fluxes, where each used to look up the state and the Ca of each of its
+// channels in turn.
+__device__ __forceinline__ void resident_ryr_flux(const ResidentArgs& a, const ChanSmem& cs, int i,
+                                                  float us, float uj) {
+  cs.flux[i] = cs.ryr[i] ? a.k.jr_scale * ((a.k.dc0 + uj) - us) : 0.0f;
+}
+__device__ __forceinline__ void resident_lcc_flux(const ResidentArgs& a, const ChanSmem& cs, int i,
+                                                  int v, float u) {
+  const int st = cs.lcc[i];
+  const float c = cs.lrest[i] + u;
+  cs.flux[a.C.NR + i] =
+      (st == 6 || st == 12) && cs.lccv[i] == 2 ? a.k.lccA[v] * fmaf(c, a.k.lccE[v], -a.k.lccB) : 0.0f;
+}
+// Every channel, by one warp (after the protocol may have changed states).
+static __device__ void resident_fluxes(const ResidentArgs& a, const float4* src, const ChanSmem& cs,
+                                       int v, int lane) {
+  for (int i = lane; i < a.C.NR; i += 32) resident_ryr_flux(a, cs, i, src[cs.cl[i]].x, src[cs.js[i]].x);
+  for (int i = lane; i < a.C.NL; i += 32) resident_lcc_flux(a, cs, i, v, src[cs.lc[i]].x);
+}
+
+// Gating of every channel after time step `step` by the channel group of
+// partition 0 (UpdateChannelGating, cpu/RunSimulation.cpp:656-674), and the
+// fluxes of the next step.  `src` holds the state after the step; every
+// channel element is local (partition 0).  In a group of three warps the
+// last one takes the LCCs and the others the RyRs, so that neither kind waits
+// for the other's code.  hold: the RyR the next step's protocol holds open
+// (cpu/RunSimulation.cpp:540-542; -1: none).
+static __device__ void resident_gate(const ResidentArgs& a, const RealCtl& ctl, const float4* src,
+                                     const ChanSmem& cs, int64_t step, int hold, int gl, int ng) {
   const int NR = a.C.NR, NL = a.C.NL;
-  const srs_gate_consts* g = &a.P_.gc[ctl.vsel];
-  const bool coupled = g->ryr_astar_half != 0.0f;
+  const bool gating = !a.P_.nogating;
+  const int v = ctl.vsel;
+  const srs_gate_consts* g = cs.gc + v;
+  const bool coupled = gating && g->ryr_astar_half != 0.0f;
   if (coupled) {
     for (int i = gl; i < NR; i += ng) {
       int no = 0, nc = 0;
       for (int q = 0; q < 4; ++q) {
         int j = a.C.ryr_nb[4 * i + q];
         if (j >= 0) {
-          if (s_ryr[j]) ++no;
+          if (cs.ryr[j]) ++no;
           else ++nc;
         }
       }
-      s_nb[i] = no | (nc << 16);
+      cs.nb[i] = no | (nc << 16);
     }
     group_sync(ng);
   }
-  for (int q = gl; q < NR + NL; q += ng) {
-    if (q < NR) {
-      const int i = q;
-      int no = 0, nc = 0;
-      if (coupled) {
-        no = s_nb[i] & 0xffff;
-        nc = s_nb[i] >> 16;
+  const int nr = ng > 64 ? ng - 32 : ng, l0 = ng > 64 ? nr : 0;  // RyR threads, first LCC thread
+  if (gl < nr) {
+    for (int i = gl; i < NR; i += nr) {
+      const float us = src[cs.cl[i]].x, uj = src[cs.js[i]].x;
+      if (gating) {
+        int no = 0, nc = 0;
+        if (coupled) {
+          no = cs.nb[i] & 0xffff;
+          nc = cs.nb[i] >> 16;
+        }
+        double rr = cs.res[i];
+        const int open = srs_gate_ryr(g, cs.ryr[i], us + a.k.c0, uj + a.k.c0j, no, nc, &rr, ctl.seed,
+                                      (uint32_t)i, (uint64_t)step);
+        cs.ryr[i] = open || i == hold;
+        cs.res[i] = rr;
+      } else if (i == hold) {
+        cs.ryr[i] = 1;
       }
-      float ca_s = src[cs.cl[i]].x + a.k.c0;
-      float ca_j = src[cs.js[i]].x + a.k.c0j;
-      double rr = s_res[i];
-      s_ryr[i] = srs_gate_ryr(g, s_ryr[i], ca_s, ca_j, no, nc, &rr, ctl.seed, (uint32_t)i,
-                              (uint64_t)ctl.step);
-      s_res[i] = rr;
-    } else {
-      const int i = q - NR;
-      float ca_l = src[cs.lc[i]].x + cs.lrest[i];
-      double rr = s_res[NR + i];
-      int st = s_lcc[i], vs = s_lccv[i];
-      srs_gate_lcc(g, &st, &vs, ca_l, &rr, ctl.seed, (uint32_t)(NR + i), (uint64_t)ctl.step);
-      s_lcc[i] = st;
-      s_lccv[i] = vs;
-      s_res[NR + i] = rr;
+      resident_ryr_flux(a, cs, i, us, uj);
     }
   }
-  group_sync(ng);
+  if (gl >= l0) {
+    for (int i = gl - l0; i < NL; i += ng - l0) {
+      const float u = src[cs.lc[i]].x;
+      if (gating) {
+        double rr = cs.res[NR + i];
+        int st = cs.lcc[i], vs = cs.lccv[i];
+        srs_gate_lcc(g, &st, &vs, u + cs.lrest[i], &rr, ctl.seed, (uint32_t)(NR + i), (uint64_t)step);
+        cs.lcc[i] = st;
+        cs.lccv[i] = vs;
+        cs.res[NR + i] = rr;
+      }
+      resident_lcc_flux(a, cs, i, v, u);
+    }
+  }
 }
 
 // Protocol of step ctl.step (rank 0, warp 0; lane 0 does the work).
@@ -181,12 +219,14 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
   uint32_t* s_cjs = s_ccl + NR;
   uint32_t* s_clc = s_cjs + NR;
   float* s_lrest = reinterpret_cast<float*>(s_clc + NL);
-  const ChanSmem cs{s_ccl, s_cjs, s_clc, s_lrest};
   double* s_res = reinterpret_cast<double*>(
       (reinterpret_cast<uintptr_t>(s_lrest + NL) + 7) & ~(uintptr_t)7);
-  // channel-entry CSR of partition 0, staged once per launch
-  int32_t* s_cptr = reinterpret_cast<int32_t*>(s_res + NCH);
-  ChanEntry32* s_clist = reinterpret_cast<ChanEntry32*>(
+  float* s_flux = reinterpret_cast<float*>(s_res + NCH);
+  const ChanSmem cs{s_ccl, s_cjs, s_clc, s_lrest, s_ryr, s_lcc, s_lccv, s_nb, s_res, s_flux, tail->gc};
+  // channel-entry CSR of partition 0, staged once per launch: (channel's index
+  // in s_flux, +-1 / V0)
+  int32_t* s_cptr = reinterpret_cast<int32_t*>(s_flux + NCH);
+  float2* s_clist = reinterpret_cast<float2*>(
       (reinterpret_cast<uintptr_t>(s_cptr + a.n_chtet[0] + 1) + 15) & ~(uintptr_t)15);
 
   uint32_t rank = 0;
@@ -200,23 +240,26 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
   const int nthr = blockDim.x;
   const int n_loc = a.n_local[rank];
   const int n_ch = (rank == 0) ? a.n_chtet[0] : 0;  // channel elements: rank 0 only
-  // In partition 0 the channel group (the first ng threads: two warps when
-  // the CTA has at least four) owns the channel elements, gates the channels
-  // right after updating them and runs the protocol; the other warps share
-  // the rest.  Elsewhere every thread strides over the whole partition.
-  const int ng = nthr >= 128 ? 64 : 32;
+  // In partition 0 the channel group (the first resident_group threads) owns
+  // the channel elements, gates the channels right after updating them and runs
+  // the protocol; the other warps share the rest.  Elsewhere every thread
+  // strides over the whole partition.
+  const int ng = resident_group(nthr);
   const bool split = (rank == 0) && (n_ch > 0) && (nthr > ng);
   const bool chan_group = split && tid < ng;
   const bool chan_warp = (rank == 0) && (warp == 0);
   const int n_int = a.n_int[rank];  // interior elements follow the channel elements
-  const TetRec* geo = a.geo + (size_t)rank * P;
+  const float4 *geo_a = a.geo_a + (size_t)rank * P, *geo_b = a.geo_b + (size_t)rank * P;
   const uint32_t off_mask = (1u << a.off_bits) - 1u;
   const Consts32& k = a.k;
   const Protocol& P_ = a.P_;
   if (rank == 0) {
     const int nnz = a.ch_ptr[n_ch];
     for (int i = tid; i <= n_ch; i += nthr) s_cptr[i] = a.ch_ptr[i];
-    for (int i = tid; i < nnz; i += nthr) s_clist[i] = a.ch_list[i];
+    for (int i = tid; i < nnz; i += nthr) {
+      const ChanEntry32 e = a.ch_list[i];
+      s_clist[i] = make_float2(__int_as_float(e.kind < 2 ? e.ch : NR + e.ch), e.s);
+    }
     for (int i = tid; i < NR; i += nthr) {
       s_ccl[i] = a.ryr_cleft_code[i] & off_mask;
       s_cjs[i] = a.ryr_jsr_code[i] & off_mask;
@@ -233,6 +276,7 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
       tail->base[1][q] = (C > 1) ? map_rank(smem_addr(buf1), q) : smem_addr(buf1);
     }
   }
+  if (tid < 2) tail->gc[tid] = P_.gc[tid];
   if (tid == 0) tail->bad = 0;
   // address of rank 0's termination flags, as seen from this CTA
   uint32_t done_addr0 = smem_addr(&tail->done_flag[0]);
@@ -264,6 +308,7 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
       if (a.prestep_first && !tail->ctl.done)
         resident_prestep(a, tail->ctl, buf0, s_ryr, s_lcc, s_lccv, r, a.initial_row, lane, cs);
       if (lane == 0) tail->done_flag[3] = tail->ctl.done;
+      resident_fluxes(a, buf0, cs, tail->ctl.vsel, lane);
     }
     step_barrier<C>();
     const bool skip = ((C > 1) ? ld_dsmem_s32(done_addr0 + 12u) : tail->done_flag[3]) != 0;
@@ -283,7 +328,8 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
       // them otherwise.
       cl_arrive<C>();
       bool pending = true;
-      int64_t next_ev = 0;  // channel warp: next step with protocol work (0: the first)
+      int64_t next_ev = 0;  // channel group: next step with protocol work (0: the first)
+      const int64_t step0 = rank == 0 ? tail->ctl.step : 0;
       for (int s = 0; s < a.steps; ++s) {
         const float4* src = cur ? buf1 : buf0;
         float4* dst = cur ? buf0 : buf1;
@@ -301,7 +347,6 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
             if (lane == 0) rec[W - 1] = tail->ctl.vsel;
           }
         }
-        const int v = tail->ctl.vsel;
         // one range of elements of this partition; elements that carry
         // channels (head of partition 0) add the release flux of their
         // channels, computed from the state of this step
@@ -318,17 +363,15 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
           // geometry of the next element is loaded one iteration ahead
           float4 ga_n = make_float4(0, 0, 0, 0), gb_n = ga_n;
           if (first < hi) {
-            const float4* gp = reinterpret_cast<const float4*>(geo + first);
-            ga_n = __ldg(gp);
-            gb_n = __ldg(gp + 1);
+            ga_n = __ldg(geo_a + first);
+            gb_n = __ldg(geo_b + first);
           }
           int i = first;
           for (; i < hi; i += stride) {
             const float4 ga = ga_n, gb = gb_n;
             if (i + stride < hi) {
-              const float4* gp = reinterpret_cast<const float4*>(geo + i + stride);
-              ga_n = __ldg(gp);
-              gb_n = __ldg(gp + 1);
+              ga_n = __ldg(geo_a + i + stride);
+              gb_n = __ldg(geo_b + i + stride);
             }
             uint32_t w0 = __float_as_uint(gb.x), w1 = __float_as_uint(gb.y);
             uint32_t c0 = w0 & 0xffffu, c1 = w0 >> 16, c2 = w1 & 0xffffu, c3 = w1 >> 16;
@@ -336,19 +379,8 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
             float flux = 0.0f;
             if constexpr (decltype(chan)::value) {
               for (int q = s_cptr[i]; q < s_cptr[i + 1]; ++q) {
-                ChanEntry32 e = s_clist[q];
-                float J = 0.0f;
-                if (e.kind < 2) {
-                  if (s_ryr[e.ch]) {
-                    float us = src[s_ccl[e.ch]].x;
-                    float uj = src[s_cjs[e.ch]].x;
-                    J = k.jr_scale * ((k.dc0 + uj) - us);
-                  }
-                } else if ((s_lcc[e.ch] == 6 || s_lcc[e.ch] == 12) && s_lccv[e.ch] == 2) {
-                  float c = s_lrest[e.ch] + src[i].x;
-                  J = k.lccA[v] * fmaf(c, k.lccE[v], -k.lccB);
-                }
-                flux = fmaf(J, e.s, flux);
+                const float2 e = s_clist[q];
+                flux = fmaf(s_flux[__float_as_int(e.x)], e.y, flux);
               }
             }
             float4 n0, n1, n2, n3;
@@ -358,17 +390,18 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
               n2 = ld_smem_f4(bs[0] + c2 * 16u);
               n3 = ld_smem_f4(bs[0] + c3 * 16u);
             } else if constexpr (decltype(local)::value) {
-              n0 = ld_smem_f4(src_local + (c0 & off_mask) * 16u);
-              n1 = ld_smem_f4(src_local + (c1 & off_mask) * 16u);
-              n2 = ld_smem_f4(src_local + (c2 & off_mask) * 16u);
-              n3 = ld_smem_f4(src_local + (c3 & off_mask) * 16u);
+              // interior elements' codes carry no rank
+              n0 = ld_smem_f4(src_local + c0 * 16u);
+              n1 = ld_smem_f4(src_local + c1 * 16u);
+              n2 = ld_smem_f4(src_local + c2 * 16u);
+              n3 = ld_smem_f4(src_local + c3 * 16u);
             } else {
               n0 = ld_dsmem_f4(bs[c0 >> a.off_bits] + (c0 & off_mask) * 16u);
               n1 = ld_dsmem_f4(bs[c1 >> a.off_bits] + (c1 & off_mask) * 16u);
               n2 = ld_dsmem_f4(bs[c2 >> a.off_bits] + (c2 & off_mask) * 16u);
               n3 = ld_dsmem_f4(bs[c3 >> a.off_bits] + (c3 & off_mask) * 16u);
             }
-            float4 out, cm = comp_load4(cmq + i);
+            float4 out, cm = comp_load4_x2(cmq + i);
             float imo, ci = comp_load1(ciq[i]);
             if constexpr (TRAJ) {
               const size_t o = ((size_t)s * a.R + r) * ((size_t)C * P) + (size_t)rank * P + i;
@@ -384,7 +417,7 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
             }
             dst[i] = out;
             immb[i] = imo;
-            comp_store4(cmq + i, cm);
+            comp_store4_x2(cmq + i, cm);
             ciq[i] = comp_store1(ci);
           }
           idx = i - hi;
@@ -392,41 +425,41 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
         // channel elements, then gating of this step and the protocol of the
         // next, by warp 0 of partition 0 (split) or after the whole CTA
         auto channels = [&]() {
+          const int64_t step = step0 + s;
+          const bool held = P_.run_protocol && P_.init_ryr != -1 && step + 1 < P_.hold_end;
+          const int hold = held ? P_.init_ryr : -1;
+          const int gn = split ? ng : 32;  // threads that gate
+          if (split && !chan_group) return;
+          int idx = tid;
           if (split) {
-            if (chan_group) {
-              int idx = tid;
-              update(idx, 0, n_ch, ng, std::false_type{}, std::true_type{});
-              group_sync(ng);  // the group wrote the channel elements itself
-              if (!P_.nogating) resident_gate(a, tail->ctl, dst, s_ryr, s_lcc, s_lccv, s_res, s_nb, cs, tid, ng);
-            }
+            update(idx, 0, n_ch, ng, std::false_type{}, std::true_type{});
+            group_sync(ng);
           } else {
-            int idx = tid;
             update(idx, 0, n_ch, nthr, std::false_type{}, std::true_type{});
             __syncthreads();
-            if (chan_warp && !P_.nogating)
-              resident_gate(a, tail->ctl, dst, s_ryr, s_lcc, s_lccv, s_res, s_nb, cs, lane, 32);
+            if (!chan_warp) return;
           }
-          if (chan_warp) {
-            RealCtl& ctl = tail->ctl;
-            if (lane == 0) {
-              ctl.step += 1;
-              ctl.t += P_.dt;
-              // the RyR hold of this step's protocol (cpu/RunSimulation.cpp:540-542)
-              if (P_.run_protocol && P_.init_ryr != -1 && ctl.step < P_.hold_end) s_ryr[P_.init_ryr] = 1;
-            }
-            __syncwarp();
-            // the protocol runs only at the steps where it has work (the RyR
-            // hold is applied above)
-            if (ctl.step >= next_ev) {
+          RealCtl& ctl = tail->ctl;
+          if (tid == 0) ctl.t += P_.dt;
+          resident_gate(a, ctl, dst, cs, step, hold, tid, gn);
+          if (tid == 0) ctl.step = step + 1;
+          // the protocol runs only at the steps where it has work (the RyR
+          // hold is applied by the gating)
+          if (step + 1 >= next_ev) {
+            group_sync(gn);
+            if (chan_warp) {
               resident_prestep(a, ctl, dst, s_ryr, s_lcc, s_lccv, r, 0, lane, cs);
-              if (lane == 0) next_ev = protocol_next_event(P_, ctl, !P_.nogating);
-              next_ev = __shfl_sync(0xffffffffu, next_ev, 0);
+              if (lane == 0) tail->next_ev = protocol_next_event(P_, ctl, true);
+              __syncwarp();
+              resident_fluxes(a, dst, cs, ctl.vsel, lane);
             }
-            if (lane == 0) {
-              tail->done_flag[s & 3] = ctl.done;
-              // a speculating launch must not end a run before its last step
-              if (spec && ctl.done && s + 1 < a.steps) bad |= 2;
-            }
+            group_sync(gn);
+            next_ev = tail->next_ev;
+          }
+          if (tid == 0) {
+            tail->done_flag[s & 3] = ctl.done;
+            // a speculating launch must not end a run before its last step
+            if (spec && ctl.done && s + 1 < a.steps) bad |= 2;
           }
         };
         // termination decided at the end of step s - 1

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <functional>
 #include <chrono>
 #include <cmath>
@@ -56,6 +57,7 @@ struct srs_sim {
   std::vector<int> eng_of_ref, ref_of_eng;
   // FP32 rest values per engine element
   std::vector<double> rest_ca, rest_imm;
+  float bsl_min = 0, bsl_max = 0;  // range of the nonzero SL capacities x K_D
   RestValues rv;
   double vm = 0, nsr = 0;
   // channel state (device)
@@ -113,7 +115,7 @@ struct srs_sim {
   int32_t* d_wt_idx = nullptr;
   double* d_wt_w = nullptr;
   int adj_ls_version = -1;
-  AdjRec* d_adj_geo = nullptr;  // reverse-sweep records of the CTA grouping
+  const float4 *d_adj_geo_a = nullptr, *d_adj_geo_b = nullptr;  // reverse-sweep records of the CTA grouping
   int adj_geo_m = 0;
   float4* d_adjp_aT = nullptr;  // plain engine: transposed coefficients [N]
   float2* d_adjp_bs = nullptr;  // plain engine: (bsl, sum a + kb) with the domain flags
@@ -134,6 +136,27 @@ int dev_upload(srs_sim* s, T** dst, const T* src, size_t n) {
   s->allocs.push_back(p);
   if (n) SRS_CUDA(cudaMemcpy(p, src, n * sizeof(T), cudaMemcpyHostToDevice));
   *dst = (T*)p;
+  return SRS_OK;
+}
+// 32-byte records as their first halves, then their second halves.
+template <class Rec>
+std::vector<float4> record_halves(const std::vector<Rec>& rec) {
+  static_assert(sizeof(Rec) == 2 * sizeof(float4), "records of two vector loads");
+  std::vector<float4> h(2 * rec.size());
+  for (size_t i = 0; i < rec.size(); ++i) {
+    std::memcpy(&h[i], &rec[i], sizeof(float4));
+    std::memcpy(&h[rec.size() + i], reinterpret_cast<const char*>(&rec[i]) + sizeof(float4), sizeof(float4));
+  }
+  return h;
+}
+template <class Rec>
+int dev_upload_halves(srs_sim* s, const float4** a, const float4** b, const std::vector<Rec>& rec) {
+  const std::vector<float4> h = record_halves(rec);
+  float4* d;
+  int rc = dev_upload(s, &d, h.data(), h.size());
+  if (rc != SRS_OK) return rc;
+  *a = d;
+  *b = d + rec.size();
   return SRS_OK;
 }
 template <class T>
@@ -225,6 +248,25 @@ void fill_protocol_consts(srs_sim* s) {
   P.row_w = SRS_STATES_ROW_BASE + (P.ryr_out ? s->NR : 0);
 }
 
+// |Ca| (uM) below which both divisions of the FP32 element update are in the
+// range of div_in_range, or -1 where the parameters leave it open:
+//   SERCA: den = sd0 + sd1 Ki + sd2 Ki^2, num = -sn0 + sn1 Ki + 3.2e12 Ki^2,
+//   Ki = (c inv_kdi)^2; sd0 bounds den from below, sn0 keeps num off the
+//   smallest magnitudes (it vanishes only through cancellation, whose
+//   remainder is a multiple of about 2^-48 sn0);
+//   rapid buffer: den = (khi + c)^2 + bsl, its numerator is tested per element.
+// 2^14 uM is sixteen times the resting JSR Ca.
+float div_range_cmax(const Consts32& k, float bsl_min, float bsl_max) {
+  const float cmax = 16384.0f;
+  const double Ki = (double)cmax * k.inv_kdi * (double)cmax * k.inv_kdi, top = std::ldexp(1.0, 59);
+  const double den = k.sd0 + (double)k.sd1 * Ki + (double)k.sd2 * Ki * Ki;
+  const double num = std::fabs(k.sn0) + std::fabs((double)k.sn1) * Ki + 3.24873e12 * Ki * Ki;
+  const double kc = (double)k.khi + cmax;
+  const bool serca = k.sd0 >= 1e-3f && k.sd1 >= 0.0f && k.sd2 >= 0.0f && k.sn0 >= 1e-3f && den < top && num < top;
+  const bool sl = bsl_max == 0.0f || (bsl_min >= 1e-9f && k.khi >= 0.0f && kc * kc + bsl_max < top);
+  return serca && sl ? cmax : -1.0f;
+}
+
 Consts32 make_consts32(const srs_sim* s) {
   const double* R = s->p.reals;
   const RestValues& rv = s->rv;
@@ -265,6 +307,7 @@ Consts32 make_consts32(const srs_sim* s) {
     k.lccE[v] = (float)s->P.lccE[v];
   }
   k.lccB = (float)s->P.lccB;
+  k.div_cmax = div_range_cmax(k, s->bsl_min, s->bsl_max);
   return k;
 }
 
@@ -373,8 +416,14 @@ int setup_plain64(srs_sim* s) {
   return SRS_OK;
 }
 
+float bsl_of(const srs_sim* s, int j) {
+  const double* R = s->p.reals;
+  double bhi = s->m.TT[j] * R[R_B_TOT_SL_HI] / (s->m.V0[j] * (1e-15));
+  return (float)(bhi * R[R_K_D_SL_HI]);
+}
+
 // ---- FP32 engines: checks shared by both ------------------------------------
-int check_fp32_supported(const srs_sim* s, bool resident) {
+int check_fp32_supported(srs_sim* s, bool resident) {
   const Mesh& m = s->m;
   const Operator& op = s->op;
   if (s->p.reals[R_B_TOT_SL_LO] != 0.0)
@@ -385,6 +434,11 @@ int check_fp32_supported(const srs_sim* s, bool resident) {
                                     ": the FP32 engines need its cleft element in the cytosol and "
                                     "its JSR element in the JSR");
   for (int j = 0; j < m.N; ++j) {
+    const float bsl = bsl_of(s, j);
+    if (bsl != 0.0f) {
+      s->bsl_min = s->bsl_max == 0.0f ? bsl : std::min(s->bsl_min, bsl);
+      s->bsl_max = s->bsl_max == 0.0f ? bsl : std::max(s->bsl_max, bsl);
+    }
     for (int k = 0; k < 4; ++k) {
       int n = op.nij[4 * (size_t)j + k];
       if (op.aij[5 * (size_t)j + 1 + k] != 0 && m.domain[n] != m.domain[j])
@@ -409,12 +463,6 @@ void fp32_rest(srs_sim* s) {
     s->rest_ca[e] = jsr ? s->rv.ca0_jsr : s->rv.ca0;
     s->rest_imm[e] = jsr ? s->rv.csqn : (s->m.tropc[j] ? s->rv.trpn : 0.0);
   }
-}
-
-float bsl_of(const srs_sim* s, int j) {
-  const double* R = s->p.reals;
-  double bhi = s->m.TT[j] * R[R_B_TOT_SL_HI] / (s->m.V0[j] * (1e-15));
-  return (float)(bhi * R[R_K_D_SL_HI]);
 }
 
 int setup_plain32(srs_sim* s) {
@@ -479,15 +527,107 @@ int setup_plain32(srs_sim* s) {
   return SRS_OK;
 }
 
+// f(0) .. f(n - 1), dealt in turn to at most `most` host threads (the caller
+// among them).
+template <class F>
+void host_parallel(int n, int most, F&& f) {
+  const int nt = std::max(1, std::min({n, most, (int)std::thread::hardware_concurrency()}));
+  auto work = [&](int t) {
+    for (int i = t; i < n; i += nt) f(i);
+  };
+  std::vector<std::thread> pool;
+  for (int t = 1; t < nt; ++t) pool.emplace_back(work, t);
+  work(0);
+  for (auto& th : pool) th.join();
+}
+
 // ---- FP32 resident engine ----------------------------------------------------
+// Elements of partition 0 (the channels'): every element thread of the
+// cluster gets the same number, the channel group takes the channel elements.
+int partition0_size(int N, int n_ch, int C, int threads) {
+  if (C == 1) return N;
+  const int ng = resident_group(threads);
+  if (n_ch <= 0 || threads <= ng) return (int)((int64_t)N / C);
+  const double lam = (double)(N - n_ch) / ((double)C * threads - ng);
+  return std::min(N, std::max(n_ch, n_ch + (int)std::lround(lam * (threads - ng))));
+}
+
+// Order inside the groups of eight elements that a quarter of a warp reads
+// together.  A 16-byte shared-memory read serves eight lanes at a time, one
+// from each of the eight 16-byte banks, and an element's bank is its position
+// modulo eight: eight lanes reading their k-th neighbours conflict where two
+// of those share a bank.  Elements of a group trade places (own reads and
+// writes stay conflict-free) as long as that lowers the number of colliding
+// pairs over all gathers.  order: the partition's elements after the channel
+// elements; n_int: how many of them are interior (the two ranges stay apart);
+// bank0: bank of the first one; pos: their places in order; nbr(j, k): the
+// neighbour if it is among them, else -1.
+template <class Nbr>
+void spread_banks(int* order, int n, int n_int, int bank0, const std::vector<int>& pos, const Nbr& nbr) {
+  const int groups = (n + 7) / 8;
+  // reads of each gather (group * 4 + k) by bank, eight counts of eight bits
+  std::vector<uint64_t> cnt(4 * (size_t)groups, 0);
+  std::vector<std::array<int, 4>> ref(n);  // the gathers that read an element
+  std::vector<int> nref(n, 0), id(n);      // id: element (its place at the start) by position
+  auto shift = [&](int i) { return 8 * ((bank0 + i) & 7); };
+  for (int i = 0; i < n; ++i) {
+    id[i] = i;
+    for (int k = 0; k < 4; ++k) {
+      const int z = nbr(order[i], k);
+      if (z < 0) continue;
+      for (int l = 0; l < 4; ++l)
+        if (nbr(z, l) == order[i]) {
+          ref[i][nref[i]++] = (pos[z] / 8) * 4 + l;
+          break;
+        }
+    }
+    for (int q = 0; q < nref[i]; ++q) cnt[ref[i][q]] += 1ull << shift(i);
+  }
+  for (int sweep = 0; sweep < 3; ++sweep) {
+    int moved = 0;
+    for (int g = 0; g < groups; ++g) {
+      const int lo = 8 * g, m = std::min(n, lo + 8) - lo;
+      uint64_t sum[8];  // counts of an element's gathers together
+      auto total = [&](int x) {
+        const int e = id[lo + x];
+        sum[x] = 0;
+        for (int q = 0; q < nref[e]; ++q) sum[x] += cnt[ref[e][q]];
+      };
+      for (int x = 0; x < m; ++x) total(x);
+      auto at = [&](int x, int y) { return (int)(sum[x] >> shift(lo + y) & 0xff); };
+      for (int x = 0; x < m; ++x)
+        for (int y = x + 1; y < m; ++y) {
+          if ((lo + x < n_int) != (lo + y < n_int)) continue;
+          const int ex = id[lo + x], ey = id[lo + y];
+          // colliding pairs gained by x moving to y's bank and y to x's; a
+          // gather that reads both does not change (each counted one there)
+          int delta = at(x, y) - at(x, x) + nref[ex] + at(y, x) - at(y, y) + nref[ey];
+          if (delta >= 2 * std::min(nref[ex], nref[ey])) continue;
+          for (int q = 0; q < nref[ex]; ++q)
+            for (int p = 0; p < nref[ey]; ++p) delta -= ref[ex][q] == ref[ey][p] ? 2 : 0;
+          if (delta >= 0) continue;
+          const uint64_t bx = 1ull << shift(lo + x), by = 1ull << shift(lo + y);
+          for (int q = 0; q < nref[ex]; ++q) cnt[ref[ex][q]] += by - bx;
+          for (int q = 0; q < nref[ey]; ++q) cnt[ref[ey][q]] += bx - by;
+          std::swap(id[lo + x], id[lo + y]);
+          for (int z = 0; z < m; ++z) total(z);
+          ++moved;
+        }
+    }
+    if (!moved) break;
+  }
+  const std::vector<int> before(order, order + n);
+  for (int i = 0; i < n; ++i) order[i] = before[id[i]];
+}
+
 int resident_partition(srs_sim* s, int C, int threads) {
   // Order: the elements that carry channels, then breadth-first layers
   // outward from them over the diffusion faces (so partition 0 holds the
   // channels' neighbourhood and partitions are cut between layers); the
   // sequence is cut into C contiguous partitions that give every element
-  // thread the same number of elements (in partition 0 the channel group of
-  // 64 threads -- 32 in small CTAs -- takes the channel elements and the
-  // gating instead).  Inside each
+  // thread the same number of elements (in partition 0 the channel group,
+  // resident_group threads, takes the channel elements and the gating
+  // instead).  Inside each
   // partition: channel elements (partition 0 only), then interior elements
   // (every neighbour in the same partition), then boundary elements.
   const int N = s->N;
@@ -533,25 +673,16 @@ int resident_partition(srs_sim* s, int C, int threads) {
   s->part_nch.assign(C, 0);
   s->part_nint.assign(C, 0);
   int Pmax = 0;
-  {
-    const int ng = threads >= 128 ? 64 : 32;
-    const bool split = C > 1 && n_ch > 0 && threads > ng;
-    int len0 = (int)((int64_t)N / C);
-    if (split) {
-      const double lam = (double)(N - n_ch) / ((double)C * threads - ng);
-      len0 = std::min(N, std::max(n_ch, n_ch + (int)std::lround(lam * (threads - ng))));
-    }
-    if (C == 1) len0 = N;
-    s->part_start[0] = 0;
-    s->part_len[0] = len0;
-    for (int q = 1; q < C; ++q) {
-      const int b0 = len0 + (int)((int64_t)(N - len0) * (q - 1) / (C - 1));
-      const int e0 = len0 + (int)((int64_t)(N - len0) * q / (C - 1));
-      s->part_start[q] = b0;
-      s->part_len[q] = e0 - b0;
-    }
-    for (int q = 0; q < C; ++q) Pmax = std::max(Pmax, s->part_len[q]);
+  const int len0 = partition0_size(N, n_ch, C, threads);
+  s->part_start[0] = 0;
+  s->part_len[0] = len0;
+  for (int q = 1; q < C; ++q) {
+    const int b0 = len0 + (int)((int64_t)(N - len0) * (q - 1) / (C - 1));
+    const int e0 = len0 + (int)((int64_t)(N - len0) * q / (C - 1));
+    s->part_start[q] = b0;
+    s->part_len[q] = e0 - b0;
   }
+  for (int q = 0; q < C; ++q) Pmax = std::max(Pmax, s->part_len[q]);
   if (n_ch > s->part_len[0])
     return fail(SRS_ERR_UNSUPPORTED, "channel elements do not fit in one partition");
   s->part_nch[0] = n_ch;
@@ -565,20 +696,41 @@ int resident_partition(srs_sim* s, int C, int threads) {
     }
     return true;
   };
+  auto kind_of = [&](int j) {
+    return m.domain[j] == DOMAIN_JSR ? 0 : 1 + (m.tropc[j] ? 1 : 0) + (m.TT[j] != 0.0 ? 2 : 0);
+  };
   s->ch_interior = 1;
   for (int i = 0; i < n_ch; ++i) s->ch_interior &= interior(seq[i]) ? 1 : 0;
-  std::vector<int> order;
+  std::vector<int> order, range[10];
   order.reserve(N);
   for (int q = 0; q < C; ++q) {
     const int b0 = s->part_start[q], e0 = b0 + s->part_len[q];
     const int c0 = q == 0 ? n_ch : 0;
     for (int i = b0; i < b0 + c0; ++i) order.push_back(seq[i]);
-    for (int i = b0 + c0; i < e0; ++i)
-      if (interior(seq[i])) order.push_back(seq[i]);
-    s->part_nint[q] = (int)order.size() - b0 - c0;
-    for (int i = b0 + c0; i < e0; ++i)
-      if (!interior(seq[i])) order.push_back(seq[i]);
+    // inside each range by kind (JSR; cytosol without and with troponin C;
+    // the same with SL buffer), so that few warps take more than one path
+    // through the element update (1024 dyads: 101.9 -> 100.4 us per step)
+    for (auto& r : range) r.clear();
+    for (int i = b0 + c0; i < e0; ++i) {
+      const int j = seq[i];
+      range[(interior(j) ? 0 : 5) + kind_of(j)].push_back(j);
+    }
+    for (int k = 0; k < 10; ++k) {
+      if (k == 5) s->part_nint[q] = (int)order.size() - b0 - c0;
+      order.insert(order.end(), range[k].begin(), range[k].end());
+    }
   }
+  std::vector<int> pos(N, -1);  // position in the element's own partition; -1: a channel element
+  for (int q = 0; q < C; ++q)
+    for (int i = s->part_nch[q]; i < s->part_len[q]; ++i) pos[order[s->part_start[q] + i]] = i - s->part_nch[q];
+  host_parallel(C, N < 3000 ? 1 : 8, [&](int q) {
+    const int c0 = s->part_nch[q];
+    spread_banks(order.data() + s->part_start[q] + c0, s->part_len[q] - c0, s->part_nint[q], c0, pos,
+                 [&](int j, int k) {
+                   const int u = nbr(j, k);
+                   return u >= 0 && part_of[u] == q && pos[u] >= 0 ? u : -1;
+                 });
+  });
   int bits = 1;
   while ((1 << bits) < Pmax) ++bits;
   int rank_bits = 0;
@@ -652,6 +804,9 @@ int setup_resident(srs_sim* s, int C, int threads) {
       for (int k = 0; k < 4; ++k) {
         geo[e].a[k] = (float)aj[1 + k];
         geo[e].nb[k] = code_of(s, s->eng_of_ref[nj[k]]);
+        // the codes of interior elements are offsets in their own partition
+        const int q = e / s->P_stride, i = e % s->P_stride - s->part_nch[q];
+        if (i >= 0 && i < s->part_nint[q]) geo[e].nb[k] &= (uint16_t)((1u << s->off_bits) - 1u);
       }
       geo[e].bsl = bsl_of(s, j);
       geo[e].flags = (s->m.domain[j] == DOMAIN_JSR ? 1u : 0u) | (s->m.tropc[j] ? 2u : 0u) |
@@ -663,7 +818,7 @@ int setup_resident(srs_sim* s, int C, int threads) {
   a.R = s->R;
   a.P = s->P_stride;
   a.off_bits = s->off_bits;
-  SRS_TRY(dev_upload(s, (TetRec**)&a.geo, geo.data(), geo.size()));
+  SRS_TRY(dev_upload_halves(s, &a.geo_a, &a.geo_b, geo));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_local, s->part_len.data(), s->part_len.size()));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_chtet, s->part_nch.data(), s->part_nch.size()));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_int, s->part_nint.data(), s->part_nint.size()));
@@ -1874,20 +2029,6 @@ int sm_count() {
   return n;
 }
 
-// f(0) .. f(n - 1), dealt in turn to at most `most` host threads (the caller
-// among them).
-template <class F>
-void host_parallel(int n, int most, F&& f) {
-  const int nt = std::max(1, std::min({n, most, (int)std::thread::hardware_concurrency()}));
-  auto work = [&](int t) {
-    for (int i = t; i < n; i += nt) f(i);
-  };
-  std::vector<std::thread> pool;
-  for (int t = 1; t < nt; ++t) pool.emplace_back(work, t);
-  work(0);
-  for (auto& th : pool) th.join();
-}
-
 // The line scan's weights by sample on the device: the untiled form reads
 // them, and the adjoint's ticks (which upload them when they first run).
 int linescan_csr(srs_sim* s) {
@@ -2227,7 +2368,7 @@ struct StateSnap {
 // per-element array keeps its index).  The two domain flags ride in sign
 // bits: bsl and sa are never negative.
 int adjoint_geometry(srs_sim* s, int m, int bits) {
-  if (s->d_adj_geo && s->adj_geo_m == m) return SRS_OK;
+  if (s->d_adj_geo_a && s->adj_geo_m == m) return SRS_OK;
   const int Pf = s->P_stride, NE = (int)eng_count(s);
   auto mcode = [&](int e) -> uint16_t {
     const int q = e / Pf, off = e % Pf;
@@ -2258,10 +2399,11 @@ int adjoint_geometry(srs_sim* s, int m, int bits) {
     if (bsl < 0.0f || sa < 0.0f || std::signbit(bsl) || std::signbit(sa))
       return fail(SRS_ERR_MESH, "negative SL capacity or coupling coefficient");
   }
-  if (s->d_adj_geo) {
-    SRS_CUDA(cudaMemcpy(s->d_adj_geo, geo.data(), geo.size() * sizeof(AdjRec), cudaMemcpyHostToDevice));
+  if (s->d_adj_geo_a) {
+    const std::vector<float4> h = record_halves(geo);
+    SRS_CUDA(cudaMemcpy((void*)s->d_adj_geo_a, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
   } else {
-    SRS_TRY(dev_upload(s, &s->d_adj_geo, geo.data(), geo.size()));
+    SRS_TRY(dev_upload_halves(s, &s->d_adj_geo_a, &s->d_adj_geo_b, geo));
   }
   s->adj_geo_m = m;
   return SRS_OK;
@@ -2692,7 +2834,8 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
     aa.m_sub = best_m;
     aa.off_bits = best_bits;
     aa.ch_off_bits = s->off_bits;
-    aa.geo = s->d_adj_geo;
+    aa.geo_a = s->d_adj_geo_a;
+    aa.geo_b = s->d_adj_geo_b;
   }
   AdjPlainArgs pa{};
   if (plain) {

@@ -46,6 +46,9 @@ struct Consts32 {
   float jr_scale;
   float dc0;
   float lccA[2], lccE[2], lccB;
+  // |Ca| below which the divisions of the element update stay in the range of
+  // div_in_range (srs_fp32_update.cuh); negative: never
+  float div_cmax;
 };
 
 struct ChanEntry32 {
@@ -99,6 +102,9 @@ int plain32_kernels_per_step(const Plain32Args& a);
 int launch_plain32_step(const Plain32Args& a, cudaStream_t st);
 int launch_plain32_prestep(const Plain32Args& a, int write_initial_row, cudaStream_t st);
 
+// Element record of the resident engine.  On the device its two halves lie
+// apart (ResidentArgs geo_a, geo_b): a warp's 32 records are then two loads of
+// 512 consecutive bytes, eight shared-memory/L1 wavefronts instead of sixteen.
 struct __align__(16) TetRec {
   float a[4];
   uint16_t nb[4];
@@ -106,7 +112,8 @@ struct __align__(16) TetRec {
   uint32_t flags;
 };
 
-// Per-element record of the reverse sweep (32 bytes, two vector loads).
+// Per-element record of the reverse sweep (halves apart on the device, as
+// TetRec).
 struct __align__(16) AdjRec {
   float aT[4];     // coefficient of this element in each neighbour's row
   uint16_t nb[4];  // neighbour codes of the adjoint's CTA grouping
@@ -123,7 +130,8 @@ struct ResidentArgs {
   int32_t P;
   int32_t off_bits;
   int32_t steps;
-  const TetRec* geo;
+  const float4* geo_a;  // coefficients
+  const float4* geo_b;  // neighbour codes, bsl, flags
   int32_t prestep_first;  // run the protocol of the first step before it
   int32_t initial_row;    // ... and write the t = 0 states row
   const int32_t* n_local; // [C] elements in each partition
@@ -235,7 +243,8 @@ struct AdjArgs {
   int32_t ch_off_bits;     // off_bits of the forward layout (channel codes)
   int32_t n_steps;  // steps of the segment; the kernel runs t = n_steps .. 1
   int64_t s0;       // global index of the state the segment starts from
-  const AdjRec* geo;  // [C*P] per-element records of the CTA grouping
+  const float4* geo_a;  // [C*P] per-element records of the CTA grouping: coefficients
+  const float4* geo_b;  // ... neighbour codes, bsl, sa
   const int32_t* n_local;
   const int32_t* n_chtet;
   const int32_t* n_int;    // [C] interior elements after the channel elements
@@ -356,6 +365,14 @@ SRS_RESIDENT_DECLARE(6)
 SRS_RESIDENT_DECLARE(8)
 SRS_RESIDENT_DECLARE(16)
 #undef SRS_RESIDENT_DECLARE
+// Threads of partition 0 that own the channel elements and gate the channels:
+// three warps, the last one for the LCCs, where the step waits for the
+// channels (large CTAs: 3.81 -> 2.93 us per step of a 16-CTA cluster of 320
+// threads); two where the elements bound it and a third warp is missed there
+// (1024 realizations, 8 x 192 threads: 117 against 126 us).
+__host__ __device__ constexpr int resident_group(int threads) {
+  return threads >= 320 ? 96 : threads >= 128 ? 64 : 32;
+}
 int launch_resident(const ResidentArgs& a, int C, int n_clusters, int threads, size_t smem,
                     cudaStream_t st);
 int resident_max_clusters(int C, int threads, size_t smem);
