@@ -6,6 +6,8 @@
 #include <algorithm>
 #include <array>
 #include <functional>
+#include <map>
+#include <mutex>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -550,6 +552,85 @@ int partition0_size(int N, int n_ch, int C, int threads) {
   if (n_ch <= 0 || threads <= ng) return (int)((int64_t)N / C);
   const double lam = (double)(N - n_ch) / ((double)C * threads - ng);
   return std::min(N, std::max(n_ch, n_ch + (int)std::lround(lam * (threads - ng))));
+}
+
+// Co-resident clusters of C CTAs at one CTA per SM.  It depends on how the
+// device groups its SMs, so it is asked for once per device and size.
+int clusters_at_one_per_sm(int C, size_t optin) {
+  static std::mutex mtx;
+  static std::map<std::pair<int, int>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mtx);
+  auto it = known.find({dev, C});
+  if (it == known.end()) it = known.emplace(std::make_pair(dev, C), resident_max_clusters(C, 512, optin)).first;
+  return it->second;
+}
+
+// Cluster size and threads per CTA where the caller leaves them (0) open: the
+// candidate with the smallest estimated time of a step for all realizations,
+//   rounds * t,  rounds = realizations / co-resident clusters, rounded up,
+//   t = (t_lat^4 + t_thr^4)^(1/4) us,
+//   t_lat = 2.05 + 0.28 elements per thread + 6e-4 threads (the chain of one
+// step: barriers, gating, a thread's elements one after the other) and t_thr = 1.2e-3 elements per SM (what an SM issues and moves).
+// Fitted to steps of the 10,368-element dyad: 5 x 320, two CTAs per SM, 5.6 us;
+// 3 x 512, one, 5.3; 8 x 192, three, 5.1; 16 x 320 for two realizations 2.9.
+// The smallest cluster that fits, which this replaces, took 133 us per step of
+// 1024 realizations (3 x 512) against 100 (5 x 320), and two rounds of 36
+// clusters for 37 realizations.
+int choose_resident(const srs_sim* s, int C_in, int T_in, int* C_out, int* T_out) {
+  const Mesh& m = s->m;
+  std::vector<char> ch(s->N, 0);
+  for (int i = 0; i < m.NR; ++i) ch[m.ryr_ele[i]] = ch[m.ryr_jsr[i]] = 1;
+  for (int i = 0; i < m.NL; ++i) ch[m.lcc_ele[i]] = 1;
+  int n_ch = 0;
+  for (char c : ch) n_ch += c;
+  int dev = 0, n_sm = 0, optin = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  struct Candidate {
+    double cost;
+    int C, T;
+    size_t smem;
+  };
+  std::vector<Candidate> cand;
+  for (int C : {1, 2, 3, 4, 5, 6, 8, 16}) {
+    if (C_in > 0 && C != C_in) continue;
+    int one = 0;  // clusters at one CTA per SM
+    for (int T : {160, 192, 256, 320, 384, 512, 640}) {
+      if (T_in > 0) T = T_in;
+      const int len0 = partition0_size(s->N, n_ch, C, T);
+      int P = len0;
+      if (C > 1) P = std::max(P, (s->N - len0 + C - 2) / (C - 1));
+      P = (P + 3) & ~3;
+      const size_t smem = resident_smem_bytes(P, s->NR, s->NL, n_ch, 2 * s->NR + s->NL);
+      int bits = 1, rank_bits = 0;
+      while ((1 << bits) < P) ++bits;
+      while ((1 << rank_bits) < C) ++rank_bits;
+      if (smem <= (size_t)optin && n_ch <= len0 && bits + rank_bits <= 16) {
+        // 96 registers a thread: 20 warps per SM
+        const int k = std::max(1, std::min((int)(per_sm / (smem + 1024)), 20 / (T / 32)));
+        if (!one) one = std::max(1, clusters_at_one_per_sm(C, (size_t)optin));
+        const int ncl = std::min(one * k, s->R);
+        const int rounds = (s->R + ncl - 1) / ncl;
+        const double per = std::max(1.0, std::ceil((double)ncl * C / n_sm)) * P;  // elements per SM
+        const double lat = 2.05 + 0.28 * P / T + 6e-4 * T, thr = 1.2e-3 * per;
+        cand.push_back({rounds * std::sqrt(std::sqrt(lat * lat * lat * lat + thr * thr * thr * thr)), C, T, smem});
+      }
+      if (T_in > 0) break;
+    }
+  }
+  std::stable_sort(cand.begin(), cand.end(),
+                   [](const Candidate& x, const Candidate& y) { return x.cost < y.cost; });
+  for (const Candidate& c : cand)
+    if (resident_max_clusters(c.C, c.T, c.smem) > 0) {
+      *C_out = c.C;
+      *T_out = c.T;
+      return SRS_OK;
+    }
+  return fail(SRS_ERR_UNSUPPORTED, "mesh too large for the resident engine");
 }
 
 // Order inside the groups of eight elements that a quarter of a warp reads
@@ -1402,26 +1483,17 @@ int srs_sim_create(const srs_grid* g, const srs_params* ps, const srs_sim_desc* 
     if (d->precision == SRS_FP64) rc = setup_plain64(s);
     else if (d->engine == SRS_ENGINE_PLAIN) rc = setup_plain32(s);
     else {
-      // resident: smallest cluster whose partition fits in shared memory
-      int threads = d->threads_per_cta > 0 ? d->threads_per_cta : 512;
-      if (threads > SRS_RESIDENT_MAX_THREADS || threads % 32)
+      int C = d->cluster_size, threads = d->threads_per_cta;
+      if (threads > 0 && (threads > SRS_RESIDENT_MAX_THREADS || threads % 32))
         rc = fail(SRS_ERR_INPUT, "resident engine: threads_per_cta must be a multiple of 32, <= " +
                                      std::to_string(SRS_RESIDENT_MAX_THREADS));
-      int C = d->cluster_size;
-      if (C <= 0) {
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        for (int c : {1, 2, 3, 4, 5, 6, 8, 16}) {
-          int Pm = (s->N + c - 1) / c;
-          Pm = (Pm + 3) & ~3;
-          if (resident_smem_bytes(Pm, s->NR, s->NL, 2 * s->NR + s->NL, 2 * s->NR + s->NL) <=
-              (size_t)optin) {
-            C = c;
-            break;
-          }
+      if (!rc && (C <= 0 || threads <= 0)) {
+        rc = choose_resident(s, C, threads, &C, &threads);
+        if (rc && d->cluster_size > 0) {  // setup_resident says what is wrong with it
+          rc = SRS_OK;
+          C = d->cluster_size;
+          threads = 512;
         }
-        if (C <= 0) rc = fail(SRS_ERR_UNSUPPORTED, "mesh too large for the resident engine");
       }
       if (!rc) rc = setup_resident(s, C, threads);
     }
