@@ -149,6 +149,7 @@ extern "C" int srs_explicit_step_fp64_noalloc(const srs_noalloc_step* d) {
   a.S_out = d->states_out;
   for (int q = 0; q < 56; ++q) a.p[q] = d->reals[q];
   a.nsr = d->ca_nsr;
+  plain64_consts(&a);
   Protocol& P = a.P;
   gate_consts(ps, d->v_m, &P.gc[0]);
   P.gc[1] = P.gc[0];

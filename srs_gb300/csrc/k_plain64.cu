@@ -12,7 +12,10 @@
 // compiled with -fmad=false, so with identical inputs the result matches the
 // reference's FP64 step bit for bit.  This engine is the FP64 oracle run of
 // the GPU path; the FP32 engines are measured against it.
+#include <cmath>
+
 #include "srs_engine.h"
+#include "srs_plain64_update.cuh"
 #include "srs_protocol.cuh"
 
 namespace srs {
@@ -44,52 +47,39 @@ __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
     double a3 = a.aij[5 * j + 3], a4 = a.aij[5 * j + 4];
     int n1 = a.nij[4 * j], n2 = a.nij[4 * j + 1], n3 = a.nij[4 * j + 2], n4 = a.nij[4 * j + 3];
     // UpdateReactionTerms (cpu/RunSimulation.cpp:25-125)
-    double b_ca = p[5] * (c_ca * a0 + Sca[n1] * a1 + Sca[n2] * a2 + Sca[n3] * a3 + Sca[n4] * a4) +
-                  a.br[0 * N + j];
-    double b_dye = p[11] * (Sdye[j] * a0 + Sdye[n1] * a1 + Sdye[n2] * a2 + Sdye[n3] * a3 +
-                            Sdye[n4] * a4) + a.br[3 * N + j];
-    double b_atp = p[7] * (Satp[j] * a0 + Satp[n1] * a1 + Satp[n2] * a2 + Satp[n3] * a3 +
-                           Satp[n4] * a4) + a.br[1 * N + j];
-    double b_cmdn = p[8] * (Scmdn[j] * a0 + Scmdn[n1] * a1 + Scmdn[n2] * a2 + Scmdn[n3] * a3 +
-                            Scmdn[n4] * a4) + a.br[2 * N + j];
-    double b_trpn = 0, b_csqn = 0;
+    const double ac[5] = {a0, a1, a2, a3, a4};
+    const double dye = Sdye[j], atp = Satp[j], cmdn = Scmdn[j];
+    double b_ca = diffuse64(p[5], c_ca, Sca[n1], Sca[n2], Sca[n3], Sca[n4], ac, a.br[0 * N + j]);
+    double b_dye = diffuse64(p[11], dye, Sdye[n1], Sdye[n2], Sdye[n3], Sdye[n4], ac, a.br[3 * N + j]);
+    double b_atp = diffuse64(p[7], atp, Satp[n1], Satp[n2], Satp[n3], Satp[n4], ac, a.br[1 * N + j]);
+    double b_cmdn = diffuse64(p[8], cmdn, Scmdn[n1], Scmdn[n2], Scmdn[n3], Scmdn[n4], ac, a.br[2 * N + j]);
     const int fl = a.flags[j];
-    double r_net, c_b;
+    const double dt = a.P.dt;
+    // the immobile buffers: a rate of zero leaves the value (-0 becomes +0)
+    double o_trpn = plus_zero(Strpn[j]), o_csqn = plus_zero(Scsqn[j]);
+    double r_net;
     if (!(fl & 1)) {
       if (fl & 2) {
-        c_b = Strpn[j];
-        r_net = p[26] * (p[24] - c_b) * c_ca - p[25] * c_b;
+        const double t = Strpn[j];
+        r_net = react64(p[26], p[24], p[25], t, c_ca);
         b_ca += -r_net;
-        b_trpn = r_net;
-        double K_i = c_ca / p[49];
-        K_i = K_i * K_i;
-        double K_sr = a.nsr / p[50];
-        K_sr = K_sr * K_sr;
-        double D_cycle = 0.104217 + 17.923 * K_sr + K_i * (1.75583e6 + K_sr * 7.61673e6) +
-                         K_i * K_i * (6.08463e11 + K_sr * 4.50544e11);
-        double v_cycle =
-            (K_i * K_i * 3.24873e12 + K_i * (9.17846e6 - 11478.2 * K_sr) - 0.329904 * K_sr) /
-            D_cycle;
-        double d_ca = (2e-3) * v_cycle * p[51];
-        b_ca -= d_ca;
+        o_trpn = t + r_net * dt;
+        b_ca -= serca64(a, c_ca);
       }
-      c_b = Sdye[j];
-      r_net = p[33] * (p[31] - c_b) * c_ca - p[32] * c_b;
+      r_net = react64(p[33], p[31], p[32], dye, c_ca);
       b_ca += -r_net;
       b_dye += r_net;
-      c_b = Satp[j];
-      r_net = p[20] * (p[18] - c_b) * c_ca - p[19] * c_b;
+      r_net = react64(p[20], p[18], p[19], atp, c_ca);
       b_ca += -r_net;
       b_atp += r_net;
-      c_b = Scmdn[j];
-      r_net = p[23] * (p[21] - c_b) * c_ca - p[22] * c_b;
+      r_net = react64(p[23], p[21], p[22], cmdn, c_ca);
       b_ca += -r_net;
       b_cmdn += r_net;
     } else {
-      c_b = Scsqn[j];
-      r_net = p[39] * (p[34] - c_b) * c_ca - p[40] * c_b;
+      const double q = Scsqn[j];
+      r_net = react64(p[39], p[34], p[40], q, c_ca);
       b_ca += -r_net;
-      b_csqn = r_net;
+      o_csqn = q + r_net * dt;
       b_ca += (a.nsr - c_ca) * p[36];
     }
     // Channel fluxes (UpdateRyRFlux / UpdateLCCFlux, :127-164), in order.
@@ -115,23 +105,17 @@ __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
         }
       }
     }
-    // UpdateFastBuffer (:15-22)
-    {
-      double khi = p[28], klo = p[30];
-      double B = 1 + (a.bhi[j] * khi / ((khi + c_ca) * (khi + c_ca))) +
-                 (a.blo[j] * klo / ((klo + c_ca) * (klo + c_ca)));
-      b_ca /= B;
-    }
+    b_ca = fast_buffer64(a, b_ca, c_ca, a.bhi[j], a.blo[j]);
     // Euler update (:640-644)
-    const double dt = a.P.dt;
     double* O = So;
-    O[0 * N + j] = c_ca + b_ca * dt;
-    O[1 * N + j] = Satp[j] + b_atp * dt;
-    O[2 * N + j] = Scmdn[j] + b_cmdn * dt;
-    O[3 * N + j] = Strpn[j] + b_trpn * dt;
-    O[4 * N + j] = Scsqn[j] + b_csqn * dt;
-    O[5 * N + j] = Sdye[j] + b_dye * dt;
-    if (!isfinite(O[j])) atomicOr(&ctlp->status, 1u);
+    const double ca_new = c_ca + b_ca * dt;
+    O[0 * N + j] = ca_new;
+    O[1 * N + j] = atp + b_atp * dt;
+    O[2 * N + j] = cmdn + b_cmdn * dt;
+    O[3 * N + j] = o_trpn;
+    O[4 * N + j] = o_csqn;
+    O[5 * N + j] = dye + b_dye * dt;
+    if (!finite64(ca_new)) atomicOr(&ctlp->status, 1u);
   }
   // ---- last block of this realization: gating + next step's protocol ----
   __shared__ int s_last;
@@ -186,6 +170,20 @@ __global__ void k_plain64_prestep(Plain64Args a, int write_initial_row) {
   if (write_initial_row && a.P.run_protocol) write_row(a.P, a.C, ctl, ryr, lcc, lccv, rows, ctl.t, ca);
   prestep(a.P, a.C, ctl, ryr, lcc, lccv, rows, ca);
   a.CS.ctl[r] = ctl;
+}
+
+// The element-independent terms of the SERCA flux in the reference's
+// operations (cpu/RunSimulation.cpp:83-91).
+void plain64_consts(Plain64Args* a) {
+  double K_sr = a->nsr / a->p[50];
+  K_sr = K_sr * K_sr;
+  a->sd0 = 0.104217 + 17.923 * K_sr;
+  a->sd1 = 1.75583e6 + K_sr * 7.61673e6;
+  a->sd2 = 6.08463e11 + K_sr * 4.50544e11;
+  a->sn1 = 9.17846e6 - 11478.2 * K_sr;
+  a->sn0 = 0.329904 * K_sr;
+  const double k = std::fabs(a->p[49]);
+  a->inv_kdi = k > 0x1p-500 && k < 0x1p500 ? 1.0 / a->p[49] : 0.0;
 }
 
 int launch_plain64_step(const Plain64Args& a, cudaStream_t st) {

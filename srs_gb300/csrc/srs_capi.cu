@@ -95,6 +95,8 @@ struct srs_sim {
   int64_t launches = 0;
   cudaGraphExec_t graph_plain = nullptr;
   int graph_plain_len = 0;
+  PlainLoop loop{};  // plain engines: steps in one launch (blocks 0: not used)
+  size_t loop_smem = 0;
   void* h_stage = nullptr;  // pinned host staging for state uploads
   size_t h_stage_bytes = 0;
   // the FP32 staging holds this many copies of one realization's state
@@ -422,6 +424,13 @@ float bsl_of(const srs_sim* s, int j) {
   const double* R = s->p.reals;
   double bhi = s->m.TT[j] * R[R_B_TOT_SL_HI] / (s->m.V0[j] * (1e-15));
   return (float)(bhi * R[R_K_D_SL_HI]);
+}
+
+int sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n;
 }
 
 // ---- FP32 engines: checks shared by both ------------------------------------
@@ -1113,6 +1122,8 @@ int normalize_buffers(srs_sim* s, const std::vector<int64_t>& steps_before) {
   std::vector<RealCtl> ctl(s->R);
   SRS_CUDA(cudaMemcpy(ctl.data(), s->d_ctl, sizeof(RealCtl) * s->R, cudaMemcpyDeviceToHost));
   const size_t N = s->N;
+  for (int r = 0; r < s->R; ++r)
+    if (ctl[r].status & 2u) return fail(SRS_ERR_TIMEOUT, "a step's barrier did not complete");
   for (int r = 0; r < s->R; ++r) {
     if (((ctl[r].step - steps_before[r]) & 1) == 0) continue;
     if (s->d.precision == SRS_FP64) {
@@ -1146,6 +1157,7 @@ void refresh_args(srs_sim* s) {
     s->a64.CS = cs;
     s->a64.counters = s->d_counters;
     s->a64.nsr = s->nsr;
+    plain64_consts(&s->a64);
   } else if (s->d.engine == SRS_ENGINE_PLAIN) {
     s->a32.P = s->P;
     s->a32.C = s->ch;
@@ -1216,8 +1228,87 @@ int plain_prestep(srs_sim* s, int write_initial_row) {
   return SRS_OK;
 }
 
-// n plain steps starting from buffer 0 (graph-replayed in pairs).
+// Whether the plain engine runs its steps in one launch (k_plain_loop.cu), and
+// the channels of its element blocks.  A fidelity run may end at any step of a
+// realization, which the looping kernels do not watch for; coupled RyRs are
+// gated from each other's states, which a block of its own elements lacks.
+int setup_plain_loop(srs_sim* s) {
+  if (s->p.ints[I_FLAG_FIDELITY_SIM] || s->p.reals[R_RYR_A_STAR] != 0.0 || s->N >= PLAIN32_SPLIT_N)
+    return SRS_OK;
+  const bool f64 = s->d.precision == SRS_FP64;
+  std::vector<int32_t> ptr, bptr, id, loc;
+  std::vector<ChanEntry> list;
+  chan_lists(s, &ptr, &list);
+  loc.resize(list.size());
+  int most = 0, blocks = 0, per = 1;
+  // as few elements a thread as fit
+  for (; per <= 4; per *= 2) {
+    const int tile = (f64 ? PLAIN_LOOP_TILE64 : PLAIN_LOOP_T32) * per;
+    blocks = (s->N + tile - 1) / tile;
+    bptr.assign(1, 0);
+    id.clear();
+    most = 0;
+    std::vector<int> at(s->NCH, -1);
+    for (int b = 0; b < blocks; ++b) {
+      const int q0 = ptr[b * tile], q1 = ptr[std::min(s->N, (b + 1) * tile)], i0 = (int)id.size();
+      for (int q = q0; q < q1; ++q) {
+        const int c = list[q].kind < 2 ? list[q].ch : s->NR + list[q].ch;
+        if (at[c] < i0) {
+          at[c] = (int)id.size();
+          id.push_back(c);
+        }
+        loc[q] = at[c] - i0;
+      }
+      bptr.push_back((int32_t)id.size());
+      most = std::max(most, (int)id.size() - i0);
+    }
+    s->loop_smem = plain_loop_smem_bytes(s->NR, s->NL, most);
+    if (s->loop_smem > 36 * 1024) return SRS_OK;  // thousands of channels
+    if (plain_loop_fits(f64, per, (int64_t)s->R * (blocks + 1), s->loop_smem)) break;
+  }
+  if (per > 4) return SRS_OK;
+  SRS_TRY(dev_alloc(s, &s->loop.bar, (size_t)s->R));
+  SRS_TRY(dev_upload(s, (int32_t**)&s->loop.ch_ptr, bptr.data(), bptr.size()));
+  SRS_TRY(dev_upload(s, (int32_t**)&s->loop.ch_id, id.data(), id.size()));
+  SRS_TRY(dev_upload(s, (int32_t**)&s->loop.loc, loc.data(), loc.size()));
+  s->loop.ch_max = most;
+  s->loop.per_thread = per;
+  s->loop.n_sm = sm_count();
+  s->loop.blocks = blocks;
+  return SRS_OK;
+}
+
+int plain_loop_launch(srs_sim* s, int steps) {
+  PlainLoop l = s->loop;
+  l.steps = steps;
+  SRS_CUDA(cudaMemsetAsync(l.bar, 0, sizeof(unsigned) * s->R, s->st));
+  int rc;
+  if (s->d.precision == SRS_FP64) {
+    Plain64Args a = s->a64;
+    a.S_in = s->d_S[0];
+    a.S_out = s->d_S[1];
+    rc = launch_plain64_loop(a, l, s->loop_smem, s->st);
+  } else {
+    Plain32Args a = s->a32;
+    a.M_in = s->d_M[0];
+    a.I_in = s->d_I[0];
+    a.M_out = s->d_M[1];
+    a.I_out = s->d_I[1];
+    rc = launch_plain32_loop(a, l, s->loop_smem, s->st);
+  }
+  s->launches++;
+  if (rc) return fail(SRS_ERR_CUDA, std::string("step loop launch: ") + cudaGetErrorString(cudaGetLastError()));
+  return SRS_OK;
+}
+
+// n plain steps starting from buffer 0: in launches of up to 4096 steps where
+// the problem fits on the device, else one launch per step (graph-replayed).
 int plain_steps(srs_sim* s, int64_t n) {
+  if (s->loop.blocks > 0) {
+    for (int64_t done = 0; done < n; done += 4096)
+      SRS_TRY(plain_loop_launch(s, (int)std::min<int64_t>(4096, n - done)));
+    return SRS_OK;
+  }
   const int G = 32;  // launches per graph replay (even)
   int64_t done = 0;
   if (n >= G) {
@@ -1480,9 +1571,10 @@ int srs_sim_create(const srs_grid* g, const srs_params* ps, const srs_sim_desc* 
   if (!rc) rc = alloc_channel_state(s);
   if (!rc) fill_protocol_consts(s);
   if (!rc) {
-    if (d->precision == SRS_FP64) rc = setup_plain64(s);
-    else if (d->engine == SRS_ENGINE_PLAIN) rc = setup_plain32(s);
-    else {
+    if (d->engine == SRS_ENGINE_PLAIN) {
+      rc = d->precision == SRS_FP64 ? setup_plain64(s) : setup_plain32(s);
+      if (!rc) rc = setup_plain_loop(s);
+    } else {
       int C = d->cluster_size, threads = d->threads_per_cta;
       if (threads > 0 && (threads > SRS_RESIDENT_MAX_THREADS || threads % 32))
         rc = fail(SRS_ERR_INPUT, "resident engine: threads_per_cta must be a multiple of 32, <= " +
@@ -1779,6 +1871,7 @@ int run_finish(srs_sim* s, srs_run_output* out, const std::vector<int64_t>& befo
   s->P.row_cap = 0;
   refresh_args(s);
   if (st_bits & 1) return fail(SRS_ERR_NONFINITE, "a realization produced a non-finite Ca value");
+  if (st_bits & 2) return fail(SRS_ERR_TIMEOUT, "a step's barrier did not complete");
   if (st_bits & 4) return fail(SRS_ERR_INPUT, "row_capacity too small for the run");
   if (st_bits & 8) return fail(SRS_ERR_STATE, "internal: termination inside a speculating launch");
   return SRS_OK;
@@ -2093,13 +2186,6 @@ int srs_batch_run_simulation(srs_batch* b, srs_run_output* outs) {
 }  // extern "C"
 
 namespace {
-
-int sm_count() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n;
-}
 
 // The line scan's weights by sample on the device: the untiled form reads
 // them, and the adjoint's ticks (which upload them when they first run).

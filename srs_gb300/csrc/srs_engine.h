@@ -24,11 +24,15 @@ struct Plain64Args {
   double* S_out;
   double p[56];
   double nsr;
+  // terms of the SERCA flux that do not depend on the element, and 1 / K_D_i
+  // (zero where its exponent is extreme), filled by plain64_consts
+  double sd0, sd1, sd2, sn1, sn0, inv_kdi;
   Protocol P;
   Channels C;
   ChanState CS;
   unsigned int* counters;
 };
+void plain64_consts(Plain64Args* a);
 int launch_plain64_step(const Plain64Args& a, cudaStream_t st);
 int launch_plain64_prestep(const Plain64Args& a, int write_initial_row, cudaStream_t st);
 
@@ -101,6 +105,27 @@ constexpr int PLAIN32_SPLIT_N = 65536;
 int plain32_kernels_per_step(const Plain32Args& a);
 int launch_plain32_step(const Plain32Args& a, cudaStream_t st);
 int launch_plain32_prestep(const Plain32Args& a, int write_initial_row, cudaStream_t st);
+
+// The plain engines' steps in one launch (k_plain_loop.cu).  S_in / M_in / I_in
+// are buffer 0 of the state, S_out / M_out / I_out buffer 1; after n steps the
+// state is in buffer n % 2.
+struct PlainLoop {
+  int32_t steps;
+  int32_t blocks;         // element blocks per realization
+  int32_t per_thread;     // elements a thread (FP64: a lane of each of four warps) takes
+  int32_t n_sm;
+  unsigned* bar;          // [R] arrivals at the step barriers, zero before the launch
+  int32_t ch_max;         // most channels an element block gates
+  const int32_t* ch_ptr;  // [blocks + 1] CSR of the channels each block gates
+  const int32_t* ch_id;   // RyR, or NR + LCC
+  const int32_t* loc;     // per entry of chan_list: the channel's place in its block's list
+};
+constexpr int PLAIN_LOOP_T32 = 128;
+constexpr int PLAIN_LOOP_TILE64 = 32;  // elements of an FP64 block
+size_t plain_loop_smem_bytes(int NR, int NL, int ch_max);
+bool plain_loop_fits(bool f64, int per_thread, int64_t blocks, size_t smem);
+int launch_plain32_loop(const Plain32Args& a, const PlainLoop& l, size_t smem, cudaStream_t st);
+int launch_plain64_loop(const Plain64Args& a, const PlainLoop& l, size_t smem, cudaStream_t st);
 
 // Element record of the resident engine.  On the device its two halves lie
 // apart (ResidentArgs geo_a, geo_b): a warp's 32 records are then two loads of
