@@ -10,9 +10,8 @@
 // fixed-size array below instead of in cudaMalloc'ed memory.
 //
 // The array exists once per GPU that loads this library and stays allocated
-// until the process exits.  Every call shares it and it keeps the contents
-// of the last call, so each call clears what must start at zero before its
-// step.  Calls whose work overlaps on the GPU (different streams, or several
+// until the process exits.  Every call shares it; a step's last block leaves its
+// counter at zero for the next call.  Calls whose work overlaps on the GPU (different streams, or several
 // host threads) race on the array: serialise them.
 //
 // Set-up: the first call on a device, with that device current, looks up the
@@ -180,6 +179,18 @@ extern "C" int srs_explicit_step_fp64_noalloc(const srs_noalloc_step* d) {
   a.CS.rows = nullptr;
   a.counters = sc->counters;
 
+  // Small problems: one launch, which brings its step and keys along.  The
+  // counters are zero before it (the array starts so, and the last block of a
+  // step leaves its counter so).
+  if (plain64_keys_fit(a)) {
+    Plain64Keys<true> keys;
+    keys.step = d->step;
+    keys.status = d->status;
+    std::memcpy(keys.seeds, d->seeds, sizeof(uint64_t) * d->n_realizations);
+    if (launch_plain64_keys(a, keys, st))
+      return set_last_error(SRS_ERR_CUDA, std::string("step: ") + cudaGetErrorString(cudaGetLastError()));
+    return SRS_OK;
+  }
   NoallocInit in;
   std::memset(&in, 0, sizeof(in));
   in.R = d->n_realizations;

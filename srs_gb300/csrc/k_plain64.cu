@@ -21,7 +21,72 @@
 namespace srs {
 
 
-__device__ __forceinline__ double plain64_ca(const double* S_r, int e) { return S_r[e]; }
+// Channel fluxes of element j (UpdateRyRFlux / UpdateLCCFlux, :127-164) added
+// to its Ca rate in the reference's order.
+__device__ __forceinline__ double channels64(const Plain64Args& a, const double* Sca, int j, double c_ca,
+                                             double b_ca, const int32_t* ryr, const int32_t* lcc,
+                                             const int32_t* lccv, int v) {
+  for (int q = a.chan_ptr[j]; q < a.chan_ptr[j + 1]; ++q) {
+    ChanEntry e = a.chan_list[q];
+    if (e.kind < 2) {
+      if (ryr[e.ch]) {
+        double J = a.P.v_ryr * (Sca[a.C.ryr_jsr[e.ch]] - Sca[a.C.ryr_cleft[e.ch]]) * a.P.v_cell;
+        if (e.kind == 0) b_ca += J / a.v0[j];
+        else b_ca -= J / a.v0[j];
+      }
+    } else if ((lcc[e.ch] == 6 || lcc[e.ch] == 12) && lccv[e.ch] == 2) {
+      double J = a.P.lccA[v] * (c_ca * a.P.lccE[v] - a.P.lccB) / a.P.lccEm1[v] / a.v0[j];
+      b_ca += J;
+    }
+  }
+  return b_ca;
+}
+
+// The last block of realization r to get here gates its channels from the new
+// Ca and, but for the allocation-free form (KEYS), runs the protocol of the next
+// step.  chan: this block holds channel elements, whose new Ca the last block
+// must see.
+template <bool KEYS = false>
+__device__ __forceinline__ void plain64_tail(const Plain64Args& a, int r, const RealCtl& ctl0, const double* Sn,
+                                             bool chan) {
+  __shared__ int s_last;
+  __shared__ int32_t s_nb[1024];
+  if (chan) {
+    __threadfence();
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    unsigned int done = atomicAdd(a.counters + r, 1u);
+    s_last = (done == gridDim.x - 1);
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  RealCtl ctl = ctl0;
+  auto ca = [&](int e) -> double { return *((volatile const double*)(Sn + e)); };
+  int32_t* ryr_w = a.CS.ryr + (size_t)r * a.C.NR;
+  int32_t* lcc_w = a.CS.lcc + (size_t)r * a.C.NL;
+  int32_t* lccv_w = a.CS.lccv + (size_t)r * a.C.NL;
+  double* res = a.CS.res + (size_t)r * (a.C.NR + a.C.NL);
+  if (!a.P.nogating) {
+    gate_all(a.P, a.C, ctl.vsel, ctl.seed, ctl.step, ryr_w, lcc_w, lccv_w, res, s_nb,
+             threadIdx.x, blockDim.x, ca, []() { __syncthreads(); });
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    a.counters[r] = 0;  // as the next step finds it
+    if constexpr (!KEYS) {
+      ctl.step += 1;
+      ctl.t += a.P.dt;
+      prestep(a.P, a.C, ctl, ryr_w, lcc_w, lccv_w,
+              a.CS.rows + (size_t)r * a.P.row_cap * a.P.row_w, ca);
+      RealCtl* c = a.CS.ctl + r;
+      ctl.status |= c->status;  // bits of the other blocks
+      *c = ctl;
+    }
+    __threadfence();
+  }
+}
 
 __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
   const int r = blockIdx.y;
@@ -82,29 +147,7 @@ __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
       o_csqn = q + r_net * dt;
       b_ca += (a.nsr - c_ca) * p[36];
     }
-    // Channel fluxes (UpdateRyRFlux / UpdateLCCFlux, :127-164), in order.
-    if (fl & 4) {
-      const int v = ctlp->vsel;
-      for (int q = a.chan_ptr[j]; q < a.chan_ptr[j + 1]; ++q) {
-        ChanEntry e = a.chan_list[q];
-        if (e.kind == 0) {
-          if (ryr[e.ch]) {
-            double J = a.P.v_ryr * (Sca[a.C.ryr_jsr[e.ch]] - Sca[a.C.ryr_cleft[e.ch]]) * a.P.v_cell;
-            b_ca += J / a.v0[j];
-          }
-        } else if (e.kind == 1) {
-          if (ryr[e.ch]) {
-            double J = a.P.v_ryr * (Sca[a.C.ryr_jsr[e.ch]] - Sca[a.C.ryr_cleft[e.ch]]) * a.P.v_cell;
-            b_ca -= J / a.v0[j];
-          }
-        } else {
-          if ((lcc[e.ch] == 6 || lcc[e.ch] == 12) && lccv[e.ch] == 2) {
-            double J = a.P.lccA[v] * (c_ca * a.P.lccE[v] - a.P.lccB) / a.P.lccEm1[v] / a.v0[j];
-            b_ca += J;
-          }
-        }
-      }
-    }
+    if (fl & 4) b_ca = channels64(a, S, j, c_ca, b_ca, ryr, lcc, lccv, ctlp->vsel);
     b_ca = fast_buffer64(a, b_ca, c_ca, a.bhi[j], a.blo[j]);
     // Euler update (:640-644)
     double* O = So;
@@ -117,43 +160,60 @@ __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
     O[5 * N + j] = dye + b_dye * dt;
     if (!finite64(ca_new)) atomicOr(&ctlp->status, 1u);
   }
-  // ---- last block of this realization: gating + next step's protocol ----
-  __shared__ int s_last;
-  __shared__ int32_t s_nb[1024];
-  // the last block gates from the new Ca of the channel elements: blocks
-  // holding channel elements make their writes visible before counting in
-  if (__syncthreads_or(j < N && (a.flags[j] & 4) != 0)) {
-    __threadfence();
-    __syncthreads();
+  plain64_tail(a, r, *ctlp, So, __syncthreads_or(j < N && (a.flags[j] & 4) != 0) != 0);
+}
+
+// The same for problems of few elements: 32 elements a block, the update dealt
+// to four warps (srs_plain64_update.cuh).  KEYS: the allocation-free form, whose
+// step and seeds come with the launch (NoallocKeys) instead of from RealCtl.
+template <bool KEYS>
+__global__ void __launch_bounds__(128) k_plain64_split(const __grid_constant__ Plain64Args a,
+                                                       const __grid_constant__ Plain64Keys<KEYS> keys) {
+  __shared__ double s_rate[5][32];
+  const int r = blockIdx.y;
+  RealCtl ctl{};
+  unsigned* status;
+  if constexpr (KEYS) {
+    ctl.step = keys.step;
+    ctl.seed = keys.seeds[r];
+    ctl.lcc_close_step = -1;
+    status = keys.status;
+  } else {
+    ctl = a.CS.ctl[r];
+    status = &a.CS.ctl[r].status;
+    if (ctl.done) return;  // uniform per realization
   }
-  if (threadIdx.x == 0) {
-    unsigned int done = atomicAdd(a.counters + r, 1u);
-    s_last = (done == gridDim.x - 1);
+  const int N = a.N, lane = threadIdx.x & 31, role = ((threadIdx.x >> 5) + blockIdx.x) & 3;
+  const int j = blockIdx.x * 32 + lane;
+  const int e = min(j, N - 1);  // the last element stands in
+  const size_t n = N, ro = (size_t)r * 6 * N;
+  const double* S = a.S_in + ro;
+  double* So = a.S_out + ro;
+  const Geo64 g = geometry64(a, e);
+  const double c = S[e];
+  double x0 = S[role64_x0(role) * n + e], x1 = S[role64_x1(role) * n + e];
+  const double b0 = role64(a, role, g, e, lane, S, c, x0, x1, s_rate);
+  if (j < N && role > 0) {
+    So[role64_x0(role) * n + e] = x0;
+    if (role < 3) So[role64_x1(role) * n + e] = x1;
   }
   __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  RealCtl ctl = *ctlp;
-  const double* Sn = So;  // Ca after the update
-  auto ca = [&](int e) -> double { return *((volatile const double*)(Sn + e)); };
-  int32_t* ryr_w = a.CS.ryr + (size_t)r * a.C.NR;
-  int32_t* lcc_w = a.CS.lcc + (size_t)r * a.C.NL;
-  int32_t* lccv_w = a.CS.lccv + (size_t)r * a.C.NL;
-  double* res = a.CS.res + (size_t)r * (a.C.NR + a.C.NL);
-  if (!a.P.nogating) {
-    gate_all(a.P, a.C, ctl.vsel, ctl.seed, ctl.step, ryr_w, lcc_w, lccv_w, res, s_nb,
-             threadIdx.x, blockDim.x, ca, []() { __syncthreads(); });
-    __syncthreads();
+  if (role == 0) {
+    double b_ca = sum64(a, g.fl, lane, c, b0, s_rate);
+    if (g.fl & 4) {
+      const int32_t* ryr = a.CS.ryr + (size_t)r * a.C.NR;
+      const int32_t* lcc = a.CS.lcc + (size_t)r * a.C.NL;
+      const int32_t* lccv = a.CS.lccv + (size_t)r * a.C.NL;
+      b_ca = channels64(a, S, e, c, b_ca, ryr, lcc, lccv, ctl.vsel);
+    }
+    b_ca = fast_buffer64(a, b_ca, c, a.bhi[e], a.blo[e]);
+    const double ca_new = c + b_ca * a.P.dt;
+    if (j < N) {
+      So[e] = ca_new;
+      if (!finite64(ca_new) && status) atomicOr(status, 1u);
+    }
   }
-  if (threadIdx.x == 0) {
-    ctl.step += 1;
-    ctl.t += a.P.dt;
-    prestep(a.P, a.C, ctl, ryr_w, lcc_w, lccv_w,
-            a.CS.rows + (size_t)r * a.P.row_cap * a.P.row_w, ca);
-    *ctlp = ctl;
-    a.counters[r] = 0;
-    __threadfence();
-  }
+  plain64_tail<KEYS>(a, r, ctl, So, __syncthreads_or(g.fl & 4) != 0);
 }
 
 // Protocol work before the first step of a run (and the t = 0 row).
@@ -186,12 +246,27 @@ void plain64_consts(Plain64Args* a) {
   a->inv_kdi = k > 0x1p-500 && k < 0x1p500 ? 1.0 / a->p[49] : 0.0;
 }
 
-int launch_plain64_step(const Plain64Args& a, cudaStream_t st) {
-  // Few realizations: 64-thread blocks spread the element updates (and their
-  // FP64 arithmetic) over more SMs than 256-thread blocks would.
+// Tiles of 32 elements up to which the update is dealt to four warps: six blocks
+// per SM.  Beyond, the FP64 pipes are busy anyway and a thread per element
+// avoids passing values between warps.
+static bool split64(const Plain64Args& a) { return (int64_t)((a.N + 31) / 32) * a.R <= 6 * 152; }
+
+static void launch_step64(const Plain64Args& a, cudaStream_t st) {
+  // few realizations: 64-thread blocks spread the element updates (and their
+  // FP64 arithmetic) over more SMs than 256-thread blocks would
   const int bs = (size_t)((a.N + 255) / 256) * a.R < 304 ? 64 : 256;
-  dim3 grid((a.N + bs - 1) / bs, a.R);
-  k_plain64_step<<<grid, bs, 0, st>>>(a);
+  k_plain64_step<<<dim3((a.N + bs - 1) / bs, a.R), bs, 0, st>>>(a);
+}
+
+int launch_plain64_step(const Plain64Args& a, cudaStream_t st) {
+  if (split64(a)) k_plain64_split<false><<<dim3((a.N + 31) / 32, a.R), 128, 0, st>>>(a, {});
+  else launch_step64(a, st);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+bool plain64_keys_fit(const Plain64Args& a) { return split64(a); }
+int launch_plain64_keys(const Plain64Args& a, const Plain64Keys<true>& k, cudaStream_t st) {
+  k_plain64_split<true><<<dim3((a.N + 31) / 32, a.R), 128, 0, st>>>(a, k);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 int launch_plain64_prestep(const Plain64Args& a, int write_initial_row, cudaStream_t st) {

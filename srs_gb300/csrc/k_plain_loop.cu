@@ -413,15 +413,10 @@ __global__ void __launch_bounds__(PLAIN_LOOP_T32, 6) k_plain32_loop(const __grid
 }
 
 // ---- FP64 ----------------------------------------------------------------------
-// A block takes E times 32 elements with four warps, each warp its share of the
-// update (its "role"), because an FP64 warp instruction occupies a quarter of
-// an SM for 64 cycles: 112 of them in one warp are 3.5 us, dealt to four 1.2.
-//   role 0: Ca -- diffusion; after the others, the sums of Ca's rate in the
-//           reference's order, rapid buffer, Euler;
-//   role 1: troponin C or calsequestrin, SERCA;  role 2: dye and ATP;
-//   role 3: calmodulin, and the gating of the block's channels.
-// Blocks go to the SMs in turn; the roles move on by one warp with each turn, so
-// that the blocks of an SM load its quarters evenly.
+// A block takes E times 32 elements with four warps in four roles
+// (srs_plain64_update.cuh); role 3 also gates the block's channels.  Blocks go
+// to the SMs in turn; the roles move on by one warp with each turn, so that the
+// blocks of an SM load its quarters evenly.
 template <int E>
 __global__ void __launch_bounds__(128, 6) k_plain64_loop(const __grid_constant__ Plain64Args a,
                                                          const __grid_constant__ PlainLoop l) {
@@ -447,29 +442,9 @@ __global__ void __launch_bounds__(128, 6) k_plain64_loop(const __grid_constant__
   const int j0 = b * (PLAIN_LOOP_TILE64 * E) + lane;
   auto element = [&](int t) { return min(j0 + t * 32, N - 1); };  // the last one stands in
   auto valid = [&](int t) { return j0 + t * 32 < N; };
-  const double* p = a.p;
   const double dt = a.P.dt;
   const size_t n = N;
-  struct Geo {
-    double ac[5];
-    int n1, n2, n3, n4, fl;
-  };
-  auto geometry = [&](int t) {
-    const int e = element(t);
-    Geo g;
-#pragma unroll
-    for (int q = 0; q < 5; ++q) g.ac[q] = __ldg(a.aij + 5 * (size_t)e + q);
-    const int4 nn = __ldg(reinterpret_cast<const int4*>(a.nij) + e);
-    g.n1 = nn.x;
-    g.n2 = nn.y;
-    g.n3 = nn.z;
-    g.n4 = nn.w;
-    g.fl = __ldg(a.flags + e);
-    return g;
-  };
-  // this role's own values: Ca; TRPN, CSQN; dye, ATP; CMDN
-  const int sp0 = role == 0 ? 0 : role == 1 ? 3 : role == 2 ? 5 : 2;
-  const int sp1 = role == 1 ? 4 : 1;  // roles 1 and 2
+  const int sp0 = role64_x0(role), sp1 = role64_x1(role);
   double x0[E], x1[E];
 #pragma unroll
   for (int t = 0; t < E; ++t) {
@@ -477,7 +452,7 @@ __global__ void __launch_bounds__(128, 6) k_plain64_loop(const __grid_constant__
     x1[t] = role == 1 || role == 2 ? S[0][sp1 * n + element(t)] : 0.0;
     if (role == 0) s_ca[t][lane] = x0[t];
   }
-  Geo geo = geometry(0);  // kept where a lane has one element
+  Geo64 geo = geometry64(a, element(0));  // kept where a lane has one element
   unsigned* bar = l.bar + r;
   __syncthreads();
   bool ok = true;
@@ -487,72 +462,30 @@ __global__ void __launch_bounds__(128, 6) k_plain64_loop(const __grid_constant__
     double b_ca[E];
 #pragma unroll
     for (int t = 0; t < E; ++t) {
-      if (t > 0) geo = geometry(t);
+      if (t > 0) geo = geometry64(a, element(t));
       const int e = element(t);
-      const bool jsr = geo.fl & 1, trop = !jsr && (geo.fl & 2);
-      const double c = s_ca[t][lane];
-      auto diffuse = [&](const double* f, double D, double x, double br) {
-        return diffuse64(D, x, __ldcg(f + geo.n1), __ldcg(f + geo.n2), __ldcg(f + geo.n3), __ldcg(f + geo.n4),
-                         geo.ac, br);
-      };
-      if (role == 0) {
-        b_ca[t] = diffuse(src, p[5], c, __ldg(a.br + e));
-      } else if (role == 1) {
-        double rate = 0.0, y0 = plus_zero(x0[t]), y1 = plus_zero(x1[t]);
-        if (trop) {
-          rate = react64(p[26], p[24], p[25], x0[t], c);
-          s_rate[t][1][lane] = serca64(a, c);
-          y0 = x0[t] + rate * dt;
-        } else if (jsr) {
-          rate = react64(p[39], p[34], p[40], x1[t], c);
-          y1 = x1[t] + rate * dt;
-        }
-        s_rate[t][0][lane] = rate;
-        x0[t] = y0;
-        x1[t] = y1;
-      } else if (role == 2) {
-        double b_dye = diffuse(src + 5 * n, p[11], x0[t], __ldg(a.br + 3 * n + e));
-        double b_atp = diffuse(src + n, p[7], x1[t], __ldg(a.br + n + e));
-        if (!jsr) {
-          const double rd = react64(p[33], p[31], p[32], x0[t], c), ra = react64(p[20], p[18], p[19], x1[t], c);
-          s_rate[t][2][lane] = rd;
-          s_rate[t][3][lane] = ra;
-          b_dye += rd;
-          b_atp += ra;
-        }
-        x0[t] = x0[t] + b_dye * dt;
-        x1[t] = x1[t] + b_atp * dt;
-        if (valid(t)) {
-          __stcg(dst + 5 * n + e, x0[t]);
-          __stcg(dst + n + e, x1[t]);
-        }
-      } else {
-        if (t == 0 && ch.n > 0) {
-          const int v = lp.vsel;
-          const bool close = s > 0 && advance_protocol(a, lp);
-          for (int i = lane; i < ch.n; i += 32) {
-            const bool ryr = ch.id[i] < a.C.NR;
-            const double u0 = __ldcg(src + ch.e0[i]), u1 = ryr ? __ldcg(src + ch.e1[i]) : 0.0;
-            const bool open = s > 0 ? gate_local(a, ch, i, lp, v, close, (float)u0, (float)u1)
-                                    : open_local(ch, i, a.C.NR);
-            double f = closed;
-            if (open) {
-              const int w = lp.vsel;
-              f = ryr ? a.P.v_ryr * (u1 - u0) * a.P.v_cell
-                      : a.P.lccA[w] * (u0 * a.P.lccE[w] - a.P.lccB) / a.P.lccEm1[w];
-            }
-            J[i] = f;
+      if (role == 3 && t == 0 && ch.n > 0) {
+        const int v = lp.vsel;
+        const bool close = s > 0 && advance_protocol(a, lp);
+        for (int i = lane; i < ch.n; i += 32) {
+          const bool ryr = ch.id[i] < a.C.NR;
+          const double u0 = __ldcg(src + ch.e0[i]), u1 = ryr ? __ldcg(src + ch.e1[i]) : 0.0;
+          const bool open = s > 0 ? gate_local(a, ch, i, lp, v, close, (float)u0, (float)u1)
+                                  : open_local(ch, i, a.C.NR);
+          double f = closed;
+          if (open) {
+            const int w = lp.vsel;
+            f = ryr ? a.P.v_ryr * (u1 - u0) * a.P.v_cell
+                    : a.P.lccA[w] * (u0 * a.P.lccE[w] - a.P.lccB) / a.P.lccEm1[w];
           }
-          lp.step += 1;
+          J[i] = f;
         }
-        double b_cmdn = diffuse(src + 2 * n, p[8], x0[t], __ldg(a.br + 2 * n + e));
-        if (!jsr) {
-          const double rm = react64(p[23], p[21], p[22], x0[t], c);
-          s_rate[t][4][lane] = rm;
-          b_cmdn += rm;
-        }
-        x0[t] = x0[t] + b_cmdn * dt;
-        if (valid(t)) __stcg(dst + 2 * n + e, x0[t]);
+        lp.step += 1;
+      }
+      b_ca[t] = role64(a, role, geo, e, lane, src, s_ca[t][lane], x0[t], x1[t], s_rate[t]);
+      if (role >= 2 && valid(t)) {
+        __stcg(dst + sp0 * n + e, x0[t]);
+        if (role == 2) __stcg(dst + n + e, x1[t]);
       }
     }
     __syncthreads();
@@ -561,19 +494,7 @@ __global__ void __launch_bounds__(128, 6) k_plain64_loop(const __grid_constant__
       for (int t = 0; t < E; ++t) {
         const int e = element(t), fl = E > 1 ? __ldg(a.flags + e) : geo.fl;
         const double c = s_ca[t][lane];
-        double bc = b_ca[t];
-        if (!(fl & 1)) {
-          if (fl & 2) {
-            bc += -s_rate[t][0][lane];
-            bc -= s_rate[t][1][lane];
-          }
-          bc += -s_rate[t][2][lane];
-          bc += -s_rate[t][3][lane];
-          bc += -s_rate[t][4][lane];
-        } else {
-          bc += -s_rate[t][0][lane];
-          bc += (a.nsr - c) * p[36];
-        }
+        double bc = sum64(a, fl, lane, c, b_ca[t], s_rate[t]);
         if (fl & 4) {
           for (int q = a.chan_ptr[e]; q < a.chan_ptr[e + 1]; ++q) {
             const double f = J[l.loc[q]];
@@ -588,7 +509,7 @@ __global__ void __launch_bounds__(128, 6) k_plain64_loop(const __grid_constant__
         if (valid(t)) __stcg(dst + e, x0[t]);
       }
     }
-    if (E > 1) geo = geometry(0);
+    if (E > 1) geo = geometry64(a, element(0));
     __syncthreads();
     if (threadIdx.x == 0) red_release_add(bar, 1u);
     if (s + 1 < steps && !wait_all(bar, (unsigned)(s + 1) * (unsigned)(l.blocks + 1))) {

@@ -33,6 +33,18 @@ struct Plain64Args {
   unsigned int* counters;
 };
 void plain64_consts(Plain64Args* a);
+// Step index, Philox keys and status word of an allocation-free step, with the
+// launch itself (empty for the engine's own steps, which read RealCtl).
+template <bool KEYS>
+struct Plain64Keys {};
+template <>
+struct Plain64Keys<true> {
+  int64_t step;
+  unsigned* status;  // may be null
+  uint64_t seeds[SRS_NOALLOC_MAX_REALIZATIONS];
+};
+bool plain64_keys_fit(const Plain64Args& a);
+int launch_plain64_keys(const Plain64Args& a, const Plain64Keys<true>& k, cudaStream_t st);
 int launch_plain64_step(const Plain64Args& a, cudaStream_t st);
 int launch_plain64_prestep(const Plain64Args& a, int write_initial_row, cudaStream_t st);
 

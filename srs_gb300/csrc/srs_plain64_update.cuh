@@ -73,4 +73,101 @@ __device__ __forceinline__ double fast_buffer64(const Plain64Args& a, double b_c
   return b_ca / B;
 }
 
+// ---- the update dealt to four warps ----------------------------------------------
+// 32 elements, one per lane of each of four warps; each warp has its share (its
+// "role"), because an FP64 warp instruction occupies a quarter of an SM for 64
+// cycles: 112 of them in one warp are 3.5 us, dealt to four 1.2.
+//   role 0: Ca -- diffusion; after the others, the sums of Ca's rate in the
+//           reference's order, channel fluxes, rapid buffer, Euler;
+//   role 1: troponin C or calsequestrin, SERCA;  role 2: dye and ATP;
+//   role 3: calmodulin.
+struct Geo64 {
+  double ac[5];
+  int n1, n2, n3, n4, fl;
+};
+__device__ __forceinline__ Geo64 geometry64(const Plain64Args& a, int e) {
+  Geo64 g;
+#pragma unroll
+  for (int q = 0; q < 5; ++q) g.ac[q] = __ldg(a.aij + 5 * (size_t)e + q);
+  const int32_t* nn = a.nij + 4 * (size_t)e;
+  g.n1 = __ldg(nn);
+  g.n2 = __ldg(nn + 1);
+  g.n3 = __ldg(nn + 2);
+  g.n4 = __ldg(nn + 3);
+  g.fl = __ldg(a.flags + e);
+  return g;
+}
+// First of the species whose value a role holds in x0 and, roles 1 and 2, x1.
+__device__ __forceinline__ int role64_x0(int role) { return role == 0 ? 0 : role == 1 ? 3 : role == 2 ? 5 : 2; }
+__device__ __forceinline__ int role64_x1(int role) { return role == 1 ? 4 : 1; }
+
+// A role's share of one element from the state src (read past L1) and the
+// element's Ca c.  Returns Ca's diffusion (role 0); advances x0, x1 (the
+// others) and leaves the reactions in rate: immobile buffer, SERCA, dye, ATP,
+// CMDN.
+__device__ __forceinline__ double role64(const Plain64Args& a, int role, const Geo64& g, int e, int lane,
+                                         const double* src, double c, double& x0, double& x1,
+                                         double (*rate)[32]) {
+  const double* p = a.p;
+  const double dt = a.P.dt;
+  const size_t n = a.N;
+  const bool jsr = g.fl & 1, trop = !jsr && (g.fl & 2);
+  auto diffuse = [&](const double* f, double D, double x, double br) {
+    return diffuse64(D, x, __ldcg(f + g.n1), __ldcg(f + g.n2), __ldcg(f + g.n3), __ldcg(f + g.n4), g.ac, br);
+  };
+  if (role == 0) return diffuse(src, p[5], c, __ldg(a.br + e));
+  if (role == 1) {
+    double r = 0.0, y0 = plus_zero(x0), y1 = plus_zero(x1);
+    if (trop) {
+      r = react64(p[26], p[24], p[25], x0, c);
+      rate[1][lane] = serca64(a, c);
+      y0 = x0 + r * dt;
+    } else if (jsr) {
+      r = react64(p[39], p[34], p[40], x1, c);
+      y1 = x1 + r * dt;
+    }
+    rate[0][lane] = r;
+    x0 = y0;
+    x1 = y1;
+  } else if (role == 2) {
+    double b_dye = diffuse(src + 5 * n, p[11], x0, __ldg(a.br + 3 * n + e));
+    double b_atp = diffuse(src + n, p[7], x1, __ldg(a.br + n + e));
+    if (!jsr) {
+      const double rd = react64(p[33], p[31], p[32], x0, c), ra = react64(p[20], p[18], p[19], x1, c);
+      rate[2][lane] = rd;
+      rate[3][lane] = ra;
+      b_dye += rd;
+      b_atp += ra;
+    }
+    x0 = x0 + b_dye * dt;
+    x1 = x1 + b_atp * dt;
+  } else {
+    double b_cmdn = diffuse(src + 2 * n, p[8], x0, __ldg(a.br + 2 * n + e));
+    if (!jsr) {
+      const double rm = react64(p[23], p[21], p[22], x0, c);
+      rate[4][lane] = rm;
+      b_cmdn += rm;
+    }
+    x0 = x0 + b_cmdn * dt;
+  }
+  return 0.0;
+}
+// Ca's rate with the reactions added to its diffusion b_ca (role 0).
+__device__ __forceinline__ double sum64(const Plain64Args& a, int fl, int lane, double c, double b_ca,
+                                        double (*rate)[32]) {
+  if (!(fl & 1)) {
+    if (fl & 2) {
+      b_ca += -rate[0][lane];
+      b_ca -= rate[1][lane];
+    }
+    b_ca += -rate[2][lane];
+    b_ca += -rate[3][lane];
+    b_ca += -rate[4][lane];
+  } else {
+    b_ca += -rate[0][lane];
+    b_ca += (a.nsr - c) * a.p[36];
+  }
+  return b_ca;
+}
+
 }  // namespace srs
