@@ -45,6 +45,7 @@ def _units():
         ("k_res_b.o", common_cu + ["-fmad=false", "-c", os.path.join(CSRC, "k_res_b.cu")]),
         ("k_res_c.o", common_cu + ["-fmad=false", "-c", os.path.join(CSRC, "k_res_c.cu")]),
         ("k_res_d.o", common_cu + ["-fmad=false", "-c", os.path.join(CSRC, "k_res_d.cu")]),
+        ("k_state.o", common_cu + ["-fmad=false", "-c", os.path.join(CSRC, "k_state.cu")]),
         ("k_plain_loop.o", common_cu + ["-fmad=false", "-c", os.path.join(CSRC, "k_plain_loop.cu")]),
         ("srs_capi.o", common_cu + ["-fmad=false", "-c", os.path.join(CSRC, "srs_capi.cu")]),
         ("k_noalloc.o", common_cu + ["-fmad=false", "-c", os.path.join(CSRC, "k_noalloc.cu")]),

@@ -186,6 +186,8 @@ __device__ void gate_loop(const Args& a, const PlainLoop& l, int r, int steps, C
     c->tick_cache_idx = g->ctl.tick_cache_idx;
     c->tick_cache_ver = g->ctl.tick_cache_ver;
     if (bits) atomicOr(&c->status, bits);
+    if (ok) *bar = 0;  // every block has arrived for the last time
+    else *l.timeout = 1u;
   }
 }
 
@@ -410,6 +412,7 @@ __global__ void __launch_bounds__(PLAIN_LOOP_T32, 6) k_plain32_loop(const __grid
     if (!isfinite(x[t].x)) bits |= 1u;
   }
   if (bits) atomicOr(&a.CS.ctl[r].status, bits);
+  if (!ok && threadIdx.x == 0) *l.timeout = 1u;
 }
 
 // ---- FP64 ----------------------------------------------------------------------
@@ -529,6 +532,7 @@ __global__ void __launch_bounds__(128, 6) k_plain64_loop(const __grid_constant__
     if (role == 0 && !finite64(x0[t])) bits |= 1u;
   }
   if (bits) atomicOr(&a.CS.ctl[r].status, bits);
+  if (!ok && threadIdx.x == 0) *l.timeout = 1u;
 }
 
 template <class K>

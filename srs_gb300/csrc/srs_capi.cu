@@ -93,15 +93,22 @@ struct srs_sim {
   std::vector<int> part_start, part_len, part_nch, part_nint;  // resident partitions
   int ch_interior = 0;
   int64_t launches = 0;
-  cudaGraphExec_t graph_plain = nullptr;
+  cudaGraphExec_t graph_plain = nullptr;      // steps from state buffer 0 ...
+  cudaGraphExec_t graph_plain_alt = nullptr;  // ... captured when the buffers were exchanged
   int graph_plain_len = 0;
   PlainLoop loop{};  // plain engines: steps in one launch (blocks 0: not used)
   size_t loop_smem = 0;
-  void* h_stage = nullptr;  // pinned host staging for state uploads
+  void* h_stage = nullptr;         // pinned: exchanges larger than that
   size_t h_stage_bytes = 0;
-  // the FP32 staging holds this many copies of one realization's state
-  // (the last upload_state_range); 0: unknown content
-  int stage_copies = 0;
+  std::mutex stage_mtx;            // held while staging or d_export is in use
+  unsigned char* h_pin = nullptr;  // pinned: the timeout flag of the kernels' waits, staging
+  size_t h_pin_bytes = 0;
+  double* d_S0 = nullptr;          // FP64 engine: the equilibrium state [6][N]
+  int32_t* d_eng_of_ref = nullptr;  // FP32 engines: [N]
+  double* d_export = nullptr;      // a realization's state in the caller's form (large meshes)
+  // every realization has finished its run (known for parameter sets without
+  // the fidelity criterion, whose realizations finish together)
+  bool finished = false;
   // line scan
   LinescanArgs ls{};
   std::vector<double> ls_rest;  // F at the equilibrium state
@@ -415,6 +422,9 @@ int setup_plain64(srs_sim* s) {
   SRS_TRY(dev_upload(s, (int32_t**)&a.chan_ptr, ptr.data(), ptr.size()));
   SRS_TRY(dev_upload(s, (ChanEntry**)&a.chan_list, list.data(), list.size()));
   for (int b = 0; b < 2; ++b) SRS_TRY(dev_alloc(s, &s->d_S[b], (size_t)s->R * 6 * N));
+  std::vector<double> S0;
+  initial_states(s->m, s->p, &S0);
+  SRS_TRY(dev_upload(s, &s->d_S0, S0.data(), S0.size()));
   for (int q = 0; q < 56; ++q) a.p[q] = R[q];
   SRS_TRY(upload_channels_engine_order(s));
   return SRS_OK;
@@ -531,6 +541,7 @@ int setup_plain32(srs_sim* s) {
     SRS_TRY(dev_alloc(s, &s->d_M[b], (size_t)s->R * N));
     SRS_TRY(dev_alloc(s, &s->d_I[b], (size_t)s->R * N));
   }
+  SRS_TRY(dev_upload(s, &s->d_eng_of_ref, s->eng_of_ref.data(), s->eng_of_ref.size()));
   // compensation terms as halves (srs_comp.h), as in the resident engine
   SRS_TRY(dev_alloc(s, &s->d_CMq, (size_t)s->R * N));
   SRS_TRY(dev_alloc(s, &s->d_CIq, (size_t)s->R * N));
@@ -945,6 +956,7 @@ int setup_resident(srs_sim* s, int C, int threads) {
   s->ch.ryr_jsr = p2;
   s->ch.ryr_nb = p3;
   s->ch.lcc_ele = p4;
+  SRS_TRY(dev_upload(s, &s->d_eng_of_ref, s->eng_of_ref.data(), s->eng_of_ref.size()));
   SRS_TRY(dev_alloc(s, &s->d_M[0], (size_t)s->R * NE));
   SRS_TRY(dev_alloc(s, &s->d_I[0], (size_t)s->R * NE));
   SRS_TRY(dev_alloc(s, &s->d_CM, (size_t)s->R * NE));
@@ -965,8 +977,26 @@ size_t eng_count(const srs_sim* s) {
 }
 
 // ---- state conversion ---------------------------------------------------------
+// Staging of export_state with ns state values in it; states beyond
+// kExportDirect bytes are copied without.
+constexpr size_t kExportDirect = (size_t)4 << 20;
+size_t export_bytes(const srs_sim* s, size_t ns) {
+  return (ns + s->NCH) * sizeof(double) + (size_t)(s->NR + 2 * s->NL) * sizeof(int32_t);
+}
+
+// Pinned memory for an exchange with the device.  The first block stays for the
+// simulation's life (its first word is the kernels' timeout flag); an exchange
+// that does not fit it takes a second one.
+constexpr size_t kPinHead = 64;
 void* stage(srs_sim* s, size_t bytes) {
-  s->stage_copies = 0;
+  if (!s->h_pin) {
+    const size_t own = export_bytes(s, (size_t)6 * s->N);
+    const size_t n = std::max(bytes, own <= kExportDirect ? own : 0);
+    if (cudaMallocHost((void**)&s->h_pin, kPinHead + n) != cudaSuccess) return nullptr;
+    s->h_pin_bytes = n;
+    *reinterpret_cast<unsigned*>(s->h_pin) = 0;
+  }
+  if (bytes <= s->h_pin_bytes) return s->h_pin + kPinHead;
   if (bytes > s->h_stage_bytes) {
     if (s->h_stage) cudaFreeHost(s->h_stage);
     s->h_stage = nullptr;
@@ -975,6 +1005,17 @@ void* stage(srs_sim* s, size_t bytes) {
     s->h_stage_bytes = bytes;
   }
   return s->h_stage;
+}
+
+int clear_compensation(srs_sim* s, size_t o, size_t n) {
+  if (s->d_CMq) {  // a half of 0 is 0
+    SRS_CUDA(cudaMemsetAsync(s->d_CMq + o, 0, n * sizeof(ushort4), s->st));
+    SRS_CUDA(cudaMemsetAsync(s->d_CIq + o, 0, n * sizeof(uint16_t), s->st));
+  } else {
+    SRS_CUDA(cudaMemsetAsync(s->d_CM + o, 0, n * sizeof(float4), s->st));
+    SRS_CUDA(cudaMemsetAsync(s->d_CI + o, 0, n * sizeof(float), s->st));
+  }
+  return SRS_OK;
 }
 
 // Reference-numbered absolute state -> engine layout of one realization.
@@ -1002,117 +1043,121 @@ void to_engine_fp32(const srs_sim* s, const double* S6, float4* M, float* I) {
   }
 }
 
-// Uploads one state to realizations [r0, r1) through pinned staging.
-int upload_state_range(srs_sim* s, int r0, int r1, const double* S6) {
+// Uploads one state to realization r through pinned staging.
+int upload_state(srs_sim* s, int r, const double* S6) {
+  std::lock_guard<std::mutex> lock(s->stage_mtx);
   const int N = s->N;
-  const int nr = r1 - r0;
   if (s->d.precision == SRS_FP64) {
     const size_t per = (size_t)6 * N;
-    double* h = (double*)stage(s, per * nr * sizeof(double));
+    double* h = (double*)stage(s, per * sizeof(double));
     if (!h) return fail(SRS_ERR_NOMEM, "pinned staging allocation failed");
-    for (int r = 0; r < nr; ++r) std::memcpy(h + r * per, S6, per * sizeof(double));
-    SRS_CUDA(cudaMemcpyAsync(s->d_S[0] + (size_t)r0 * per, h, per * nr * sizeof(double),
-                             cudaMemcpyHostToDevice, s->st));
+    std::memcpy(h, S6, per * sizeof(double));
+    SRS_CUDA(cudaMemcpyAsync(s->d_S[0] + (size_t)r * per, h, per * sizeof(double), cudaMemcpyHostToDevice, s->st));
     SRS_CUDA(cudaStreamSynchronize(s->st));
     return SRS_OK;
   }
-  const size_t NE = eng_count(s);
-  const int copies = s->stage_copies;
-  float4* hM = (float4*)stage(s, NE * nr * (sizeof(float4) + sizeof(float)));
+  const size_t NE = eng_count(s), o = (size_t)r * NE;
+  float4* hM = (float4*)stage(s, NE * (sizeof(float4) + sizeof(float)));
   if (!hM) return fail(SRS_ERR_NOMEM, "pinned staging allocation failed");
-  float* hI = (float*)(hM + NE * nr);
-  // A reset that repeats the previous one (same state, same realizations)
-  // finds the copies already staged: only the upload below is repeated.
-  bool staged = false;
-  if (copies == nr && nr > 1) {
-    std::vector<float4> m0(NE);
-    std::vector<float> i0(NE);
-    to_engine_fp32(s, S6, m0.data(), i0.data());
-    staged = std::memcmp(m0.data(), hM, NE * sizeof(float4)) == 0 &&
-             std::memcmp(i0.data(), hI, NE * sizeof(float)) == 0;
-  }
-  if (!staged) to_engine_fp32(s, S6, hM, hI);
-  // realization 0's state copied into the others' staging slots by up to 8
-  // host threads (the copy is memory-bound: one thread does not saturate it)
-  auto fill = [&](int ra, int rb) {
-    for (int r = ra; r < rb; ++r) {
-      std::memcpy(hM + r * NE, hM, NE * sizeof(float4));
-      std::memcpy(hI + r * NE, hI, NE * sizeof(float));
-    }
-  };
-  const int nt = std::max(1, std::min({8, (int)std::thread::hardware_concurrency(), (nr - 1) / 16}));
-  if (!staged && nt <= 1) {
-    fill(1, nr);
-  } else if (!staged) {
-    std::vector<std::thread> pool;
-    const int chunk = (nr - 1 + nt - 1) / nt;
-    for (int t = 0; t < nt; ++t) {
-      const int ra = 1 + t * chunk, rb = std::min(nr, ra + chunk);
-      if (ra < rb) pool.emplace_back(fill, ra, rb);
-    }
-    for (auto& th : pool) th.join();
-  }
-  SRS_CUDA(cudaMemcpyAsync(s->d_M[0] + (size_t)r0 * NE, hM, NE * nr * sizeof(float4),
-                           cudaMemcpyHostToDevice, s->st));
-  SRS_CUDA(cudaMemcpyAsync(s->d_I[0] + (size_t)r0 * NE, hI, NE * nr * sizeof(float),
-                           cudaMemcpyHostToDevice, s->st));
-  if (s->d_CMq) {  // q = 0 is c = 0
-    SRS_CUDA(cudaMemsetAsync(s->d_CMq + (size_t)r0 * NE, 0, NE * nr * sizeof(ushort4), s->st));
-    SRS_CUDA(cudaMemsetAsync(s->d_CIq + (size_t)r0 * NE, 0, NE * nr * sizeof(uint16_t), s->st));
-  } else {
-    SRS_CUDA(cudaMemsetAsync(s->d_CM + (size_t)r0 * NE, 0, NE * nr * sizeof(float4), s->st));
-    SRS_CUDA(cudaMemsetAsync(s->d_CI + (size_t)r0 * NE, 0, NE * nr * sizeof(float), s->st));
-  }
+  float* hI = (float*)(hM + NE);
+  to_engine_fp32(s, S6, hM, hI);
+  SRS_CUDA(cudaMemcpyAsync(s->d_M[0] + o, hM, NE * sizeof(float4), cudaMemcpyHostToDevice, s->st));
+  SRS_CUDA(cudaMemcpyAsync(s->d_I[0] + o, hI, NE * sizeof(float), cudaMemcpyHostToDevice, s->st));
+  SRS_TRY(clear_compensation(s, o, NE));
   SRS_CUDA(cudaStreamSynchronize(s->st));
-  s->stage_copies = nr;
   return SRS_OK;
 }
 
-int upload_state(srs_sim* s, int r, const double* S6) { return upload_state_range(s, r, r + 1, S6); }
-
-int download_state(srs_sim* s, int r, double* S6) {
-  const int N = s->N;
+// The equilibrium state of every realization (ResetDefaultGridStates).  The
+// FP32 engines hold deviations from it: all zero, in every array.
+int reset_states(srs_sim* s) {
   if (s->d.precision == SRS_FP64) {
-    SRS_CUDA(cudaMemcpy(S6, s->d_S[0] + (size_t)r * 6 * N, sizeof(double) * 6 * N,
-                        cudaMemcpyDeviceToHost));
+    if (launch_broadcast_state(s->d_S0, s->d_S[0], (size_t)6 * s->N, s->R, s->st))
+      return fail(SRS_ERR_CUDA, "state reset launch failed");
     return SRS_OK;
   }
-  size_t NE = eng_count(s);
-  std::vector<float4> M(NE), CMh(NE);
-  std::vector<float> I(NE), CIh(NE);
-  SRS_CUDA(cudaMemcpy(M.data(), s->d_M[0] + r * NE, NE * sizeof(float4), cudaMemcpyDeviceToHost));
-  SRS_CUDA(cudaMemcpy(I.data(), s->d_I[0] + r * NE, NE * sizeof(float), cudaMemcpyDeviceToHost));
-  if (s->d_CMq) {
-    std::vector<ushort4> Q(NE);
-    std::vector<uint16_t> QI(NE);
-    SRS_CUDA(cudaMemcpy(Q.data(), s->d_CMq + r * NE, NE * sizeof(ushort4), cudaMemcpyDeviceToHost));
-    SRS_CUDA(cudaMemcpy(QI.data(), s->d_CIq + r * NE, NE * sizeof(uint16_t), cudaMemcpyDeviceToHost));
-    for (size_t e = 0; e < NE; ++e) {
-      CMh[e] = make_float4(comp_decode_host(Q[e].x), comp_decode_host(Q[e].y), comp_decode_host(Q[e].z),
-                           comp_decode_host(Q[e].w));
-      CIh[e] = comp_decode_host(QI[e]);
-    }
+  const size_t n = (size_t)s->R * eng_count(s);
+  SRS_CUDA(cudaMemsetAsync(s->d_M[0], 0, n * sizeof(float4), s->st));
+  SRS_CUDA(cudaMemsetAsync(s->d_I[0], 0, n * sizeof(float), s->st));
+  return clear_compensation(s, 0, n);
+}
+
+// Realization r in the caller's form (any output may be null): the conversion
+// and the gathering run on the device (k_export_state).  Up to a few MB it
+// writes pinned host memory and the caller's arrays are filled from there;
+// larger states go to a device buffer and are copied out of it.
+int export_state(srs_sim* s, int r, double* S, int* ryr, int* lcc, int* lccv, double* res) {
+  std::lock_guard<std::mutex> lock(s->stage_mtx);
+  const size_t N = s->N, NE = eng_count(s), ns = S ? 6 * N : 0;
+  const bool direct = export_bytes(s, ns) > kExportDirect;
+  double* h = (double*)stage(s, export_bytes(s, direct ? 0 : ns));
+  if (!h) return fail(SRS_ERR_NOMEM, "pinned staging allocation failed");
+  if (direct && !s->d_export) SRS_TRY(dev_alloc(s, &s->d_export, 6 * N));
+  ExportArgs a{};
+  a.N = s->N;
+  a.NR = s->NR;
+  a.NL = s->NL;
+  if (s->d.precision == SRS_FP64) {
+    a.S64 = s->d_S[0] + (size_t)r * 6 * N;
   } else {
-    SRS_CUDA(cudaMemcpy(CMh.data(), s->d_CM + r * NE, NE * sizeof(float4), cudaMemcpyDeviceToHost));
-    SRS_CUDA(cudaMemcpy(CIh.data(), s->d_CI + r * NE, NE * sizeof(float), cudaMemcpyDeviceToHost));
+    a.M = s->d_M[0] + r * NE;
+    a.I = s->d_I[0] + r * NE;
+    if (s->d_CMq) {
+      a.CMq = s->d_CMq + r * NE;
+      a.CIq = s->d_CIq + r * NE;
+    } else {
+      a.CM = s->d_CM + r * NE;
+      a.CI = s->d_CI + r * NE;
+    }
+    a.eng_of_ref = s->d_eng_of_ref;
+    // flags: an array of the plain engine, the last word of the resident
+    // engine's record halves
+    const bool plain = s->d.engine == SRS_ENGINE_PLAIN;
+    a.flags = plain ? s->a32.flags : reinterpret_cast<const uint32_t*>(s->ar.geo_b) + 3;
+    a.flag_stride = plain ? 1 : 4;
+    const RestValues& rv = s->rv;
+    const double rest[6] = {rv.ca0, rv.atp, rv.cmdn, rv.trpn, rv.csqn, rv.dye};
+    std::copy(rest, rest + 6, a.rest);
+    a.rest_ca_jsr = rv.ca0_jsr;
   }
-  const RestValues& rv = s->rv;
-  for (size_t e = 0; e < NE; ++e) {
-    int j = s->ref_of_eng[e];
-    if (j < 0) continue;
-    bool jsr = s->m.domain[j] == DOMAIN_JSR;
-    double f = jsr ? 0.0 : 1.0;
-    // compensated sum: the state is u - comp (the comp term holds the
-    // rounding error of the last update)
-    S6[SP_CA * (size_t)N + j] = s->rest_ca[e] + ((double)M[e].x - (double)CMh[e].x);
-    S6[SP_ATP * (size_t)N + j] = f * rv.atp + ((double)M[e].y - (double)CMh[e].y);
-    S6[SP_CMDN * (size_t)N + j] = f * rv.cmdn + ((double)M[e].z - (double)CMh[e].z);
-    S6[SP_DYE * (size_t)N + j] = f * rv.dye + ((double)M[e].w - (double)CMh[e].w);
-    double imm = s->rest_imm[e] + ((double)I[e] - (double)CIh[e]);
-    S6[SP_TRPN * (size_t)N + j] = jsr ? 0.0 : imm;
-    S6[SP_CSQN * (size_t)N + j] = jsr ? imm : 0.0;
-  }
+  a.ryr = s->d_ryr + (size_t)r * s->NR;
+  a.lcc = s->d_lcc + (size_t)r * s->NL;
+  a.lccv = s->d_lccv + (size_t)r * s->NL;
+  a.res = s->d_res + (size_t)r * s->NCH;
+  double* hres = h;
+  double* hS = hres + s->NCH;
+  int32_t* hi = reinterpret_cast<int32_t*>(hS + (direct ? 0 : ns));
+  a.S = S ? (direct ? s->d_export : hS) : nullptr;
+  a.res_out = res ? hres : nullptr;
+  a.ryr_out = ryr ? hi : nullptr;
+  a.lcc_out = lcc ? hi + s->NR : nullptr;
+  a.lccv_out = lccv ? hi + s->NR + s->NL : nullptr;
+  if (launch_export_state(a, s->st)) return fail(SRS_ERR_CUDA, "state export launch failed");
+  if (direct) SRS_CUDA(cudaMemcpyAsync(S, s->d_export, ns * sizeof(double), cudaMemcpyDeviceToHost, s->st));
+  SRS_CUDA(cudaStreamSynchronize(s->st));
+  if (S && !direct) std::memcpy(S, hS, ns * sizeof(double));
+  if (res) std::memcpy(res, hres, s->NCH * sizeof(double));
+  if (ryr) std::memcpy(ryr, hi, s->NR * sizeof(int32_t));
+  if (lcc) std::memcpy(lcc, hi + s->NR, s->NL * sizeof(int32_t));
+  if (lccv) std::memcpy(lccv, hi + s->NR + s->NL, s->NL * sizeof(int32_t));
   return SRS_OK;
+}
+
+// Error of a bounded wait that gave up; the barrier counters start afresh.
+int check_timeout(srs_sim* s) {
+  volatile unsigned* flag = reinterpret_cast<volatile unsigned*>(s->h_pin);
+  if (!flag || !*flag) return SRS_OK;
+  *flag = 0;
+  cudaMemsetAsync(s->loop.bar, 0, sizeof(unsigned) * s->R, s->st);
+  return fail(SRS_ERR_TIMEOUT, "a step's barrier did not complete");
+}
+
+// The plain engines' state buffers 0 and 1 change places.
+void swap_buffers(srs_sim* s) {
+  std::swap(s->d_S[0], s->d_S[1]);
+  std::swap(s->d_M[0], s->d_M[1]);
+  std::swap(s->d_I[0], s->d_I[1]);
+  std::swap(s->graph_plain, s->graph_plain_alt);
 }
 
 // After a run of the plain engines realization r's state sits in buffer
@@ -1122,8 +1167,13 @@ int normalize_buffers(srs_sim* s, const std::vector<int64_t>& steps_before) {
   std::vector<RealCtl> ctl(s->R);
   SRS_CUDA(cudaMemcpy(ctl.data(), s->d_ctl, sizeof(RealCtl) * s->R, cudaMemcpyDeviceToHost));
   const size_t N = s->N;
-  for (int r = 0; r < s->R; ++r)
-    if (ctl[r].status & 2u) return fail(SRS_ERR_TIMEOUT, "a step's barrier did not complete");
+  SRS_TRY(check_timeout(s));
+  int odd = 0;
+  for (int r = 0; r < s->R; ++r) odd += (int)((ctl[r].step - steps_before[r]) & 1);
+  if (odd == s->R) {  // the buffers change places
+    swap_buffers(s);
+    return SRS_OK;
+  }
   for (int r = 0; r < s->R; ++r) {
     if (((ctl[r].step - steps_before[r]) & 1) == 0) continue;
     if (s->d.precision == SRS_FP64) {
@@ -1184,6 +1234,10 @@ void refresh_args(srs_sim* s) {
     s->ar.I = s->d_I[0];
     s->ar.CM = s->d_CM;
     s->ar.CI = s->d_CI;
+  }
+  if (s->graph_plain_alt) {
+    cudaGraphExecDestroy(s->graph_plain_alt);
+    s->graph_plain_alt = nullptr;
   }
   if (s->graph_plain) {
     cudaGraphExecDestroy(s->graph_plain);
@@ -1281,7 +1335,7 @@ int setup_plain_loop(srs_sim* s) {
 int plain_loop_launch(srs_sim* s, int steps) {
   PlainLoop l = s->loop;
   l.steps = steps;
-  SRS_CUDA(cudaMemsetAsync(l.bar, 0, sizeof(unsigned) * s->R, s->st));
+  l.timeout = reinterpret_cast<unsigned*>(s->h_pin);
   int rc;
   if (s->d.precision == SRS_FP64) {
     Plain64Args a = s->a64;
@@ -1611,10 +1665,12 @@ int srs_sim_create(const srs_grid* g, const srs_params* ps, const srs_sim_desc* 
 void srs_sim_destroy(srs_sim* s) {
   if (!s) return;
   if (s->graph_plain) cudaGraphExecDestroy(s->graph_plain);
+  if (s->graph_plain_alt) cudaGraphExecDestroy(s->graph_plain_alt);
   if (s->st) cudaStreamSynchronize(s->st);
   for (void* p : s->allocs) cudaFree(p);
   for (auto& b : s->adj_bufs) cudaFree(b.first);
   if (s->h_stage) cudaFreeHost(s->h_stage);
+  if (s->h_pin) cudaFreeHost(s->h_pin);
   if (s->st) cudaStreamDestroy(s->st);
   delete s;
 }
@@ -1645,10 +1701,9 @@ int srs_sim_get_config(const srs_sim* s, srs_sim_config* c) {
   c->smem_bytes = (int)s->smem;
   c->kernel_launches = s->launches;
   const int64_t NE = (int64_t)eng_count(s);
-  const int64_t per_state = s->d.precision == SRS_FP64 ? (int64_t)6 * s->N * 8 : NE * 20;
   c->ctl_bytes = (int64_t)s->R * (int64_t)sizeof(RealCtl);
-  c->reset_h2d_bytes = (int64_t)s->R * (per_state + (int64_t)(s->NR + 2 * s->NL) * 4 +
-                                         (int64_t)s->NCH * 8) + c->ctl_bytes;
+  c->reset_h2d_bytes = (int64_t)s->R * ((int64_t)(s->NR + 2 * s->NL) * 4 + (int64_t)s->NCH * 8) +
+                       c->ctl_bytes;
   c->engine_elements = NE;
   return SRS_OK;
 }
@@ -1659,12 +1714,7 @@ int srs_sim_reset(srs_sim* s) {
   const srs_params& p = s->p;
   const int* I = p.ints;
   const double* Rr = p.reals;
-  std::vector<double> S6;
-  initial_states(m, p, &S6);
   const int NR = s->NR, NL = s->NL, NCH = s->NCH;
-  std::vector<int32_t> ryr((size_t)s->R * NR, 0), lcc((size_t)s->R * NL, 1), lccv((size_t)s->R * NL, 2);
-  std::vector<double> res((size_t)s->R * NCH);
-  std::vector<RealCtl> ctl(s->R);
   // The RyR hold of RunSimulation indexes RyR_States[INIT_RYR] under every
   // protocol (cpu/RunSimulation.cpp:540), so the index is checked always.
   if (I[I_INIT_RYR] != -1 && (I[I_INIT_RYR] < 0 || I[I_INIT_RYR] >= NR))
@@ -1672,10 +1722,27 @@ int srs_sim_reset(srs_sim* s) {
                                    "), must be -1 to ignore, or between 0 and the number of RyRs");
   if (I[I_FLAG_LCC] && (I[I_LCC_INDEX] < 0 || I[I_LCC_INDEX] >= NL))
     return fail(SRS_ERR_INPUT, "LCC trigger index out of range");
-  for (int r = 0; r < s->R; ++r) {
+  // resting Ca by domain, for the random choice below
+  auto ca_rest = [&](int j) { return m.domain[j] == DOMAIN_CYTO ? s->rv.ca0 : s->rv.ca0_jsr; };
+  // channel states, residuals and control blocks in one pinned buffer, the
+  // residuals' logarithms by up to eight host threads
+  const size_t n_ctl = s->R * sizeof(RealCtl), n_res = (size_t)s->R * NCH * sizeof(double),
+               n_ryr = (size_t)s->R * NR * sizeof(int32_t), n_lcc = (size_t)s->R * NL * sizeof(int32_t);
+  std::lock_guard<std::mutex> lock(s->stage_mtx);
+  SRS_CUDA(cudaStreamSynchronize(s->st));
+  check_timeout(s);  // a wait that gave up ends with the run that it was in
+  unsigned char* h = (unsigned char*)stage(s, n_ctl + n_res + n_ryr + 2 * n_lcc);
+  if (!h) return fail(SRS_ERR_NOMEM, "pinned staging allocation failed");
+  RealCtl* ctl = (RealCtl*)h;
+  double* res = (double*)(h + n_ctl);
+  int32_t *ryr = (int32_t*)(h + n_ctl + n_res), *lcc = ryr + (size_t)s->R * NR, *lccv = lcc + (size_t)s->R * NL;
+  auto one = [&](int r) {
     const uint64_t seed = s->seeds[r];
     int32_t* ry = &ryr[(size_t)r * NR];
     int32_t* lc = &lcc[(size_t)r * NL];
+    std::fill(ry, ry + NR, 0);
+    std::fill(lc, lc + NL, 1);
+    std::fill(&lccv[(size_t)r * NL], &lccv[(size_t)r * NL] + NL, 2);
     // initial channel opening (cpu/main.cpp:217-250)
     if (I[I_FLAG_LCC]) {
       lc[I[I_LCC_INDEX]] = 6;
@@ -1693,8 +1760,8 @@ int srs_sim_reset(srs_sim* s) {
           int j = m.ryr_nb[4 * i + k];
           if (j >= 0) (ry[j] ? no : nc)++;
         }
-        double ca_ss = S6[SP_CA * (size_t)m.N + m.ryr_ele[i]];
-        double phi = Rr[R_RYR_PHI_M] * S6[SP_CA * (size_t)m.N + m.ryr_jsr[i]] + Rr[R_RYR_PHI_B];
+        double ca_ss = ca_rest(m.ryr_ele[i]);
+        double phi = Rr[R_RYR_PHI_M] * ca_rest(m.ryr_jsr[i]) + Rr[R_RYR_PHI_B];
         double X = std::exp(0.5 * Rr[R_RYR_A_STAR] * (nc * Rr[R_RYR_EPS_CC] - no * Rr[R_RYR_EPS_OO]));
         rate[i] = X * phi * Rr[R_RYR_K_PLUS] * std::pow(ca_ss, Rr[R_RYR_ETA]);
         tot += rate[i];
@@ -1724,14 +1791,17 @@ int srs_sim_reset(srs_sim* s) {
     int n_open = 0;
     for (int i = 0; i < NR; ++i) n_open += ry[i];
     c.n_open_tick = n_open;
-  }
-  SRS_TRY(upload_state_range(s, 0, s->R, S6.data()));
-  SRS_CUDA(cudaMemcpy(s->d_ryr, ryr.data(), ryr.size() * 4, cudaMemcpyHostToDevice));
-  SRS_CUDA(cudaMemcpy(s->d_lcc, lcc.data(), lcc.size() * 4, cudaMemcpyHostToDevice));
-  SRS_CUDA(cudaMemcpy(s->d_lccv, lccv.data(), lccv.size() * 4, cudaMemcpyHostToDevice));
-  SRS_CUDA(cudaMemcpy(s->d_res, res.data(), res.size() * 8, cudaMemcpyHostToDevice));
-  SRS_CUDA(cudaMemcpy(s->d_ctl, ctl.data(), ctl.size() * sizeof(RealCtl), cudaMemcpyHostToDevice));
-  SRS_CUDA(cudaMemset(s->d_counters, 0, sizeof(unsigned) * s->R));
+  };
+  host_parallel(s->R, (size_t)s->R * NCH < 4096 ? 1 : 8, one);
+  SRS_TRY(reset_states(s));
+  SRS_CUDA(cudaMemcpyAsync(s->d_ctl, ctl, n_ctl, cudaMemcpyHostToDevice, s->st));
+  SRS_CUDA(cudaMemcpyAsync(s->d_res, res, n_res, cudaMemcpyHostToDevice, s->st));
+  SRS_CUDA(cudaMemcpyAsync(s->d_ryr, ryr, n_ryr, cudaMemcpyHostToDevice, s->st));
+  SRS_CUDA(cudaMemcpyAsync(s->d_lcc, lcc, n_lcc, cudaMemcpyHostToDevice, s->st));
+  SRS_CUDA(cudaMemcpyAsync(s->d_lccv, lccv, n_lcc, cudaMemcpyHostToDevice, s->st));
+  SRS_CUDA(cudaMemsetAsync(s->d_counters, 0, sizeof(unsigned) * s->R, s->st));
+  SRS_CUDA(cudaStreamSynchronize(s->st));
+  s->finished = false;
   return SRS_OK;
 }
 
@@ -1748,13 +1818,7 @@ int srs_sim_set_state(srs_sim* s, int r, const double* states, const int* ryr, c
 
 int srs_sim_get_state(srs_sim* s, int r, double* states, int* ryr, int* lcc, int* lccv, double* res) {
   if (!s || r < 0 || r >= s->R) return fail(SRS_ERR_INPUT, "bad realization index");
-  SRS_CUDA(cudaStreamSynchronize(s->st));
-  if (states) SRS_TRY(download_state(s, r, states));
-  if (ryr) SRS_CUDA(cudaMemcpy(ryr, s->d_ryr + (size_t)r * s->NR, s->NR * 4, cudaMemcpyDeviceToHost));
-  if (lcc) SRS_CUDA(cudaMemcpy(lcc, s->d_lcc + (size_t)r * s->NL, s->NL * 4, cudaMemcpyDeviceToHost));
-  if (lccv) SRS_CUDA(cudaMemcpy(lccv, s->d_lccv + (size_t)r * s->NL, s->NL * 4, cudaMemcpyDeviceToHost));
-  if (res) SRS_CUDA(cudaMemcpy(res, s->d_res + (size_t)r * s->NCH, s->NCH * 8, cudaMemcpyDeviceToHost));
-  return SRS_OK;
+  return export_state(s, r, states, ryr, lcc, lccv, res);
 }
 
 int srs_sim_set_globals(srs_sim* s, double v_m, double ca_nsr) {
@@ -1768,12 +1832,21 @@ int srs_sim_set_globals(srs_sim* s, double v_m, double ca_nsr) {
 
 int srs_explicit_step(srs_sim* s, int64_t n_steps) {
   if (!s || n_steps < 0) return fail(SRS_ERR_INPUT, "bad argument");
-  std::vector<int64_t> before = ctl_steps(s);
-  s->P.run_protocol = 0;
-  refresh_args(s);
+  if (s->P.run_protocol) {
+    s->P.run_protocol = 0;
+    refresh_args(s);
+  }
+  const bool plain = s->d.engine != SRS_ENGINE_RESIDENT;
+  // Realizations that may finish one by one leave their buffers at different
+  // parities; the others take the same steps, n or (finished) none.
+  const bool uneven = plain && s->p.ints[I_FLAG_FIDELITY_SIM];
+  std::vector<int64_t> before;
+  if (uneven) before = ctl_steps(s);
   SRS_TRY(advance(s, n_steps));
   SRS_CUDA(cudaStreamSynchronize(s->st));
-  SRS_TRY(normalize_buffers(s, before));
+  if (uneven) return normalize_buffers(s, before);
+  SRS_TRY(check_timeout(s));
+  if (plain && !s->finished && (n_steps & 1)) swap_buffers(s);
   return SRS_OK;
 }
 
@@ -1861,7 +1934,9 @@ int run_finish(srs_sim* s, srs_run_output* out, const std::vector<int64_t>& befo
   SRS_CUDA(cudaMemcpy(out->rows, s->d_rows, (size_t)s->R * out->row_capacity * rw * sizeof(float),
                       cudaMemcpyDeviceToHost));
   int st_bits = 0;
+  s->finished = true;
   for (int r = 0; r < s->R; ++r) {
+    s->finished = s->finished && ctl[r].done;
     if (out->n_rows) out->n_rows[r] = ctl[r].n_rows;
     if (out->t_end) out->t_end[r] = ctl[r].t;
     if (out->n_steps) out->n_steps[r] = ctl[r].step;
@@ -3293,9 +3368,8 @@ int srs_sim_total_ca(srs_sim* s, double* out) {
 int srs_write_grid_vtk(srs_sim* s, int r, const char* path, int run, int rank, int n, double t) {
   if (!s || !path || r < 0 || r >= s->R) return fail(SRS_ERR_INPUT, "bad argument");
   std::vector<double> S6((size_t)6 * s->N);
-  SRS_TRY(download_state(s, r, S6.data()));
   std::vector<int32_t> ryr(s->NR);
-  SRS_CUDA(cudaMemcpy(ryr.data(), s->d_ryr + (size_t)r * s->NR, s->NR * 4, cudaMemcpyDeviceToHost));
+  SRS_TRY(export_state(s, r, S6.data(), ryr.data(), nullptr, nullptr, nullptr));
   return write_grid_vtk(path, s->m, run, rank, n, t, &S6[0], &S6[(size_t)SP_DYE * s->N], ryr.data());
 }
 

@@ -126,7 +126,8 @@ struct PlainLoop {
   int32_t blocks;         // element blocks per realization
   int32_t per_thread;     // elements a thread (FP64: a lane of each of four warps) takes
   int32_t n_sm;
-  unsigned* bar;          // [R] arrivals at the step barriers, zero before the launch
+  unsigned* bar;          // [R] arrivals at the step barriers, zero before and after a launch
+  unsigned* timeout;      // pinned host word: set when a wait gave up
   int32_t ch_max;         // most channels an element block gates
   const int32_t* ch_ptr;  // [blocks + 1] CSR of the channels each block gates
   const int32_t* ch_id;   // RyR, or NR + LCC
@@ -233,6 +234,29 @@ constexpr int LINESCAN_CHUNK = 64;
 constexpr int LINESCAN_TILE_R = 16;
 int linescan_splits(int n_samples, int n_state, int R, int n_sm);
 int launch_linescan(const LinescanArgs& a, int R, cudaStream_t st);
+
+// ---- state exchange (k_state.cu) ----------------------------------------------
+struct ExportArgs {
+  int32_t N, NR, NL;
+  const double* S64;            // FP64 engine: the realization's state [6][N]; or the FP32 engines':
+  const float4* M;              // the realization's arrays in engine order
+  const float* I;
+  const float4* CM;
+  const float* CI;
+  const ushort4* CMq;           // (compensation compact, when set)
+  const uint16_t* CIq;
+  const int32_t* eng_of_ref;    // [N]
+  const uint32_t* flags;        // bit 0 JSR, bit 1 troponin C, by engine element
+  int32_t flag_stride;          // words between elements' flags
+  double rest[6], rest_ca_jsr;  // Ca (cytosol), ATP, CMDN, TRPN, CSQN, dye; Ca (JSR)
+  const int32_t *ryr, *lcc, *lccv;
+  const double* res;
+  double* S;                    // outputs (null: not wanted)
+  int32_t *ryr_out, *lcc_out, *lccv_out;
+  double* res_out;
+};
+int launch_export_state(const ExportArgs& a, cudaStream_t st);
+int launch_broadcast_state(const double* src, double* dst, size_t n, int R, cudaStream_t st);
 
 // ---- total Ca per compartment (k_mass.cu) ------------------------------------
 struct MassArgs {
