@@ -29,6 +29,7 @@
 #include "srs_adjoint.cuh"
 #include "srs_engine.h"
 #include "srs_fp32_update.cuh"
+#include "srs_pdl.cuh"
 #include "srs_protocol.cuh"
 
 namespace srs {
@@ -36,18 +37,28 @@ namespace srs {
 // ===========================================================================
 // Plain FP32 engine
 // ===========================================================================
+// What an element's step reads of the mesh alone.
+struct PlainGeo {
+  float4 a;
+  int4 nb;
+  uint32_t fl;
+};
+__device__ __forceinline__ PlainGeo plain32_geometry(const Plain32Args& a, int j) {
+  return PlainGeo{__ldg(a.a + j), __ldg(a.nb + j), __ldg(a.flags + j)};
+}
+
 // One element of one realization: release flux of its channels, then the
 // FP32 update (tet_update).  TRAJ: also record the state the step starts
 // from and the Ca rate (the adjoint's trajectory).
 template <bool TRAJ>
-__device__ __forceinline__ void plain32_element(const Plain32Args& a, int r, int j) {
+__device__ __forceinline__ void plain32_element(const Plain32Args& a, int r, int j, const PlainGeo& geo) {
   RealCtl* ctlp = a.CS.ctl + r;
   const int N = a.N;
   const float4* M = a.M_in + (size_t)r * N;
   const float* I = a.I_in + (size_t)r * N;
   float4* Mo = a.M_out + (size_t)r * N;
   float* Io = a.I_out + (size_t)r * N;
-  const uint32_t fl = a.flags[j];
+  const uint32_t fl = geo.fl;
   {
     float flux = 0.0f;
     if (fl & 4u) {
@@ -70,7 +81,7 @@ __device__ __forceinline__ void plain32_element(const Plain32Args& a, int r, int
         flux = fmaf(J, e.s, flux);
       }
     }
-    const int4 nb = a.nb[j];
+    const int4 nb = geo.nb;
     const size_t o = (size_t)r * N + j;
     const float4 x = M[j];
     const float im = I[j];
@@ -87,13 +98,13 @@ __device__ __forceinline__ void plain32_element(const Plain32Args& a, int r, int
     float imo;
     if constexpr (TRAJ) {
       float g;
-      tet_update(a.k, x, im, M[nb.x], M[nb.y], M[nb.z], M[nb.w], a.a[j], fl, a.bsl[j],
+      tet_update(a.k, x, im, M[nb.x], M[nb.y], M[nb.z], M[nb.w], geo.a, fl, a.bsl[j],
                  a.kb ? a.kb[j] : 0.0f, flux, cm, ci, &out, &imo, &g);
       a.traj_u[o] = x;
       a.traj_ig[o] = make_float2(im, g);
       a.traj_ib[o] = sl_inv_factor(a.k, a.bsl[j], ((fl & 1u) ? a.k.c0j : a.k.c0) + x.x);
     } else {
-      tet_update(a.k, x, im, M[nb.x], M[nb.y], M[nb.z], M[nb.w], a.a[j], fl, a.bsl[j],
+      tet_update(a.k, x, im, M[nb.x], M[nb.y], M[nb.z], M[nb.w], geo.a, fl, a.bsl[j],
                  a.kb ? a.kb[j] : 0.0f, flux, cm, ci, &out, &imo);
     }
     Mo[j] = out;
@@ -159,10 +170,13 @@ __device__ __forceinline__ void plain32_gate(const Plain32Args& a, int r, int32_
 template <bool TRAJ>
 __global__ void __launch_bounds__(256) k_plain32_step(Plain32Args a) {
   const int r = blockIdx.x;
-  if (a.CS.ctl[r].done) return;
   const int j = blockIdx.y * blockDim.x + threadIdx.x;
-  const uint32_t fl = j < a.N ? a.flags[j] : 0u;
-  if (j < a.N) plain32_element<TRAJ>(a, r, j);
+  PlainGeo geo = plain32_geometry(a, min(j, a.N - 1));
+  pdl_wait();
+  pdl_next();
+  if (a.CS.ctl[r].done) return;
+  const uint32_t fl = j < a.N ? geo.fl : 0u;
+  if (j < a.N) plain32_element<TRAJ>(a, r, j, geo);
   __shared__ int s_last;
   __shared__ int32_t s_nb[1024];
   // The last block of the realization gates its channels from the new Ca of
@@ -187,6 +201,10 @@ __global__ void __launch_bounds__(256) k_plain32_step(Plain32Args a) {
 template <bool TRAJ>
 __global__ void __launch_bounds__(256, 6) k_plain32_update(Plain32Args a) {
   const int r = blockIdx.x;
+  const int j = blockIdx.y * blockDim.x + threadIdx.x;
+  const PlainGeo geo = plain32_geometry(a, min(j, a.N - 1));
+  pdl_wait();
+  pdl_next();
   if (a.CS.ctl[r].done) return;
   if (threadIdx.x == 0 && a.pf_rows > 0 && blockIdx.y + a.pf_rows < gridDim.y) {
     const size_t e0 = (size_t)(blockIdx.y + a.pf_rows) * blockDim.x;
@@ -202,16 +220,87 @@ __global__ void __launch_bounds__(256, 6) k_plain32_update(Plain32Args a) {
       prefetch_span(a.CI + o, n * sizeof(float));
     }
   }
-  const int j = blockIdx.y * blockDim.x + threadIdx.x;
-  if (j < a.N) plain32_element<TRAJ>(a, r, j);
+  if (j < a.N) plain32_element<TRAJ>(a, r, j, geo);
 }
 
+// Gating and the next step's protocol after k_plain32_update.  The kernel is a
+// chain of latencies (one block a realization): with the channels' elements read
+// before the wait, a state read is one round trip, RyR and LCC side by side.
 template <bool TRAJ>
 __global__ void __launch_bounds__(256) k_plain32_gate(Plain32Args a) {
-  const int r = blockIdx.x;
-  if (a.CS.ctl[r].done) return;
+  const int r = blockIdx.x, NR = a.C.NR, NL = a.C.NL;
   __shared__ int32_t s_nb[1024];
-  plain32_gate<TRAJ>(a, r, s_nb);
+  const int i0 = threadIdx.x;
+  int e0 = 0, e1 = 0;
+  float rest0 = 0.0f, rest1 = 0.0f;
+  auto elements = [&](int i) {
+    e0 = i < NR ? a.C.ryr_cleft[i] : a.C.lcc_ele[i - NR];
+    e1 = i < NR ? a.C.ryr_jsr[i] : e0;
+    rest0 = a.rest_ca[e0];
+    rest1 = a.rest_ca[e1];
+  };
+  if (i0 < NR + NL) elements(i0);
+  pdl_wait();
+  pdl_next();
+  RealCtl* ctlp = a.CS.ctl + r;
+  if (ctlp->done) return;
+  if (a.P.gc[0].ryr_astar_half != 0.0f || a.P.gc[1].ryr_astar_half != 0.0f) {  // coupled gating
+    plain32_gate<TRAJ>(a, r, s_nb);
+    return;
+  }
+  const float4* M = a.M_out + (size_t)r * a.N;
+  int32_t* ryr = a.CS.ryr + (size_t)r * NR;
+  int32_t* lcc = a.CS.lcc + (size_t)r * NL;
+  int32_t* lccv = a.CS.lccv + (size_t)r * NL;
+  double* res = a.CS.res + (size_t)r * (NR + NL);
+  const int vsel = ctlp->vsel;
+  const uint64_t seed = ctlp->seed;
+  const int64_t step = ctlp->step;
+  const srs_gate_consts* g = &a.P.gc[vsel];
+  int32_t* rec = nullptr;
+  if constexpr (TRAJ) {
+    rec = a.traj_ch + (size_t)r * (NR + 2 * NL + 1);
+    if (threadIdx.x == 0) rec[NR + 2 * NL] = vsel;
+  }
+  for (int i = i0; i < NR + NL; i += blockDim.x) {
+    if (i != i0) elements(i);
+    const float c0 = rest0 + M[e0].x, c1 = rest1 + M[e1].x;
+    double q = res[i];
+    if (i < NR) {
+      const int open = ryr[i];
+      if constexpr (TRAJ) rec[i] = open;
+      if (!a.P.nogating) {
+        ryr[i] = srs_gate_ryr(g, open, c0, c1, 0, 0, &q, seed, (uint32_t)i, (uint64_t)step);
+        res[i] = q;
+      }
+    } else {
+      int st = lcc[i - NR], vs = lccv[i - NR];
+      if constexpr (TRAJ) {
+        rec[i] = st;
+        rec[NL + i] = vs;
+      }
+      if (!a.P.nogating) {
+        srs_gate_lcc(g, &st, &vs, c0, &q, seed, (uint32_t)i, (uint64_t)step);
+        lcc[i - NR] = st;
+        lccv[i - NR] = vs;
+        res[i] = q;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (a.P.run_protocol) {
+      RealCtl ctl = *ctlp;
+      ctl.step += 1;
+      ctl.t += a.P.dt;
+      prestep(a.P, a.C, ctl, ryr, lcc, lccv, a.CS.rows + (size_t)r * a.P.row_cap * a.P.row_w,
+              [&](int e) -> double { return (double)(a.rest_ca[e] + M[e].x); });
+      *ctlp = ctl;
+    } else {
+      ctlp->step = step + 1;
+      ctlp->t += a.P.dt;
+    }
+  }
 }
 
 __global__ void k_plain32_prestep(Plain32Args a, int write_initial_row) {
@@ -235,22 +324,17 @@ int launch_plain32_step(const Plain32Args& a, cudaStream_t st) {
   if ((a.N + 255) / 256 > 65535) return -1;  // grid y limit: 16.7 M elements
   dim3 grid(a.R, (a.N + 255) / 256);
   const bool traj = a.traj_u != nullptr;
+  cudaError_t e;
   if (a.N >= PLAIN32_SPLIT_N) {
-    if (traj) {
-      k_plain32_update<true><<<grid, 256, 0, st>>>(a);
-      k_plain32_gate<true><<<a.R, 256, 0, st>>>(a);
-    } else {
-      k_plain32_update<false><<<grid, 256, 0, st>>>(a);
-      k_plain32_gate<false><<<a.R, 256, 0, st>>>(a);
-    }
+    e = launch_pdl(traj ? k_plain32_update<true> : k_plain32_update<false>, grid, 256, 0, st, a);
+    if (e == cudaSuccess) e = launch_pdl(traj ? k_plain32_gate<true> : k_plain32_gate<false>, a.R, 256, 0, st, a);
   } else {
     // few realizations: 64-thread blocks spread the step over more SMs
     const int bs = (size_t)((a.N + 255) / 256) * a.R < 304 ? 64 : 256;
     const dim3 g2(a.R, (a.N + bs - 1) / bs);
-    if (traj) k_plain32_step<true><<<g2, bs, 0, st>>>(a);
-    else k_plain32_step<false><<<g2, bs, 0, st>>>(a);
+    e = launch_pdl(traj ? k_plain32_step<true> : k_plain32_step<false>, g2, bs, 0, st, a);
   }
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  return e == cudaSuccess ? 0 : -1;
 }
 int launch_plain32_prestep(const Plain32Args& a, int write_initial_row, cudaStream_t st) {
   k_plain32_prestep<<<a.R, 32, 0, st>>>(a, write_initial_row);

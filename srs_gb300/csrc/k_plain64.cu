@@ -15,6 +15,7 @@
 #include <cmath>
 
 #include "srs_engine.h"
+#include "srs_pdl.cuh"
 #include "srs_plain64_update.cuh"
 #include "srs_protocol.cuh"
 
@@ -89,6 +90,8 @@ __device__ __forceinline__ void plain64_tail(const Plain64Args& a, int r, const 
 }
 
 __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
+  pdl_wait();
+  pdl_next();
   const int r = blockIdx.y;
   RealCtl* ctlp = a.CS.ctl + r;
   if (ctlp->done) return;  // uniform per realization
@@ -170,6 +173,8 @@ template <bool KEYS>
 __global__ void __launch_bounds__(128) k_plain64_split(const __grid_constant__ Plain64Args a,
                                                        const __grid_constant__ Plain64Keys<KEYS> keys) {
   __shared__ double s_rate[5][32];
+  pdl_wait();
+  pdl_next();
   const int r = blockIdx.y;
   RealCtl ctl{};
   unsigned* status;
@@ -255,18 +260,19 @@ static void launch_step64(const Plain64Args& a, cudaStream_t st) {
   // few realizations: 64-thread blocks spread the element updates (and their
   // FP64 arithmetic) over more SMs than 256-thread blocks would
   const int bs = (size_t)((a.N + 255) / 256) * a.R < 304 ? 64 : 256;
-  k_plain64_step<<<dim3((a.N + bs - 1) / bs, a.R), bs, 0, st>>>(a);
+  launch_pdl(k_plain64_step, dim3((a.N + bs - 1) / bs, a.R), bs, 0, st, a);
 }
 
 int launch_plain64_step(const Plain64Args& a, cudaStream_t st) {
-  if (split64(a)) k_plain64_split<false><<<dim3((a.N + 31) / 32, a.R), 128, 0, st>>>(a, {});
+  if (split64(a))
+    launch_pdl(k_plain64_split<false>, dim3((a.N + 31) / 32, a.R), 128, 0, st, a, Plain64Keys<false>{});
   else launch_step64(a, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 bool plain64_keys_fit(const Plain64Args& a) { return split64(a); }
 int launch_plain64_keys(const Plain64Args& a, const Plain64Keys<true>& k, cudaStream_t st) {
-  k_plain64_split<true><<<dim3((a.N + 31) / 32, a.R), 128, 0, st>>>(a, k);
+  launch_pdl(k_plain64_split<true>, dim3((a.N + 31) / 32, a.R), 128, 0, st, a, k);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 int launch_plain64_prestep(const Plain64Args& a, int write_initial_row, cudaStream_t st) {
