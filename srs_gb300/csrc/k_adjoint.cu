@@ -90,8 +90,15 @@ __device__ __forceinline__ float tick_injection(const AdjArgs& a, const double* 
 // storage during the segment) and lambda_Ca / B(x_{n-2}), with the tick
 // injection of step n-1 already added.  The last step writes lambda_{s0}
 // back to the global arrays for the next segment.
+//
+// A step waits on shared memory and on its own chains, so warps count: 640
+// threads of 96 registers, reading an element's record when they come to it,
+// against 512 of 128 that read it one element ahead (64 x 10,368 elements, 512
+// steps: 6.7 against 7.7 ms; 800 threads of 80 registers spill: 8.5).  The species
+// are computed in packed pairs (adj_local) and interior elements' codes are
+// offsets in this CTA (no look-up of the owner's window): 5 % together.
 template <int C>
-__global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
+__global__ void __launch_bounds__(640, 1) k_adjoint32(AdjArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int P = a.P;           // stride of the forward engine's partitions
   const int msub = a.m_sub;    // forward partitions per CTA
@@ -240,9 +247,8 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
     // per-warp FP64 accumulators of this realization's gradient
     for (int q = tid; q < nw * NA; q += nthr) red[q] = 0.0;
     int cur = 0;
-    float gstep[NA];  // this thread's contributions of the last few steps (FP32)
-#pragma unroll
-    for (int p = 0; p < NA; ++p) gstep[p] = 0.0f;
+    AdjGrad gstep;  // this thread's contributions of the last few steps (FP32)
+    gstep.clear();
     // barrier phases: the arrive after the publication of step t's slots is
     // waited on after the interior elements of step t, whose neighbours'
     // slots all live in this CTA (the __syncthreads orders those)
@@ -269,8 +275,7 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
       }
       return sp;
     };
-    // the element's record and trajectory, loaded one element ahead (and,
-    // for a thread's first element, during the previous step)
+    // the element's record and trajectory
     struct Pre {
       float4 at, gb, x;
       float2 ig;
@@ -285,13 +290,12 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
       q.cp = t > 1 ? sp.cprev[i].x : 0.0f;
       return q;
     };
-    Pre first = {};
-    bool have_first = false;
     for (int t = len; t >= 1; --t) {
       const int64_t n = a.s0 + t;  // this step maps x_{n-1} to x_n
       const float4* pub = cur ? pub1 : pub0;
       float4* nxt = cur ? pub0 : pub1;
       const uint32_t* bs = s_base + 16 * cur;
+      const uint32_t pub_local = smem_addr(pub);
       const int32_t* rec = a.traj_ch + ((size_t)(t - 1) * a.R + r) * W;
       const double* coef_next = t > 1 ? tick_coef(a, n - 1, r) : nullptr;
       if (a.stage) {
@@ -310,8 +314,9 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
       }
       const StepPtr sp = step_ptrs(t);
 
-      // OWN: the owner state of lambda is in shared memory (else global)
-      auto element = [&](int i, const Pre& pre, auto own) {
+      // OWN: the owner state of lambda is in shared memory (else global);
+      // local: an interior element, whose codes carry no rank
+      auto element = [&](int i, const Pre& pre, auto own, auto local) {
         constexpr bool OWN = decltype(own)::value;
         float lx, li, ci;
         if constexpr (OWN) {
@@ -342,38 +347,22 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
           n1 = ld_smem_f4(bs[0] + c1 * 16u);
           n2 = ld_smem_f4(bs[0] + c2 * 16u);
           n3 = ld_smem_f4(bs[0] + c3 * 16u);
+        } else if constexpr (decltype(local)::value) {
+          n0 = ld_smem_f4(pub_local + c0 * 16u);
+          n1 = ld_smem_f4(pub_local + c1 * 16u);
+          n2 = ld_smem_f4(pub_local + c2 * 16u);
+          n3 = ld_smem_f4(pub_local + c3 * 16u);
         } else {
           n0 = ld_dsmem_f4(bs[c0 >> a.off_bits] + (c0 & mask) * 16u);
           n1 = ld_dsmem_f4(bs[c1 >> a.off_bits] + (c1 & mask) * 16u);
           n2 = ld_dsmem_f4(bs[c2 >> a.off_bits] + (c2 & mask) * 16u);
           n3 = ld_dsmem_f4(bs[c3 >> a.off_bits] + (c3 & mask) * 16u);
         }
-        // transposed diffusion: S = sum_k aT_k lambda(nb_k) - (sum_k a_k) lambda(self)
-        float Sc = at.x * n0.x;
-        Sc = fmaf(at.y, n1.x, Sc);
-        Sc = fmaf(at.z, n2.x, Sc);
-        Sc = fmaf(at.w, n3.x, Sc);
-        Sc = fmaf(-sa, me.x, Sc);
-        float Sa = at.x * n0.y;
-        Sa = fmaf(at.y, n1.y, Sa);
-        Sa = fmaf(at.z, n2.y, Sa);
-        Sa = fmaf(at.w, n3.y, Sa);
-        Sa = fmaf(-sa, me.y, Sa);
-        float Sm = at.x * n0.z;
-        Sm = fmaf(at.y, n1.z, Sm);
-        Sm = fmaf(at.z, n2.z, Sm);
-        Sm = fmaf(at.w, n3.z, Sm);
-        Sm = fmaf(-sa, me.z, Sm);
-        float Sy = at.x * n0.w;
-        Sy = fmaf(at.y, n1.w, Sy);
-        Sy = fmaf(at.z, n2.w, Sy);
-        Sy = fmaf(at.w, n3.w, Sy);
-        Sy = fmaf(-sa, me.w, Sy);
-        float* g = gstep;  // this element's terms go straight into the thread's sums
+        AdjGrad& g = gstep;  // this element's terms go straight into the thread's sums
         const float w = me.x;
-        const AdjTerms lt = adj_local(k, ak, x, xim, me, li, jsr, trpn, Sc, Sa, Sm, Sy, g);
-        float oc = lt.oc, dG = lt.dG;
-        const float oa = lt.oa, om = lt.om, oy = lt.oy, oi = lt.oi, c = lt.c;
+        const AdjTerms lt = adj_local(k, ak, x, xim, me, li, jsr, trpn, at, sa, n0, n1, n2, n3, g);
+        float oc = lt.oxy.x, dG = lt.dG;
+        const float c = lt.c;
         if (i < n_ch) {
           // channel elements and their RyR partners all sit in partition 0
           for (int q = s_cptr[i]; q < s_cptr[i + 1]; ++q) {
@@ -387,7 +376,7 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
                 if (e.kind == 0) {
                   oc = fmaf(-k.jr_scale, qv, oc);
                   const float cj = k.c0j + sp.tu[oc_code & ch_mask].x;
-                  g[SRS_ADJ_V_RYR] = fmaf(qv * ak.v_cell, cj - c, g[SRS_ADJ_V_RYR]);
+                  g.v_ryr = fmaf(qv * ak.v_cell, cj - c, g.v_ryr);
                 } else {
                   oc = fmaf(k.jr_scale, qv, oc);
                 }
@@ -400,13 +389,14 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
         }
         adj_rapid(k, ak, bsl, c, G, w, dG, oc, g);
         // compensated update of lambda
-        float4 L = make_float4(lx, me.y, me.z, me.w);
+        const float2 ndt = p_bc(-k.dt);
+        float2 Lxy = make_float2(lx, me.y), Lzw = hi2(me), cxy = lo2(cm), czw = hi2(cm);
         float lnew = li;
-        kadd(L.x, cm.x, k.dt * oc);
-        kadd(L.y, cm.y, k.dt * oa);
-        kadd(L.z, cm.z, k.dt * om);
-        kadd(L.w, cm.w, k.dt * oy);
-        kadd(lnew, ci, k.dt * oi);
+        kadd(Lxy, cxy, ndt, make_float2(oc, lt.oxy.y));
+        kadd(Lzw, czw, ndt, lt.ozw);
+        kadd(lnew, ci, -k.dt, lt.oi);
+        const float4 L = make_float4(Lxy.x, Lxy.y, Lzw.x, Lzw.y);
+        cm = make_float4(cxy.x, cxy.y, czw.x, czw.y);
         if (t > 1) {
           const float cprev = (jsr ? k.c0j : k.c0) + pre.cp;
           const float inj = tick_injection(a, coef_next, (int)(rank * Pc + i));
@@ -427,47 +417,32 @@ __global__ void __launch_bounds__(512, 1) k_adjoint32(AdjArgs a) {
           a.lam_cim[roff + i] = ci;
         }
       };
-      auto element_s = [&](int i, const Pre& q) { element(i, q, std::true_type{}); };
-      auto element_g = [&](int i, const Pre& q) { element(i, q, std::false_type{}); };
-      // the schedule in two phases around the cluster wait; the loads of a
-      // thread's next element are issued before its current one is computed
-      auto sweep = [&](auto&& f) {
+      // the schedule in two phases around the cluster wait
+      auto sweep = [&](auto own) {
         int q = tid;
-        Pre p = first;
-        if (!have_first && q < n_sched) p = preload(sched[q], sp, t);
-        auto run = [&](int end) {
+        auto run = [&](int end, auto local) {
           for (; q < end; q += nthr) {
-            Pre nx = p;
-            if (q + nthr < n_sched) nx = preload(sched[q + nthr], sp, t);
-            f((int)sched[q], p);
-            p = nx;
+            const int i = sched[q];
+            const Pre p = preload(i, sp, t);
+            element(i, p, own, local);
           }
         };
-        run(n_pre);
+        run(n_pre, std::true_type{});
         cl_wait<C>();
-        run(n_sched);
+        run(n_sched, std::false_type{});
       };
-      if (a.own_in_smem) sweep(element_s);
-      else sweep(element_g);
-      // the first element of the next step (its trajectory slot is resident
-      // without staging; staged slots are waited on at the step's start)
-      have_first = false;
-      if (!a.stage && t > 1 && tid < n_sched) {
-        first = preload(sched[tid], step_ptrs(t - 1), t - 1);
-        have_first = true;
-      }
+      if (a.own_in_smem) sweep(std::true_type{});
+      else sweep(std::false_type{});
       __syncthreads();
       cl_arrive<C>();
       // every 16 steps (and at the end) the warp's FP32 sums go into its FP64
       // accumulators: the long sum over the steps runs in double precision
       if (((t - 1) & 15) == 0) {
-#pragma unroll
-        for (int p = 0; p < NA; ++p) {
-          float v = gstep[p];
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) red[warp * NA + p] += (double)v;
-          gstep[p] = 0.0f;
-        }
+        float sums[NA];
+        gstep.get(sums);
+        const float v = warp_sums<NA>(sums, lane);
+        if (lane < NA) red[warp * NA + lane] += (double)v;
+        gstep.clear();
       }
       cur ^= 1;
     }

@@ -42,28 +42,6 @@ __device__ __forceinline__ float plain_injection(const AdjPlainArgs& a, const do
   return (float)inj;
 }
 
-// Sums of N values over the warp: lane p returns the sum of value p (lanes from N
-// on: anything).  Each exchange halves the values a lane carries, 19 shuffles
-// for 18 values instead of five a value; the sum of each value is taken over the
-// same tree (lanes 16, 8, 4, 2, 1 apart), so it is the same number.
-template <int N>
-__device__ __forceinline__ float warp_sums(const float (&g)[N], int lane) {
-  float v[32];
-#pragma unroll
-  for (int p = 0; p < 32; ++p) v[p] = p < N ? g[p] : 0.0f;
-#pragma unroll
-  for (int h = 16; h >= 1; h >>= 1) {
-    const bool up = (lane & h) != 0;
-#pragma unroll
-    for (int p = 0; p < h; ++p) {
-      if (p >= N) continue;  // nothing in either half
-      const float keep = up ? v[p + h] : v[p], give = up ? v[p] : v[p + h];
-      v[p] = keep + __shfl_xor_sync(0xffffffffu, give, h);
-    }
-  }
-  return v[0];
-}
-
 }  // namespace
 
 // Start of a segment: publish lambda_{s1} (with the tick injection of step
@@ -97,9 +75,8 @@ __global__ void __launch_bounds__(ADJP_THREADS, 4) k_adjp_step(AdjPlainArgs a) {
   const int NR = a.NR, NL = a.NL, W = NR + 2 * NL + 1;
   const int32_t* rec = a.rec + (size_t)r * W;
   const double* coef = a.coef_next ? a.coef_next + (size_t)r * a.n_samples : nullptr;
-  float g[NA];
-#pragma unroll
-  for (int p = 0; p < NA; ++p) g[p] = 0.0f;
+  AdjGrad g;
+  g.clear();
   const int j0 = blockIdx.y * blockDim.x + threadIdx.x, stride = gridDim.y * blockDim.x;
   int4 nb_next = a.nb[min(j0, a.N - 1)];  // one element ahead: the slots' addresses
   pdl_wait();
@@ -121,41 +98,20 @@ __global__ void __launch_bounds__(ADJP_THREADS, 4) k_adjp_step(AdjPlainArgs a) {
     float lx = a.lam_c[o], li = a.lam_im[o];
     float4 cm = comp_load4_x2(a.lam_c4q + o);
     float ci = comp_load1(a.lam_cimq[o]);
-    // transposed diffusion: S = sum_k aT_k lambda(nb_k) - (sum_k a_k + kb) lambda(self)
-    float Sc = at.x * n0.x;
-    Sc = fmaf(at.y, n1.x, Sc);
-    Sc = fmaf(at.z, n2.x, Sc);
-    Sc = fmaf(at.w, n3.x, Sc);
-    Sc = fmaf(-sa, me.x, Sc);
-    float Sa = at.x * n0.y;
-    Sa = fmaf(at.y, n1.y, Sa);
-    Sa = fmaf(at.z, n2.y, Sa);
-    Sa = fmaf(at.w, n3.y, Sa);
-    Sa = fmaf(-sa, me.y, Sa);
-    float Sm = at.x * n0.z;
-    Sm = fmaf(at.y, n1.z, Sm);
-    Sm = fmaf(at.z, n2.z, Sm);
-    Sm = fmaf(at.w, n3.z, Sm);
-    Sm = fmaf(-sa, me.z, Sm);
-    float Sy = at.x * n0.w;
-    Sy = fmaf(at.y, n1.w, Sy);
-    Sy = fmaf(at.z, n2.w, Sy);
-    Sy = fmaf(at.w, n3.w, Sy);
-    Sy = fmaf(-sa, me.w, Sy);
     const float w = me.x;
-    const AdjTerms lt = adj_local(k, ak, x, ig.x, me, li, jsr, trpn, Sc, Sa, Sm, Sy, g);
-    float oc = lt.oc, dG = lt.dG;
+    const AdjTerms lt = adj_local(k, ak, x, ig.x, me, li, jsr, trpn, at, sa, n0, n1, n2, n3, g);
+    float oc = lt.oxy.x, dG = lt.dG;
     const float c = lt.c;
     if (a.kb) {
       // the Dirichlet source of the mobile buffers (their resting bound level)
       const float kbj = a.kb[j];
       if (kbj != 0.0f) {
-        g[SRS_ADJ_K_ON_DYE] = fmaf(me.w * kbj, ak.kb_on[0], g[SRS_ADJ_K_ON_DYE]);
-        g[SRS_ADJ_K_OFF_DYE] = fmaf(me.w * kbj, ak.kb_off[0], g[SRS_ADJ_K_OFF_DYE]);
-        g[SRS_ADJ_K_ON_ATP] = fmaf(me.y * kbj, ak.kb_on[1], g[SRS_ADJ_K_ON_ATP]);
-        g[SRS_ADJ_K_OFF_ATP] = fmaf(me.y * kbj, ak.kb_off[1], g[SRS_ADJ_K_OFF_ATP]);
-        g[SRS_ADJ_K_ON_CMDN] = fmaf(me.z * kbj, ak.kb_on[2], g[SRS_ADJ_K_ON_CMDN]);
-        g[SRS_ADJ_K_OFF_CMDN] = fmaf(me.z * kbj, ak.kb_off[2], g[SRS_ADJ_K_OFF_CMDN]);
+        g.on_zw.y = fmaf(me.w * kbj, ak.kb_on[0], g.on_zw.y);
+        g.off_zw.y = fmaf(me.w * kbj, ak.kb_off[0], g.off_zw.y);
+        g.on_atp = fmaf(me.y * kbj, ak.kb_on[1], g.on_atp);
+        g.off_atp = fmaf(me.y * kbj, ak.kb_off[1], g.off_atp);
+        g.on_zw.x = fmaf(me.z * kbj, ak.kb_on[2], g.on_zw.x);
+        g.off_zw.x = fmaf(me.z * kbj, ak.kb_off[2], g.off_zw.x);
       }
     }
     if (a.flags[j] & 4u) {
@@ -171,7 +127,7 @@ __global__ void __launch_bounds__(ADJP_THREADS, 4) k_adjp_step(AdjPlainArgs a) {
             if (e.kind == 0) {
               oc = fmaf(-k.jr_scale, qv, oc);
               const float cj = k.c0j + tu[pe].x;
-              g[SRS_ADJ_V_RYR] = fmaf(qv * ak.v_cell, cj - c, g[SRS_ADJ_V_RYR]);
+              g.v_ryr = fmaf(qv * ak.v_cell, cj - c, g.v_ryr);
             } else {
               oc = fmaf(k.jr_scale, qv, oc);
             }
@@ -184,12 +140,13 @@ __global__ void __launch_bounds__(ADJP_THREADS, 4) k_adjp_step(AdjPlainArgs a) {
     }
     adj_rapid(k, ak, bsl, c, ig.y, w, dG, oc, g);
     // compensated update of lambda
-    float4 L = make_float4(lx, me.y, me.z, me.w);
-    kadd(L.x, cm.x, k.dt * oc);
-    kadd(L.y, cm.y, k.dt * lt.oa);
-    kadd(L.z, cm.z, k.dt * lt.om);
-    kadd(L.w, cm.w, k.dt * lt.oy);
-    kadd(li, ci, k.dt * lt.oi);
+    const float2 ndt = p_bc(-k.dt);
+    float2 Lxy = make_float2(lx, me.y), Lzw = hi2(me), cxy = lo2(cm), czw = hi2(cm);
+    kadd(Lxy, cxy, ndt, make_float2(oc, lt.oxy.y));
+    kadd(Lzw, czw, ndt, lt.ozw);
+    kadd(li, ci, -k.dt, lt.oi);
+    const float4 L = make_float4(Lxy.x, Lxy.y, Lzw.x, Lzw.y);
+    cm = make_float4(cxy.x, cxy.y, czw.x, czw.y);
     a.lam_im[o] = li;
     comp_store4_x2(a.lam_c4q + o, cm);
     a.lam_cimq[o] = comp_store1(ci);
@@ -204,7 +161,9 @@ __global__ void __launch_bounds__(ADJP_THREADS, 4) k_adjp_step(AdjPlainArgs a) {
   // gradient of the step: warp sums, then the block's FP64 row
   __shared__ float red[ADJP_THREADS / 32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  red[warp][lane] = warp_sums<NA>(g, lane);
+  float sums[NA];
+  g.get(sums);
+  red[warp][lane] = warp_sums<NA>(sums, lane);
   __syncthreads();
   if (threadIdx.x < NA) {
     double v = 0.0;

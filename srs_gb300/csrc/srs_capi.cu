@@ -2619,6 +2619,10 @@ int adjoint_geometry(srs_sim* s, int m, int bits) {
     for (int k = 0; k < 4; ++k) {
       a[k] = (float)s->op.aij[5 * (size_t)j + 1 + k];
       geo[e].nb[k] = mcode(s->eng_of_ref[s->op.nij[4 * (size_t)j + k]]);
+      // what a step does before the cluster barrier reads this CTA alone: the
+      // codes are offsets in it
+      const int q = e / Pf, i = e % Pf - s->part_nch[q];
+      if (i < s->part_nint[q] && (i >= 0 || s->ar.ch_interior)) geo[e].nb[k] &= (uint16_t)((1u << bits) - 1u);
     }
     const float4 t = s->aT_h[e];
     geo[e].aT[0] = t.x;
@@ -3017,14 +3021,17 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
       return fail(SRS_ERR_INPUT, "cta_partitions must divide the cluster size");
     // CTA grouping: m forward partitions per CTA (clusters of C/m CTAs), the
     // owner state of lambda on chip when it fits next to the published slots,
-    // 256 or 512 threads.  Chosen by the estimated time, rounds of clusters x
-    // slots per thread; at equal estimate the 256-thread CTA wins (two CTAs per
-    // SM overlap each other's barrier waits).
+    // 256, 512 or 640 threads.  Chosen by the estimated time of a step, in units
+    // of a thread's wait for one slot: its slots, the SM's slots at the rate the
+    // SM gets through them (335 in that time), and two for the barriers; the
+    // owner state in global memory costs a tenth.  64 realizations of the
+    // 10,368-element mesh, 512 steps: two rounds of four CTAs of 512 threads 8.9
+    // ms, of 640 7.7, one round of two CTAs 7.3 and 6.7.
     int best_m = 0, best_bits = 0;
     bool best_own = false, best_stage = false;
     double best_cost = 1e300;
     const std::vector<int> thr_list =
-        d->threads_per_cta ? std::vector<int>{d->threads_per_cta} : std::vector<int>{256, 512};
+        d->threads_per_cta ? std::vector<int>{d->threads_per_cta} : std::vector<int>{256, 512, 640};
     for (int thr : thr_list) {
       for (int m = 1; m <= s->C; ++m) {
         if (s->C % m || (d->cta_partitions && m != d->cta_partitions)) continue;
@@ -3041,8 +3048,9 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
             const size_t sm = adjoint_smem_bytes(Pc, s->part_nch[0], n_ent, own != 0, stage != 0);
             const int ncl = std::min(adjoint_max_clusters(Ca, thr, sm), R);
             if (ncl <= 0) continue;
-            const double cost = std::ceil((double)R / ncl) * std::ceil((double)Pc / thr) *
-                                (own ? 1.0 : 1.15) * (stage ? 1.01 : 1.0) * (thr == 512 ? 1.02 : 1.0);
+            const double per_sm = std::ceil((double)ncl * Ca / sm_count());
+            const double cost = std::ceil((double)R / ncl) * (std::ceil((double)Pc / thr) + per_sm * Pc / 335.0 + 2.0) *
+                                (own ? 1.0 : 1.1) * (stage ? 1.01 : 1.0);
             if (cost < best_cost) {
               best_cost = cost;
               best_m = m;
