@@ -1082,6 +1082,14 @@ int reset_states(srs_sim* s) {
   return clear_compensation(s, 0, n);
 }
 
+// The FP32 engines' element flags: an array of the plain engine, the last word of
+// the resident engine's record halves.
+const uint32_t* element_flags(const srs_sim* s, int32_t* stride) {
+  const bool plain = s->d.engine == SRS_ENGINE_PLAIN;
+  *stride = plain ? 1 : 4;
+  return plain ? s->a32.flags : reinterpret_cast<const uint32_t*>(s->ar.geo_b) + 3;
+}
+
 // Realization r in the caller's form (any output may be null): the conversion
 // and the gathering run on the device (k_export_state).  Up to a few MB it
 // writes pinned host memory and the caller's arrays are filled from there;
@@ -1110,11 +1118,7 @@ int export_state(srs_sim* s, int r, double* S, int* ryr, int* lcc, int* lccv, do
       a.CI = s->d_CI + r * NE;
     }
     a.eng_of_ref = s->d_eng_of_ref;
-    // flags: an array of the plain engine, the last word of the resident
-    // engine's record halves
-    const bool plain = s->d.engine == SRS_ENGINE_PLAIN;
-    a.flags = plain ? s->a32.flags : reinterpret_cast<const uint32_t*>(s->ar.geo_b) + 3;
-    a.flag_stride = plain ? 1 : 4;
+    a.flags = element_flags(s, &a.flag_stride);
     const RestValues& rv = s->rv;
     const double rest[6] = {rv.ca0, rv.atp, rv.cmdn, rv.trpn, rv.csqn, rv.dye};
     std::copy(rest, rest + 6, a.rest);
@@ -3233,29 +3237,32 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
   } else {
     SRS_CUDA(cudaMemcpyAsync(out->grad, grad, sizeof(double) * R * SRS_N_ADJ, cudaMemcpyDeviceToHost, s->st));
   }
-  std::vector<float4> hl, hc;
-  std::vector<float> hi, hci;
   if (out->grad_state) {
-    hl.resize((size_t)R * NE);
-    hc.resize((size_t)R * NE);
-    hi.resize((size_t)R * NE);
-    hci.resize((size_t)R * NE);
-    SRS_CUDA(cudaMemcpyAsync(hl.data(), lam, sizeof(float4) * R * NE, cudaMemcpyDeviceToHost, s->st));
-    SRS_CUDA(cudaMemcpyAsync(hi.data(), lam_im, sizeof(float) * R * NE, cudaMemcpyDeviceToHost, s->st));
-    if (plain) {
-      std::vector<ushort4> q4((size_t)R * NE);
-      std::vector<uint16_t> q1((size_t)R * NE);
-      SRS_CUDA(cudaMemcpyAsync(q4.data(), lam_c4, sizeof(ushort4) * R * NE, cudaMemcpyDeviceToHost, s->st));
-      SRS_CUDA(cudaMemcpyAsync(q1.data(), lam_cim, sizeof(uint16_t) * R * NE, cudaMemcpyDeviceToHost, s->st));
-      SRS_CUDA(cudaStreamSynchronize(s->st));
-      for (size_t e = 0; e < q4.size(); ++e) {
-        hc[e] = make_float4(comp_decode_host(q4[e].x), comp_decode_host(q4[e].y), comp_decode_host(q4[e].z),
-                            comp_decode_host(q4[e].w));
-        hci[e] = comp_decode_host(q1[e]);
+    // as many realizations at a time as fill 64 MB
+    const size_t per = (size_t)6 * s->N;
+    const int chunk = (int)std::min<size_t>(R, std::max<size_t>(1, ((size_t)64 << 20) / (per * sizeof(double))));
+    ExportLambdaArgs ea{};
+    ea.N = s->N;
+    ea.NE = NE;
+    ea.eng_of_ref = s->d_eng_of_ref;
+    ea.flags = element_flags(s, &ea.flag_stride);
+    SRS_TRY(sc.get(&ea.g, per * chunk));
+    for (int r = 0; r < R; r += chunk) {
+      const int n = std::min(chunk, R - r);
+      const size_t o = (size_t)r * NE;
+      ea.lam = lam + o;
+      ea.lam_im = lam_im + o;
+      if (plain) {
+        ea.c4q = reinterpret_cast<const ushort4*>(lam_c4) + o;
+        ea.cimq = reinterpret_cast<const uint16_t*>(lam_cim) + o;
+      } else {
+        ea.c4 = lam_c4 + o;
+        ea.cim = lam_cim + o;
       }
-    } else {
-      SRS_CUDA(cudaMemcpyAsync(hc.data(), lam_c4, sizeof(float4) * R * NE, cudaMemcpyDeviceToHost, s->st));
-      SRS_CUDA(cudaMemcpyAsync(hci.data(), lam_cim, sizeof(float) * R * NE, cudaMemcpyDeviceToHost, s->st));
+      if (launch_export_lambda(ea, n, s->st)) return fail(SRS_ERR_CUDA, "gradient export launch failed");
+      s->launches++;
+      SRS_CUDA(cudaMemcpyAsync(out->grad_state + (size_t)r * per, ea.g, sizeof(double) * per * n,
+                               cudaMemcpyDeviceToHost, s->st));
     }
   }
   SRS_CUDA(cudaStreamSynchronize(s->st));
@@ -3274,24 +3281,6 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
     for (int64_t t = 0; t < n_ticks; ++t)
       for (int i = 0; i < ns; ++i) Ls += loss_t[((size_t)t * R + r) * ns + i];
     out->loss[r] = Ls;
-  }
-  if (out->grad_state) {
-    const int N = s->N;
-    for (int r = 0; r < R; ++r) {
-      double* g = out->grad_state + (size_t)r * 6 * N;
-      for (int j = 0; j < N; ++j) {
-        const size_t e = (size_t)r * NE + s->eng_of_ref[j];
-        const float4 Lv = hl[e], Cc = hc[e];
-        const double li = (double)hi[e] - (double)hci[e];
-        const bool jsr = s->m.domain[j] == DOMAIN_JSR;
-        g[SP_CA * (size_t)N + j] = (double)Lv.x - (double)Cc.x;
-        g[SP_ATP * (size_t)N + j] = (double)Lv.y - (double)Cc.y;
-        g[SP_CMDN * (size_t)N + j] = (double)Lv.z - (double)Cc.z;
-        g[SP_DYE * (size_t)N + j] = (double)Lv.w - (double)Cc.w;
-        g[SP_TRPN * (size_t)N + j] = (!jsr && s->m.tropc[j]) ? li : 0.0;
-        g[SP_CSQN * (size_t)N + j] = jsr ? li : 0.0;
-      }
-    }
   }
   {
     unsigned int st_bits = 0;

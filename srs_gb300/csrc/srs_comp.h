@@ -17,39 +17,12 @@
 // (the device's conversion; the CPU oracle restates it with the compiler's
 // _Float16), and reading back is exact on host and device alike.
 #pragma once
-#include <math.h>
 #include <stdint.h>
-#include <string.h>
 
 namespace srs {
 
 constexpr float kCompScale = 16777216.0f;          // 2^24
 constexpr float kCompInvScale = 1.0f / 16777216.0f;  // 2^-24
-
-// IEEE binary16 to binary32 (exact).
-inline float comp_half_to_float_host(uint16_t h) {
-  const uint32_t sign = (uint32_t)(h & 0x8000u) << 16;
-  const int e = (h >> 10) & 0x1F;
-  const uint32_t m = h & 0x3FFu;
-  float v;
-  if (e == 0) {
-    v = (float)m * (1.0f / 16777216.0f);  // subnormal: m * 2^-24, exact
-  } else if (e == 31) {
-    const uint32_t b = 0x7F800000u | (m << 13);  // infinity, or a NaN
-    memcpy(&v, &b, 4);
-  } else {
-    uint32_t b = ((uint32_t)(e - 15 + 127) << 23) | (m << 13);
-    memcpy(&v, &b, 4);
-  }
-  uint32_t vb;
-  memcpy(&vb, &v, 4);
-  vb |= sign;
-  memcpy(&v, &vb, 4);
-  return v;
-}
-
-// Host side: the compensation term held in the stored 16 bits.
-inline float comp_decode_host(uint16_t q) { return comp_half_to_float_host(q) * kCompInvScale; }
 
 #ifdef __CUDACC__
 // Device side.  cvt.rn.satfinite rounds to nearest even and saturates to

@@ -256,6 +256,21 @@ struct ExportArgs {
   double* res_out;
 };
 int launch_export_state(const ExportArgs& a, cudaStream_t st);
+struct ExportLambdaArgs {
+  int32_t N;
+  size_t NE;                    // elements per realization in the engine's arrays
+  const float4* lam;            // [R][NE]
+  const float* lam_im;
+  const float4* c4;             // compensation, or compact when c4q / cimq are set
+  const float* cim;
+  const ushort4* c4q;
+  const uint16_t* cimq;
+  const int32_t* eng_of_ref;
+  const uint32_t* flags;        // as in ExportArgs
+  int32_t flag_stride;
+  double* g;                    // [R][6][N]
+};
+int launch_export_lambda(const ExportLambdaArgs& a, int R, cudaStream_t st);
 int launch_broadcast_state(const double* src, double* dst, size_t n, int R, cudaStream_t st);
 
 // ---- total Ca per compartment (k_mass.cu) ------------------------------------

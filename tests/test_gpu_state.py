@@ -89,3 +89,21 @@ def test_steps_after_the_end_of_a_run(srs, meshes, prec):
     sim.reset()
     sim.explicit_step(33)
     assert all(not np.array_equal(sim.get_state(r)["states"], end[r]) for r in range(3))
+
+
+def test_state_gradient_in_chunks(srs, meshes):
+    """dL/d(initial state) of more realizations than are converted at a time (64 MB)."""
+    from conftest import LINESCAN_DESC
+    p = _params(srs)
+    g = srs.Grid(p, meshes["large"])
+    R = 12
+    assert R * 48 * g.n_ele > 64 << 20
+    gs = []
+    for seeds in (list(range(R)), [R - 1]):
+        sim = srs.Simulation(g, p, len(seeds), 32, srs.ENGINE_PLAIN, seeds=seeds)
+        n = sim.linescan_setup(**LINESCAN_DESC)
+        f0 = sim.linescan()[1]
+        assert n == len(f0)
+        gs.append(sim.adjoint(4, 2, f0, grad_state=True)[2])
+    assert np.abs(gs[0][-1]).max() > 0
+    assert np.array_equal(gs[0][-1], gs[1][0])
