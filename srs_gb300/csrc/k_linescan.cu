@@ -8,6 +8,7 @@
 // (samples x elements, engine numbering) and the constant padding sum into an
 // offset; this kernel evaluates the sum from the state in HBM for every
 // realization, accumulating in double precision.
+#include "srs_comp.h"
 #include "srs_engine.h"
 
 namespace srs {
@@ -46,8 +47,8 @@ __global__ void k_linescan(LinescanArgs a) {
 // adds them into its eight sums, one multiply-add per weight.  The bound is
 // the FP64 pipe: 1024 realizations of the 10,368-element dyad, 40 samples,
 // about 330 M weighted terms, 0.52 ms at 2 DFMA per clock and SM; the call
-// took 3.19 ms untiled and takes 0.94.  The chunks are dealt to a.splits blocks whose partial sums
-// k_linescan_sum adds in order.
+// took 3.19 ms untiled and takes 0.73.  The chunks are dealt to a.splits blocks
+// (a.split: by their work) whose partial sums k_linescan_sum adds in order.
 __global__ void __launch_bounds__(256) k_linescan_tile(LinescanArgs a, int R) {
   __shared__ double s_dye[LINESCAN_CHUNK][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -58,8 +59,7 @@ __global__ void __launch_bounds__(256) k_linescan_tile(LinescanArgs a, int R) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc[k] = 0.0;
   const int32_t* tp = a.tptr + (size_t)(live ? g : 0) * (a.n_chunk + 1);
-  const int c0 = (int)((int64_t)a.n_chunk * blockIdx.x / gridDim.x);
-  const int c1 = (int)((int64_t)a.n_chunk * (blockIdx.x + 1) / gridDim.x);
+  const int c0 = a.split[blockIdx.x], c1 = a.split[blockIdx.x + 1];
   for (int c = c0; c < c1; ++c) {
     const int e0 = c * LINESCAN_CHUNK;
     __syncthreads();
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256) k_linescan_tile(LinescanArgs a, int R) {
           const size_t o = (size_t)r * a.n_state + e;
           const float u = a.M[o].w;
           const float cm = a.CMq ? comp_load1(a.CMq[o].w) : a.CM[o].w;
-          dye = a.rest_dye[e] + ((double)u - (double)cm);
+          dye = a.rest_dye[e] + (widen(u) - widen(cm));
         }
       }
       s_dye[k][rr] = dye;
@@ -114,12 +114,12 @@ __global__ void k_linescan_sum(LinescanArgs a, int R) {
 // Warps of a tiled block: one per sample group, eight at most.
 static int tile_warps(int n_samples) { return (n_samples + 7) / 8 < 8 ? (n_samples + 7) / 8 : 8; }
 
-// Blocks that share the chunks of one tile of realizations: six per SM in
-// all, at least one chunk each.
+// Blocks that share the chunks of one tile of realizations: eight per SM in
+// all (six or twelve measured up to a tenth longer), at least one chunk each.
 int linescan_splits(int n_samples, int n_state, int R, int n_sm) {
   const int chunks = (n_state + LINESCAN_CHUNK - 1) / LINESCAN_CHUNK;
   const int tiles = (R + 31) / 32 * (((n_samples + 7) / 8 + 7) / 8);
-  const int want = (6 * n_sm + tiles - 1) / tiles;
+  const int want = (8 * n_sm + tiles - 1) / tiles;
   return chunks < want ? chunks : want;
 }
 

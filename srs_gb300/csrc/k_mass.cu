@@ -14,32 +14,48 @@
 
 namespace srs {
 
-// Rapid-buffer part b c / (K + c).  The division is skipped where it gives
-// zero (elements off the membrane, about nine in ten): the FP64 pipe issues
-// one warp instruction in 64 cycles here, and the two divisions were half of
-// an element's work.
-__device__ __forceinline__ double sl_bound(double b, double K, double c) {
-  return b == 0.0 && isfinite(c) && c != -K ? 0.0 : b * c / (K + c);
+// Rapid-buffer part b c / (K + c).
+__device__ __forceinline__ double sl_bound(double b, double K, double c) { return b * c / (K + c); }
+// c at which a buffer of no capacity binds nothing: finite, not -K (tests on the
+// bits: the FP64 pipe issues one warp instruction in 64 cycles here)
+__device__ __forceinline__ bool plain_ca(const MassArgs& a, double c) {
+  return (__double2hiint(c) & 0x7ff00000) != 0x7ff00000 && __double_as_longlong(c) != __double_as_longlong(-a.khi) &&
+         __double_as_longlong(c) != __double_as_longlong(-a.klo);
+}
+
+// The FP32 engines' state of one element: deviation less compensation, widened
+// on the integer units.
+__device__ __forceinline__ double dev_ca(const MassArgs& a, size_t o) {
+  const float c = a.CMq ? comp_load4(a.CMq + o).x : a.CM[o].x;
+  return widen(a.M[o].x) - widen(c);
 }
 
 // Grid: x over blocks of one realization's elements, y over realizations.  A
-// block per realization alone leaves a few large realizations on a few SMs
-// (32 x 542,376 elements: 11.4 ms a call; with the split and without the
-// empty divisions 1.24, bound by the FP64 pipe).  Each block writes its two sums; k_total_ca_sum adds them in order.
+// block per realization alone leaves a few large realizations on a few SMs.
+// The bound is the FP64 pipe, so an FP32 engine's element takes twelve of its
+// instructions: the five deviations less their compensation, their sum on top of
+// the summed resting values, Ca for its test and the volume's multiply-add.  The
+// rapid buffers, a division each for the one element in ten at the membrane,
+// follow over the list of those, so that whole warps divide.
+// 32 x 542,376 elements: 11.4 ms a call by one block a realization, 1.25 with
+// the split, 0.49 with this count and list.  Each block writes its two sums;
+// k_total_ca_sum adds them in order.
 __global__ void __launch_bounds__(256) k_total_ca(MassArgs a) {
   const int r = blockIdx.y;
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  const double* S = a.S64 ? a.S64 + (size_t)r * 6 * a.n_state : nullptr;
+  const size_t ro = (size_t)r * a.n_state;
   double acc[2] = {0.0, 0.0};
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.n_state; e += gridDim.x * blockDim.x) {
+  for (int e = t0; e < a.n_state; e += nt) {
     const double v0 = a.v0[e];
-    if (v0 == 0.0) continue;  // padding slot
-    double c, bound;
-    if (a.S64) {
-      const double* S = a.S64 + (size_t)r * 6 * a.n_state;
+    if (__double_as_longlong(v0) == 0) continue;  // padding slot
+    double c, sum;
+    if (S) {
       const size_t n = a.n_state;
       c = S[e];
-      bound = S[n + e] + S[2 * n + e] + S[3 * n + e] + S[4 * n + e] + S[5 * n + e];
+      sum = c + (S[n + e] + S[2 * n + e] + S[3 * n + e] + S[4 * n + e] + S[5 * n + e]);
     } else {
-      const size_t o = (size_t)r * a.n_state + e;
+      const size_t o = ro + e;
       const float4 m = a.M[o];
       const float im = a.I[o];
       float4 cm;
@@ -51,13 +67,25 @@ __global__ void __launch_bounds__(256) k_total_ca(MassArgs a) {
         cm = a.CM[o];
         ci = a.CI[o];
       }
-      const double* rs = a.rest4 + 4 * (size_t)e;
-      c = rs[0] + ((double)m.x - (double)cm.x);
-      bound = (rs[1] + ((double)m.y - (double)cm.y)) + (rs[2] + ((double)m.z - (double)cm.z)) +
-              (rs[3] + ((double)m.w - (double)cm.w)) + (a.rest_imm[e] + ((double)im - (double)ci));
+      const double dx = widen(m.x) - widen(cm.x), dy = widen(m.y) - widen(cm.y), dz = widen(m.z) - widen(cm.z),
+                   dw = widen(m.w) - widen(cm.w), di = widen(im) - widen(ci);
+      c = a.rest_ca[e] + dx;
+      sum = a.rest_sum[e] + (((dx + dy) + (dz + dw)) + di);
     }
-    const double sl = sl_bound(a.bhi[e], a.khi, c) + sl_bound(a.blo[e], a.klo, c);
-    acc[a.jsr[e] ? 1 : 0] += v0 * (c + bound + sl);
+    if (!plain_ca(a, c)) sum += sl_bound(a.bhi[e], a.khi, c) + sl_bound(a.blo[e], a.klo, c);
+    if (a.jsr[e]) acc[1] = fma(v0, sum, acc[1]);
+    else acc[0] = fma(v0, sum, acc[0]);
+  }
+  for (int q = t0; q < a.n_sl; q += nt) {
+    const int e = a.sl[q];
+    const double c = S ? S[e] : a.rest_ca[e] + dev_ca(a, ro + e);
+    if (!plain_ca(a, c)) continue;  // above
+    double b = 0.0;
+    const double bhi = a.bhi[e], blo = a.blo[e];
+    if (__double_as_longlong(bhi) != 0) b = sl_bound(bhi, a.khi, c);
+    if (__double_as_longlong(blo) != 0) b += sl_bound(blo, a.klo, c);
+    if (a.jsr[e]) acc[1] = fma(a.v0[e], b, acc[1]);
+    else acc[0] = fma(a.v0[e], b, acc[0]);
   }
   for (int o = 16; o > 0; o >>= 1) {
     acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);

@@ -84,6 +84,20 @@ __device__ __forceinline__ unsigned short comp_store1(float c) {
   asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(q) : "f"(c * kCompScale));
   return q;
 }
+// (double)f on the integer units: conversions share the FP64 pipe, which issues
+// one warp instruction in 64 cycles on sm_103a (and a conversion on a branch that
+// the compiler turns into a predicate is issued all the same).
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f);
+  uint32_t m = b & 0x7fffffffu;
+  uint32_t rebias = m >= 0x7f800000u ? 0x70000000u : 0x38000000u;  // 1151 (infinity, NaN) or 896 exponents
+  if (m < 0x00800000u) {  // zero, or a denormal: normalise
+    const int s = __clz((int)m) - 8;
+    m = m ? m << s : 0u;
+    rebias = m ? rebias - ((uint32_t)s << 20) : 0u;
+  }
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + rebias)), (int)(m << 29));
+}
 #endif
 
 }  // namespace srs

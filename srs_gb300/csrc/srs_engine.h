@@ -225,6 +225,7 @@ struct LinescanArgs {
   const uint32_t* tent;  // (sample mask << 24) | offset in the chunk
   const double* tw;      // [entry][8]
   int32_t splits;        // blocks the chunks are dealt to
+  const int32_t* split;  // [splits + 1] first chunk of each
   double* part;          // [splits][R][n_samples]
 };
 constexpr int LINESCAN_CHUNK = 64;
@@ -281,6 +282,8 @@ struct MassArgs {
   const double* bhi;      // [n_state] rapid SL buffer capacities (uM)
   const double* blo;
   double khi, klo;
+  int32_t n_sl;           // elements with rapid buffers, and their list
+  const int32_t* sl;
   const double* S64;      // FP64 engine state [R][6][n_state], or null
   const float4* M;        // FP32 engines: deviations and compensation
   const float4* CM;
@@ -288,8 +291,8 @@ struct MassArgs {
   const float* CI;
   const ushort4* CMq;     // compact compensation (srs_comp.h), when set
   const uint16_t* CIq;
-  const double* rest4;    // [n_state][4] rest of Ca, ATP, CMDN, dye
-  const double* rest_imm; // [n_state]
+  const double* rest_ca;  // [n_state] resting Ca
+  const double* rest_sum; // [n_state] resting total of the five species
   double* part;           // [R][blocks][2]: the blocks' sums
   double* out;            // [R][2]: cytosol, JSR
 };
