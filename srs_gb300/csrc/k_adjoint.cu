@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "srs_adjoint.cuh"
+#include "srs_comp.h"
 #include "srs_cluster.cuh"
 #include "srs_engine.h"
 
@@ -466,7 +467,10 @@ __global__ void __launch_bounds__(640, 1) k_adjoint32(AdjArgs a) {
 // dye(col_q) with the dye deviation of the trajectory slot (base_i: pad plus
 // the resting dye), e_i = F_i / F0_i - 1 - target_i, coef_i = e_i / F0_i
 // (= dL/dF_i) and the loss term e_i^2 / 2, kept per sample so the host sums
-// them in a fixed order.  One block per (sample, realization, tick).
+// them in a fixed order.  One block per (sample, realization, tick); bound by the
+// FP64 pipe, which takes one multiply-add a term (widen: the conversion would be
+// a second; 40 samples, four ticks of 21 x 15,288 elements 145 us with it, 104
+// without).
 __global__ void k_adj_tick(AdjTickArgs a) {
   const int i = blockIdx.x, r = blockIdx.y, z = blockIdx.z;
   // dye deviation: the fourth float of each element's state
@@ -474,7 +478,7 @@ __global__ void k_adj_tick(AdjTickArgs a) {
                                                   (size_t)r * a.n_state);
   double acc = 0.0;
   for (int q = a.ptr[i] + threadIdx.x; q < a.ptr[i + 1]; q += blockDim.x)
-    acc += a.w[q] * (double)__ldg(U + 4 * (size_t)a.col[q] + 3);
+    acc += a.w[q] * widen(__ldg(U + 4 * (size_t)a.col[q] + 3));
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   __shared__ double red[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -131,7 +131,7 @@ __device__ __forceinline__ void plain32_gate(const Plain32Args& a, int r, int32_
   const float* rest = a.rest_ca;
   auto ca = [&](int e) -> double {
     float u = ((volatile const float*)(Mo + e))[0];
-    return (double)(rest[e] + u);
+    return widen(rest[e] + u);
   };
   int32_t* ryr_w = a.CS.ryr + (size_t)r * a.C.NR;
   int32_t* lcc_w = a.CS.lcc + (size_t)r * a.C.NL;
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(256) k_plain32_gate(Plain32Args a) {
       ctl.step += 1;
       ctl.t += a.P.dt;
       prestep(a.P, a.C, ctl, ryr, lcc, lccv, a.CS.rows + (size_t)r * a.P.row_cap * a.P.row_w,
-              [&](int e) -> double { return (double)(a.rest_ca[e] + M[e].x); });
+              [&](int e) -> double { return widen(a.rest_ca[e] + M[e].x); });
       *ctlp = ctl;
     } else {
       ctlp->step = step + 1;
@@ -308,7 +308,7 @@ __global__ void k_plain32_prestep(Plain32Args a, int write_initial_row) {
   if (threadIdx.x != 0) return;
   RealCtl ctl = a.CS.ctl[r];
   const float4* M = a.M_in + (size_t)r * a.N;
-  auto ca = [&](int e) -> double { return (double)(a.rest_ca[e] + M[e].x); };
+  auto ca = [&](int e) -> double { return widen(a.rest_ca[e] + M[e].x); };
   int32_t* ryr = a.CS.ryr + (size_t)r * a.C.NR;
   int32_t* lcc = a.CS.lcc + (size_t)r * a.C.NL;
   int32_t* lccv = a.CS.lccv + (size_t)r * a.C.NL;

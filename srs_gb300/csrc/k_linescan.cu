@@ -26,7 +26,7 @@ __global__ void k_linescan(LinescanArgs a) {
       const size_t o = (size_t)r * a.n_state + e;
       const float u = a.M[o].w;
       const float c = a.CMq ? comp_load1(a.CMq[o].w) : a.CM[o].w;
-      dye = a.rest_dye[e] + ((double)u - (double)c);
+      dye = a.rest_dye[e] + (widen(u) - widen(c));
     }
     acc += a.w[q] * dye;
   }

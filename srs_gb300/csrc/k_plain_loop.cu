@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(PLAIN_LOOP_T32, 6) k_plain32_loop(const __grid
   float4* M[2] = {const_cast<float4*>(a.M_in) + ro, a.M_out + ro};
   if (b == l.blocks) {
     gate_loop(a, l, r, steps,
-              [&](int e, int buf) { return (double)(a.rest_ca[e] + __ldcg(&M[buf][e].x)); }, smem);
+              [&](int e, int buf) { return widen(a.rest_ca[e] + __ldcg(&M[buf][e].x)); }, smem);
     return;
   }
   const LocalChan ch = local_channels(a, l, r, b, smem);
