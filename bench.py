@@ -11,12 +11,13 @@ steps.
 
 Metric: simulated spark-ms per wall second (sum over realizations).
   value      device-resident: one run of W + K launches from the equilibrium
-             state (uploaded before the run); CUDA events on the engine's
+             state (set before the run); CUDA events on the engine's
              stream around each launch, the last K summed.  The state
              (1024 x 10,368 x 20 B = 212 MB) is larger than the 129 MB L2, so
              no flush is needed.
   e2e        through the public API with host buffers: srs_sim_reset
-             (initial state uploaded from pinned host memory) +
+             (channel states, residuals and control blocks uploaded from
+             pinned host memory, the equilibrium set on the device) +
              srs_run_simulation (RunSimulation protocol, states rows read
              back) for --launch-steps steps, per bench step.
   roofline   algorithmic bytes of the dominant kernel per launch =
@@ -884,7 +885,7 @@ def run_ours(args):
         tuned = tuner.tune_resident(grid, p, R, seeds=seeds)
     # One bench step = one launch of S time steps of the reference's
     # RunSimulation under the DefaultSpark protocol (RyR 24 held open, output
-    # rows every S steps), from the equilibrium state uploaded by
+    # rows every S steps), from the equilibrium state set by
     # srs_sim_reset before the run.  The run has W + K launches: the first W
     # are the warm-up, the last K the timed region, each launch timed on the
     # device (CUDA events on the engine's stream, srs_run_simulation_timed).
