@@ -16,6 +16,18 @@ __device__ __forceinline__ bool greater_bits(double c, double m) {
   return b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll;
 }
 
+// Channels whose Ca has been gathered beforehand: the element indices of Channels
+// are places in that list (RyR cleft elements, JSR elements, LCC elements).
+struct GatheredChannels {
+  struct Places {
+    int base;
+    __device__ int operator[](int i) const { return base + i; }
+  };
+  int32_t NR, NL;
+  Places ryr_cleft, ryr_jsr, lcc_ele;
+  __device__ GatheredChannels(int nr, int nl) : NR(nr), NL(nl), ryr_cleft{0}, ryr_jsr{nr}, lcc_ele{2 * nr} {}
+};
+
 // One states row (WriteToStateFiles, cpu/OutputFuncs.cpp:241-350), computed
 // serially in double precision in the reference's summation order.  It stands in
 // the step's critical path and each FP64 instruction takes 64 cycles, so a closed
@@ -23,8 +35,8 @@ __device__ __forceinline__ bool greater_bits(double c, double m) {
 // the gradient is not finite.  Six rows of 1,024 realizations with 49 RyRs: 4.4 ->
 // 3.6 ms of a run.  (The terms formed by a warp's lanes took 1.5, but cost the
 // resident step loop registers and 3 %.)
-template <class CaAt>
-__device__ void write_row(const Protocol& P, const Channels& C, RealCtl& ctl,
+template <class Ch, class CaAt>
+__device__ void write_row(const Protocol& P, const Ch& C, RealCtl& ctl,
                           const int32_t* ryr, const int32_t* lcc, const int32_t* lccv,
                           float* rows_r, double t, CaAt ca) {
   if (ctl.n_rows >= P.row_cap) {
@@ -74,8 +86,8 @@ __device__ void write_row(const Protocol& P, const Channels& C, RealCtl& ctl,
 // Protocol work that precedes time step ctl.step (one thread):
 // termination predicate, LCC closing, voltage clamp, RyR hold and the states
 // row at output ticks (cpu/RunSimulation.cpp:522-566).
-template <class CaAt>
-__device__ void prestep(const Protocol& P, const Channels& C, RealCtl& ctl, int32_t* ryr,
+template <class Ch, class CaAt>
+__device__ void prestep(const Protocol& P, const Ch& C, RealCtl& ctl, int32_t* ryr,
                         int32_t* lcc, const int32_t* lccv, float* rows_r, CaAt ca) {
   if (ctl.done || !P.run_protocol) return;
   const int64_t n = ctl.step;

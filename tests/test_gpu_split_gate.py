@@ -61,3 +61,20 @@ def test_run_protocol(srs, big, clamp):
     for x, y in zip(ra[0], rb[0]):
         assert len(x) > 3 and np.array_equal(x[:, [0, 2, 3]], y[:, [0, 2, 3]])  # t, open RyRs, open LCCs
         np.testing.assert_allclose(x[:, [1, 4, 5, 6]], y[:, [1, 4, 5, 6]], rtol=1e-4)
+
+
+def test_rows_of_many_channels(srs, tmp_path):
+    """Rows whose channels' Ca is gathered beforehand (up to 2,048 values) and read in
+    place: the same sums, up to the engine's Ca."""
+    for n in (20, 34):  # 400 and 1,156 RyRs: 807 and 2,319 values
+        base = str(tmp_path / str(n))
+        srs.write_box_mesh(base, box_x=3.0, box_y=3.0, box_z=3.0, foot_half_x=0.6, foot_half_y=0.6, n_foot_x=10,
+                           n_foot_y=10, n_out_x=6, n_out_y=6, n_above_z=22, ryr_nx=n, ryr_ny=n, n_lcc=7,
+                           lcc_half=0.5)
+        p = srs.default_parameters().set(T_STEP=1e-6, INIT_RYR=24, T_FINAL=1e-5, OUTPUT_STATES_INTERVAL=3e-6)
+        a, b = _pair(srs, base, p, 2)
+        assert (2 * a.grid.n_ryr + a.grid.n_lcc <= 2048) == (n == 20)
+        ra, rb = a.run_simulation(), b.run_simulation()
+        for x, y in zip(ra[0], rb[0]):
+            assert len(x) > 3 and np.array_equal(x[:, [0, 2, 3]], y[:, [0, 2, 3]])
+            np.testing.assert_allclose(x[:, [1, 4, 5, 6]], y[:, [1, 4, 5, 6]], rtol=1e-4)
