@@ -14,17 +14,18 @@
 // halves of c * 2^24 (srs_comp.h), rounded after every update.
 //
 // Two engines share the per-element update `tet_update`:
-//   * k_plain32_step: one launch per time step, state in HBM, grid.y over
-//     realizations, last block per realization runs gating + protocol;
+//   * k_plain32_step: one launch per time step, state in HBM, the last block of a
+//     realization runs gating + protocol (k_plain32_update + k_plain32_gate on
+//     large meshes; k_plain_loop.cu takes many steps a launch where they fit);
 //   * k_resident32<C>: persistent batched kernel.  One realization at a time
 //     per thread-block cluster of C CTAs; the mobile species (Ca, ATP, CMDN,
 //     dye) live in shared memory as float4, double buffered, partitioned over
 //     the cluster; neighbours in another CTA's partition are read through
 //     distributed shared memory.  Every element that carries a channel sits in
-//     partition 0, where warp 0 computes the release flux, updates those
-//     elements, gates the channels and runs the protocol of the next step
-//     while the other warps update everything else — one cluster barrier per
-//     time step, and the termination decision is known at that barrier.
+//     partition 0, where a group of up to three warps updates those elements,
+//     gates the channels and runs the protocol of the next step while the other
+//     warps update everything else — one cluster barrier per time step, and the
+//     termination decision is known at that barrier.
 #include "k_resident.cuh"
 #include "srs_adjoint.cuh"
 #include "srs_engine.h"

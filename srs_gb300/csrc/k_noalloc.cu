@@ -11,8 +11,8 @@
 //
 // The array exists once per GPU that loads this library and stays allocated
 // until the process exits.  Every call shares it; a step's last block leaves its
-// counter at zero for the next call.  Calls whose work overlaps on the GPU (different streams, or several
-// host threads) race on the array: serialise them.
+// counter at zero for the next call.  Calls whose work overlaps on the GPU
+// (different streams, or several host threads) race on the array: serialise them.
 //
 // Set-up: the first call on a device, with that device current, looks up the
 // array's device address (cudaGetSymbolAddress) and caches it per device.

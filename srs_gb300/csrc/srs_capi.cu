@@ -612,7 +612,8 @@ int clusters_at_one_per_sm(int C, size_t optin) {
 //   rounds * t,  rounds = realizations / co-resident clusters, rounded up,
 //   t = (t_lat^4 + t_thr^4)^(1/4) us,
 //   t_lat = 2.05 + 0.28 elements per thread + 6e-4 threads (the chain of one
-// step: barriers, gating, a thread's elements one after the other) and t_thr = 1.2e-3 elements per SM (what an SM issues and moves).
+// step: barriers, gating, a thread's elements one after the other) and
+//   t_thr = 1.2e-3 elements per SM (what an SM issues and moves).
 // Fitted to steps of the 10,368-element dyad: 5 x 320, two CTAs per SM, 5.6 us;
 // 3 x 512, one, 5.3; 8 x 192, three, 5.1; 16 x 320 for two realizations 2.9.
 // The smallest cluster that fits, which this replaces, took 133 us per step of
