@@ -434,8 +434,10 @@ int srs_multisite_mesh_write(const srs_multisite_spec* spec, const char* base, i
  * states_out, with every array a device buffer owned by the caller.  It calls
  * no cudaMalloc/cudaFree.  Its only other device memory is a fixed array
  * compiled into the library (per GPU, held until the process exits, about
- * 22 KB), shared by all calls and reused without reallocation: calls whose
- * work overlaps on the GPU race on it, so serialise them.  The first call on a device, with that device current,
+ * 22 KB).  Calls of up to 912 tiles of 32 elements (over all realizations)
+ * leave it alone; larger ones share it, reused without reallocation: each
+ * clears it first, and such calls whose work overlaps on the GPU race on it,
+ * so serialise them.  The first call on a device, with that device current,
  * looks up that array's device address (cudaGetSymbolAddress) and caches it;
  * make that first call before any stream capture.  The cache is not
  * refreshed, so cudaDeviceReset between calls is not supported.  Arrays use the reference numbering and the layouts returned by

@@ -10,9 +10,10 @@
 // fixed-size array below instead of in cudaMalloc'ed memory.
 //
 // The array exists once per GPU that loads this library and stays allocated
-// until the process exits.  Every call shares it; a step's last block leaves its
-// counter at zero for the next call.  Calls whose work overlaps on the GPU
-// (different streams, or several host threads) race on the array: serialise them.
+// until the process exits.  Calls of up to 912 tiles of 32 elements do not use
+// it: their step and keys come with the launches.  The others share it and each
+// clears what it uses first, so calls whose work overlaps on the GPU (different
+// streams, or several host threads) race on the array: serialise them.
 //
 // Set-up: the first call on a device, with that device current, looks up the
 // array's device address (cudaGetSymbolAddress) and caches it per device.
@@ -179,9 +180,8 @@ extern "C" int srs_explicit_step_fp64_noalloc(const srs_noalloc_step* d) {
   a.CS.rows = nullptr;
   a.counters = sc->counters;
 
-  // Small problems: one launch, which brings its step and keys along.  The
-  // counters are zero before it (the array starts so, and the last block of a
-  // step leaves its counter so).
+  // Small problems: update and gating, which bring their step and keys along
+  // and keep nothing for the next call.
   if (plain64_keys_fit(a)) {
     Plain64Keys<true> keys;
     keys.step = d->step;

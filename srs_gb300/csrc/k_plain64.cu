@@ -44,10 +44,8 @@ __device__ __forceinline__ double channels64(const Plain64Args& a, const double*
 }
 
 // The last block of realization r to get here gates its channels from the new
-// Ca and, but for the allocation-free form (KEYS), runs the protocol of the next
-// step.  chan: this block holds channel elements, whose new Ca the last block
-// must see.
-template <bool KEYS = false>
+// Ca and runs the protocol of the next step.  chan: this block holds channel
+// elements, whose new Ca the last block must see.
 __device__ __forceinline__ void plain64_tail(const Plain64Args& a, int r, const RealCtl& ctl0, const double* Sn,
                                              bool chan) {
   __shared__ int s_last;
@@ -76,15 +74,13 @@ __device__ __forceinline__ void plain64_tail(const Plain64Args& a, int r, const 
   }
   if (threadIdx.x == 0) {
     a.counters[r] = 0;  // as the next step finds it
-    if constexpr (!KEYS) {
-      ctl.step += 1;
-      ctl.t += a.P.dt;
-      prestep(a.P, a.C, ctl, ryr_w, lcc_w, lccv_w,
-              a.CS.rows + (size_t)r * a.P.row_cap * a.P.row_w, ca);
-      RealCtl* c = a.CS.ctl + r;
-      ctl.status |= c->status;  // bits of the other blocks
-      *c = ctl;
-    }
+    ctl.step += 1;
+    ctl.t += a.P.dt;
+    prestep(a.P, a.C, ctl, ryr_w, lcc_w, lccv_w,
+            a.CS.rows + (size_t)r * a.P.row_cap * a.P.row_w, ca);
+    RealCtl* c = a.CS.ctl + r;
+    ctl.status |= c->status;  // bits of the other blocks
+    *c = ctl;
     __threadfence();
   }
 }
@@ -168,7 +164,8 @@ __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
 
 // The same for problems of few elements: 32 elements a block, the update dealt
 // to four warps (srs_plain64_update.cuh).  KEYS: the allocation-free form, whose
-// step and seeds come with the launch (NoallocKeys) instead of from RealCtl.
+// step and seeds come with the launch (Plain64Keys) instead of from RealCtl and
+// whose gating is a launch of its own (k_plain64_gate).
 template <bool KEYS>
 __global__ void __launch_bounds__(128) k_plain64_split(const __grid_constant__ Plain64Args a,
                                                        const __grid_constant__ Plain64Keys<KEYS> keys) {
@@ -218,7 +215,54 @@ __global__ void __launch_bounds__(128) k_plain64_split(const __grid_constant__ P
       if (!finite64(ca_new) && status) atomicOr(status, 1u);
     }
   }
-  plain64_tail<KEYS>(a, r, ctl, So, __syncthreads_or(g.fl & 4) != 0);
+  if constexpr (!KEYS) plain64_tail(a, r, ctl, So, __syncthreads_or(g.fl & 4) != 0);
+}
+
+// Gating of an allocation-free step, one block a realization.  It is not left to
+// the last block of the update: that block finds itself by a counter in device
+// memory, and one that all calls share carries the error of two overlapping calls
+// into every later one.  As a chained launch (srs_pdl.cuh) it is the shorter way
+// besides: 64 steps of 3 x 384 elements 680 us against 761 with the counter, its
+// fences and the reload.
+__global__ void __launch_bounds__(128) k_plain64_gate(const __grid_constant__ Plain64Args a,
+                                                      const __grid_constant__ Plain64Keys<true> keys) {
+  __shared__ int32_t s_nb[1024];
+  const int r = blockIdx.x, NR = a.C.NR, NL = a.C.NL;
+  // the channels' elements, which no step writes, before the wait
+  int e0 = 0, e1 = 0;
+  auto elements = [&](int i) {
+    e0 = i < NR ? __ldcg(a.C.ryr_cleft + i) : __ldcg(a.C.lcc_ele + i - NR);
+    e1 = i < NR ? __ldcg(a.C.ryr_jsr + i) : e0;
+  };
+  const int i0 = threadIdx.x;
+  if (i0 < NR + NL) elements(i0);
+  pdl_wait();
+  pdl_next();
+  const double* Sn = a.S_out + (size_t)r * 6 * a.N;
+  int32_t* ryr = a.CS.ryr + (size_t)r * NR;
+  int32_t* lcc = a.CS.lcc + (size_t)r * NL;
+  int32_t* lccv = a.CS.lccv + (size_t)r * NL;
+  double* res = a.CS.res + (size_t)r * (NR + NL);
+  const srs_gate_consts* g = &a.P.gc[0];
+  if (g->ryr_astar_half != 0.0f) {  // coupled gating
+    gate_all(a.P, a.C, 0, keys.seeds[r], keys.step, ryr, lcc, lccv, res, s_nb, threadIdx.x, blockDim.x,
+             [&](int e) { return Sn[e]; }, []() { __syncthreads(); });
+    return;
+  }
+  for (int i = i0; i < NR + NL; i += blockDim.x) {
+    if (i != i0) elements(i);
+    const float c0 = (float)Sn[e0], c1 = (float)Sn[e1];
+    double q = res[i];
+    if (i < NR) {
+      ryr[i] = srs_gate_ryr(g, ryr[i], c0, c1, 0, 0, &q, keys.seeds[r], (uint32_t)i, (uint64_t)keys.step);
+    } else {
+      int st = lcc[i - NR], vs = lccv[i - NR];
+      srs_gate_lcc(g, &st, &vs, c0, &q, keys.seeds[r], (uint32_t)i, (uint64_t)keys.step);
+      lcc[i - NR] = st;
+      lccv[i - NR] = vs;
+    }
+    res[i] = q;
+  }
 }
 
 // Protocol work before the first step of a run (and the t = 0 row).
@@ -272,8 +316,9 @@ int launch_plain64_step(const Plain64Args& a, cudaStream_t st) {
 
 bool plain64_keys_fit(const Plain64Args& a) { return split64(a); }
 int launch_plain64_keys(const Plain64Args& a, const Plain64Keys<true>& k, cudaStream_t st) {
-  launch_pdl(k_plain64_split<true>, dim3((a.N + 31) / 32, a.R), 128, 0, st, a, k);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  cudaError_t e = launch_pdl(k_plain64_split<true>, dim3((a.N + 31) / 32, a.R), 128, 0, st, a, k);
+  if (e == cudaSuccess && !a.P.nogating) e = launch_pdl(k_plain64_gate, a.R, 128, 0, st, a, k);
+  return e == cudaSuccess ? 0 : -1;
 }
 int launch_plain64_prestep(const Plain64Args& a, int write_initial_row, cudaStream_t st) {
   k_plain64_prestep<<<a.R, 32, 0, st>>>(a, write_initial_row);
