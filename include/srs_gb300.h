@@ -197,6 +197,13 @@ int srs_sim_get_config(const srs_sim* s, srs_sim_config* c);
  * this implementation, no counterpart in the reference; srs_gb300/tuner.py
  * searches it. */
 int srs_sim_set_prefetch(srs_sim* s, int element_blocks);
+/* Plain engines whose steps run in one launch: how long a block waits for the
+ * others' arrival at a step's end before it gives up, in rounds of 65,536 polls
+ * (the default, 64, takes a few seconds; 0: none, for tests of this error).  After a
+ * wait that gave up the state is advanced in part: every call that waits for
+ * the device returns SRS_ERR_TIMEOUT until srs_sim_reset.
+ * SRS_ERR_UNSUPPORTED where no step waits (resident engine, large meshes). */
+int srs_sim_set_wait_limit(srs_sim* s, int rounds);
 
 /* ---- line scan (linescan/main.cpp:160-225) --------------------------------
  * PSF-weighted bound-dye fluorescence at sample points on a line, from the

@@ -1111,6 +1111,22 @@ const uint32_t* element_flags(const srs_sim* s, int32_t* stride) {
   return plain ? s->a32.flags : reinterpret_cast<const uint32_t*>(s->ar.geo_b) + 3;
 }
 
+// Error of a bounded wait that gave up, until the next reset: the state is
+// advanced in part.  Called where the stream has been waited for.
+int check_timeout(srs_sim* s) {
+  const volatile unsigned* flag = reinterpret_cast<const volatile unsigned*>(s->h_pin);
+  if (!flag || !*flag) return SRS_OK;
+  return fail(SRS_ERR_TIMEOUT, "a step's barrier did not complete; reset the simulation");
+}
+// The flags and the barriers' counters start afresh (reset, stream idle).
+int clear_timeout(srs_sim* s) {
+  volatile unsigned* flag = reinterpret_cast<volatile unsigned*>(s->h_pin);
+  if (!flag || !*flag) return SRS_OK;
+  *flag = 0;
+  SRS_CUDA(cudaMemsetAsync(s->loop.bar, 0, sizeof(unsigned) * (s->R + 1), s->st));
+  return SRS_OK;
+}
+
 // Realization r in the caller's form (any output may be null): the conversion
 // and the gathering run on the device (k_export_state).  Up to a few MB it
 // writes pinned host memory and the caller's arrays are filled from there;
@@ -1160,21 +1176,13 @@ int export_state(srs_sim* s, int r, double* S, int* ryr, int* lcc, int* lccv, do
   if (launch_export_state(a, s->st)) return fail(SRS_ERR_CUDA, "state export launch failed");
   if (direct) SRS_CUDA(cudaMemcpyAsync(S, s->d_export, ns * sizeof(double), cudaMemcpyDeviceToHost, s->st));
   SRS_CUDA(cudaStreamSynchronize(s->st));
+  SRS_TRY(check_timeout(s));
   if (S && !direct) std::memcpy(S, hS, ns * sizeof(double));
   if (res) std::memcpy(res, hres, s->NCH * sizeof(double));
   if (ryr) std::memcpy(ryr, hi, s->NR * sizeof(int32_t));
   if (lcc) std::memcpy(lcc, hi + s->NR, s->NL * sizeof(int32_t));
   if (lccv) std::memcpy(lccv, hi + s->NR + s->NL, s->NL * sizeof(int32_t));
   return SRS_OK;
-}
-
-// Error of a bounded wait that gave up; the barrier counters start afresh.
-int check_timeout(srs_sim* s) {
-  volatile unsigned* flag = reinterpret_cast<volatile unsigned*>(s->h_pin);
-  if (!flag || !*flag) return SRS_OK;
-  *flag = 0;
-  cudaMemsetAsync(s->loop.bar, 0, sizeof(unsigned) * s->R, s->st);
-  return fail(SRS_ERR_TIMEOUT, "a step's barrier did not complete");
 }
 
 // The plain engines' state buffers 0 and 1 change places.
@@ -1346,17 +1354,20 @@ int setup_plain_loop(srs_sim* s) {
     if (plain_loop_fits(f64, per, (int64_t)s->R * (blocks + 1), s->loop_smem)) break;
   }
   if (per > 4) return SRS_OK;
-  // one upload: the lists, then the barriers' counters
+  // one upload: the lists, then the barriers' counters and the flag of a wait
+  // that gave up
   const size_t n0 = bptr.size(), n1 = n0 + id.size(), n2 = n1 + loc.size();
   bptr.insert(bptr.end(), id.begin(), id.end());
   bptr.insert(bptr.end(), loc.begin(), loc.end());
-  bptr.resize(n2 + s->R, 0);
+  bptr.resize(n2 + s->R + 1, 0);
   int32_t* d;
   SRS_TRY(dev_upload(s, &d, bptr.data(), bptr.size()));
   s->loop.ch_ptr = d;
   s->loop.ch_id = d + n0;
   s->loop.loc = d + n1;
   s->loop.bar = reinterpret_cast<unsigned*>(d + n2);
+  s->loop.gave_up = s->loop.bar + s->R;
+  s->loop.rounds = 64;  // a few seconds
   s->loop.ch_max = most;
   s->loop.per_thread = per;
   s->loop.n_sm = sm_count();
@@ -1365,6 +1376,7 @@ int setup_plain_loop(srs_sim* s) {
 }
 
 int plain_loop_launch(srs_sim* s, int steps) {
+  SRS_TRY(check_timeout(s));
   PlainLoop l = s->loop;
   l.steps = steps;
   l.timeout = reinterpret_cast<unsigned*>(s->h_pin);
@@ -1724,6 +1736,13 @@ int srs_sim_set_prefetch(srs_sim* s, int element_blocks) {
   return SRS_OK;
 }
 
+int srs_sim_set_wait_limit(srs_sim* s, int rounds) {
+  if (!s || rounds < 0) return fail(SRS_ERR_INPUT, "bad argument");
+  if (s->loop.blocks == 0) return fail(SRS_ERR_UNSUPPORTED, "the simulation's steps have no bounded wait");
+  s->loop.rounds = rounds;
+  return SRS_OK;
+}
+
 int srs_sim_get_config(const srs_sim* s, srs_sim_config* c) {
   if (!s || !c) return fail(SRS_ERR_INPUT, "null argument");
   c->engine = s->d.engine;
@@ -1763,7 +1782,7 @@ int srs_sim_reset(srs_sim* s) {
   const ChanBlock blk = chan_block(s);
   std::lock_guard<std::mutex> lock(s->stage_mtx);
   SRS_CUDA(cudaStreamSynchronize(s->st));
-  check_timeout(s);  // a wait that gave up ends with the run that it was in
+  SRS_TRY(clear_timeout(s));  // a wait that gave up ends with the run that it was in
   unsigned char* h = (unsigned char*)stage(s, blk.bytes);
   if (!h) return fail(SRS_ERR_NOMEM, "pinned staging allocation failed");
   RealCtl* ctl = (RealCtl*)h;
@@ -1893,7 +1912,7 @@ int srs_sim_advance_async(srs_sim* s, int64_t n_steps) {
 int srs_sim_synchronize(srs_sim* s) {
   if (!s) return fail(SRS_ERR_INPUT, "null argument");
   SRS_CUDA(cudaStreamSynchronize(s->st));
-  return SRS_OK;
+  return check_timeout(s);
 }
 
 int srs_sim_time_advance(srs_sim* s, int64_t n_steps, float* ms) {
@@ -1909,7 +1928,7 @@ int srs_sim_time_advance(srs_sim* s, int64_t n_steps, float* ms) {
   SRS_CUDA(cudaEventElapsedTime(ms, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  return rc;
+  return rc ? rc : check_timeout(s);
 }
 
 int srs_sim_status(srs_sim* s, int* bits) {
@@ -2545,6 +2564,7 @@ int srs_linescan(srs_sim* s, double* out, double* rest) {
     SRS_CUDA(cudaMemcpyAsync(out, s->d_ls_out, sizeof(double) * s->R * a.n_samples,
                              cudaMemcpyDeviceToHost, s->st));
   SRS_CUDA(cudaStreamSynchronize(s->st));
+  SRS_TRY(check_timeout(s));
   if (rest) std::memcpy(rest, s->ls_rest.data(), sizeof(double) * a.n_samples);
   return SRS_OK;
 }
@@ -3264,6 +3284,7 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
         std::vector<RealCtl> ctl(R);
         SRS_CUDA(cudaMemcpyAsync(ctl.data(), fin.ctl, sizeof(RealCtl) * R, cudaMemcpyDeviceToHost, s->st));
         SRS_CUDA(cudaStreamSynchronize(s->st));
+        SRS_TRY(check_timeout(s));
         for (auto& c : ctl) {
           if (c.status & 1u) return fail(SRS_ERR_NONFINITE, "a realization produced a non-finite Ca value");
           if (c.done) return fail(SRS_ERR_STATE, "a realization is finished; reset it before the adjoint");
@@ -3328,6 +3349,7 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
   }
   SRS_CUDA(cudaStreamSynchronize(s->st));
   SRS_CUDA(cudaGetLastError());
+  SRS_TRY(check_timeout(s));
   if (plain) {  // the blocks' rows in a fixed order
     const double dt = (double)pa.k.dt;
     for (int r = 0; r < R; ++r)
@@ -3422,7 +3444,7 @@ int srs_sim_total_ca(srs_sim* s, double* out) {
   s->launches += 2;
   SRS_CUDA(cudaMemcpyAsync(out, m.out, sizeof(double) * 2 * s->R, cudaMemcpyDeviceToHost, s->st));
   SRS_CUDA(cudaStreamSynchronize(s->st));
-  return SRS_OK;
+  return check_timeout(s);
 }
 
 int srs_write_grid_vtk(srs_sim* s, int r, const char* path, int run, int rank, int n, double t) {

@@ -126,8 +126,10 @@ struct PlainLoop {
   int32_t blocks;         // element blocks per realization
   int32_t per_thread;     // elements a thread (FP64: a lane of each of four warps) takes
   int32_t n_sm;
+  int32_t rounds;         // of 65,536 polls in one wait before a block gives up
   unsigned* bar;          // [R] arrivals at the step barriers, zero before and after a launch
-  unsigned* timeout;      // pinned host word: set when a wait gave up
+  unsigned* gave_up;      // set when a wait gave up: later launches do nothing
+  unsigned* timeout;      // pinned host word, set with it
   int32_t ch_max;         // most channels an element block gates
   const int32_t* ch_ptr;  // [blocks + 1] CSR of the channels each block gates
   const int32_t* ch_id;   // RyR, or NR + LCC
