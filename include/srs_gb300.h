@@ -204,6 +204,10 @@ int srs_sim_set_prefetch(srs_sim* s, int element_blocks);
  * the device returns SRS_ERR_TIMEOUT until srs_sim_reset.
  * SRS_ERR_UNSUPPORTED where no step waits (resident engine, large meshes). */
 int srs_sim_set_wait_limit(srs_sim* s, int rounds);
+/* The same: shared memory that a block asks for beyond its need (default 0).
+ * For tests: with more than the device gives, its launch is refused and the
+ * steps are taken by one launch each. */
+int srs_sim_set_loop_reserve(srs_sim* s, int bytes);
 
 /* ---- line scan (linescan/main.cpp:160-225) --------------------------------
  * PSF-weighted bound-dye fluorescence at sample points on a line, from the

@@ -211,6 +211,7 @@ _SIGS = {
     "srs_sim_get_config": (C.c_int, [_P, C.POINTER(_SimConfig)]),
     "srs_sim_set_prefetch": (C.c_int, [_P, C.c_int]),
     "srs_sim_set_wait_limit": (C.c_int, [_P, C.c_int]),
+    "srs_sim_set_loop_reserve": (C.c_int, [_P, C.c_int]),
     "srs_write_grid_vtk": (C.c_int, [_P, C.c_int, C.c_char_p, C.c_int, C.c_int, C.c_int, C.c_double]),
     "srs_grid_write_vtk": (C.c_int, [_P, _P, _P, C.c_char_p, C.c_int, C.c_int, C.c_int, C.c_double]),
     "srs_box_mesh_default": (None, [C.POINTER(BoxMeshSpec)]),
@@ -428,6 +429,11 @@ class Simulation:
         """srs_sim_set_wait_limit: rounds of 65,536 polls of a step's barrier
         before a block of the looping plain engines gives up."""
         _check(_lib.srs_sim_set_wait_limit(self._h, int(rounds)))
+
+    def set_loop_reserve(self, nbytes):
+        """srs_sim_set_loop_reserve: shared memory that a block of the looping
+        plain engines asks for beyond its need."""
+        _check(_lib.srs_sim_set_loop_reserve(self._h, int(nbytes)))
 
     def set_state(self, r, states=None, ryr=None, lcc=None, lccv=None, residuals=None):
         conv = lambda a, t: None if a is None else np.ascontiguousarray(a, dtype=t)

@@ -97,7 +97,7 @@ struct srs_sim {
   cudaGraphExec_t graph_plain_alt = nullptr;  // ... captured when the buffers were exchanged
   int graph_plain_len = 0;
   PlainLoop loop{};  // plain engines: steps in one launch (blocks 0: not used)
-  size_t loop_smem = 0;
+  size_t loop_smem = 0, loop_reserve = 0;
   void* h_stage = nullptr;         // pinned: exchanges larger than that
   size_t h_stage_bytes = 0;
   std::mutex stage_mtx;            // held while staging or d_export is in use
@@ -1375,7 +1375,8 @@ int setup_plain_loop(srs_sim* s) {
   return SRS_OK;
 }
 
-int plain_loop_launch(srs_sim* s, int steps) {
+// refused: the device does not take the cooperative launch (nothing was enqueued)
+int plain_loop_launch(srs_sim* s, int steps, bool* refused) {
   SRS_TRY(check_timeout(s));
   PlainLoop l = s->loop;
   l.steps = steps;
@@ -1385,33 +1386,37 @@ int plain_loop_launch(srs_sim* s, int steps) {
     Plain64Args a = s->a64;
     a.S_in = s->d_S[0];
     a.S_out = s->d_S[1];
-    rc = launch_plain64_loop(a, l, s->loop_smem, s->st);
+    rc = launch_plain64_loop(a, l, s->loop_smem + s->loop_reserve, s->st);
   } else {
     Plain32Args a = s->a32;
     a.M_in = s->d_M[0];
     a.I_in = s->d_I[0];
     a.M_out = s->d_M[1];
     a.I_out = s->d_I[1];
-    rc = launch_plain32_loop(a, l, s->loop_smem, s->st);
+    rc = launch_plain32_loop(a, l, s->loop_smem + s->loop_reserve, s->st);
   }
-  s->launches++;
-  if (rc) return fail(SRS_ERR_CUDA, std::string("step loop launch: ") + cudaGetErrorString(cudaGetLastError()));
+  *refused = rc != 0;
+  if (rc) cudaGetLastError();  // an error of the device itself comes again with the next launch
+  else s->launches++;
   return SRS_OK;
 }
 
 // n plain steps starting from buffer 0: in launches of up to 4096 steps where
 // the problem fits on the device, else one launch per step (graph-replayed).  A
 // single step is the shorter without the cooperative launch: a call of one step
-// 20.8 against 22.4 us, of two 32 against 28.
+// 20.8 against 22.4 us, of two 32 against 28.  Whether it fits was asked when the
+// simulation was made; a launch that is refused all the same goes to the other form.
 int plain_steps(srs_sim* s, int64_t n) {
-  if (s->loop.blocks > 0 && n > 1) {
-    for (int64_t done = 0; done < n; done += 4096)
-      SRS_TRY(plain_loop_launch(s, (int)std::min<int64_t>(4096, n - done)));
-    return SRS_OK;
+  int64_t done = 0;  // even where the one form hands over to the other
+  while (s->loop.blocks > 0 && n - done > 1) {
+    const int k = (int)std::min<int64_t>(4096, n - done);
+    bool refused = false;
+    SRS_TRY(plain_loop_launch(s, k, &refused));
+    if (refused) s->loop.blocks = 0;
+    else done += k;
   }
   const int G = 32;  // launches per graph replay (even)
-  int64_t done = 0;
-  if (n >= G) {
+  if (n - done >= G) {
     if (!s->graph_plain) {
       cudaGraph_t g;
       SRS_CUDA(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
@@ -1740,6 +1745,12 @@ int srs_sim_set_wait_limit(srs_sim* s, int rounds) {
   if (!s || rounds < 0) return fail(SRS_ERR_INPUT, "bad argument");
   if (s->loop.blocks == 0) return fail(SRS_ERR_UNSUPPORTED, "the simulation's steps have no bounded wait");
   s->loop.rounds = rounds;
+  return SRS_OK;
+}
+
+int srs_sim_set_loop_reserve(srs_sim* s, int bytes) {
+  if (!s || bytes < 0) return fail(SRS_ERR_INPUT, "bad argument");
+  s->loop_reserve = bytes;
   return SRS_OK;
 }
 
