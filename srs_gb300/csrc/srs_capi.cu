@@ -13,11 +13,11 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "srs_engine.h"
 #include "srs_host.h"
+#include "srs_parallel.h"
 
 using namespace srs;
 
@@ -567,20 +567,6 @@ int setup_plain32(srs_sim* s) {
   SRS_TRY(dev_alloc(s, &s->d_CIq, (size_t)s->R * N));
   SRS_TRY(upload_channels_engine_order(s));
   return SRS_OK;
-}
-
-// f(0) .. f(n - 1), dealt in turn to at most `most` host threads (the caller
-// among them).
-template <class F>
-void host_parallel(int n, int most, F&& f) {
-  const int nt = std::max(1, std::min({n, most, (int)std::thread::hardware_concurrency()}));
-  auto work = [&](int t) {
-    for (int i = t; i < n; i += nt) f(i);
-  };
-  std::vector<std::thread> pool;
-  for (int t = 1; t < nt; ++t) pool.emplace_back(work, t);
-  work(0);
-  for (auto& th : pool) th.join();
 }
 
 // ---- FP32 resident engine ----------------------------------------------------

@@ -1,0 +1,41 @@
+// srs_parallel.h — loops of the set-up and of reset over several host threads.
+#pragma once
+#include <algorithm>
+#include <atomic>
+#include <exception>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace srs {
+
+// f(0) .. f(n - 1), taken in turn by at most `most` host threads (the caller
+// among them).  Threads that cannot be created are done without; an exception of
+// f ends the loop and is thrown again in the caller.
+template <class F>
+void host_parallel(int n, int most, F&& f) {
+  const int nt = std::max(1, std::min({n, most, (int)std::thread::hardware_concurrency()}));
+  std::atomic<int> next{0};
+  std::exception_ptr error;
+  std::mutex mtx;
+  auto work = [&]() noexcept {
+    try {
+      for (int i; (i = next.fetch_add(1)) < n;) f(i);
+    } catch (...) {
+      next.store(n);
+      std::lock_guard<std::mutex> lock(mtx);
+      if (!error) error = std::current_exception();
+    }
+  };
+  std::vector<std::thread> pool;
+  try {
+    pool.reserve(nt - 1);
+    while ((int)pool.size() < nt - 1) pool.emplace_back(work);
+  } catch (...) {  // the threads that there are do the rest
+  }
+  work();
+  for (auto& th : pool) th.join();
+  if (error) std::rethrow_exception(error);
+}
+
+}  // namespace srs
