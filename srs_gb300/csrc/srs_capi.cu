@@ -112,6 +112,7 @@ struct srs_sim {
   // line scan
   LinescanArgs ls{};
   std::vector<double> ls_rest;  // F at the equilibrium state
+  std::vector<void*> ls_allocs;  // device buffers of this set-up, freed with it
   double* d_ls_out = nullptr;
   std::vector<int32_t> ls_ptr_h, ls_col_h;  // host copy of the line-scan CSR
   std::vector<double> ls_w_h;
@@ -149,6 +150,19 @@ int dev_upload(srs_sim* s, T** dst, const T* src, size_t n) {
   *dst = (T*)p;
   return SRS_OK;
 }
+// Device buffers made in its scope belong to the line scan's set-up (the weights
+// in their forms, and the adjoint's map of them) instead of to the simulation.
+struct LinescanBuffers {
+  srs_sim* s;
+  size_t first;
+  explicit LinescanBuffers(srs_sim* sim) : s(sim), first(sim->allocs.size()) {}
+  ~LinescanBuffers() {
+    s->ls_allocs.insert(s->ls_allocs.end(), s->allocs.begin() + first, s->allocs.end());
+    s->allocs.resize(first);
+  }
+  LinescanBuffers(const LinescanBuffers&) = delete;
+  LinescanBuffers& operator=(const LinescanBuffers&) = delete;
+};
 // 32-byte records as their first halves, then their second halves.
 template <class Rec>
 std::vector<float4> record_halves(const std::vector<Rec>& rec) {
@@ -1705,6 +1719,7 @@ void srs_sim_destroy(srs_sim* s) {
   if (s->graph_plain_alt) cudaGraphExecDestroy(s->graph_plain_alt);
   if (s->st) cudaStreamSynchronize(s->st);
   for (void* p : s->allocs) cudaFree(p);
+  for (void* p : s->ls_allocs) cudaFree(p);
   for (auto& b : s->adj_bufs) cudaFree(b.first);
   if (s->h_stage) cudaFreeHost(s->h_stage);
   if (s->h_pin) cudaFreeHost(s->h_pin);
@@ -2312,6 +2327,7 @@ namespace {
 int linescan_csr(srs_sim* s) {
   LinescanArgs& a = s->ls;
   if (a.ptr) return SRS_OK;
+  LinescanBuffers own(s);
   int32_t* dp;
   SRS_TRY(dev_upload(s, (int32_t**)&a.col, s->ls_col_h.data(), s->ls_col_h.size()));
   SRS_TRY(dev_upload(s, (double**)&a.w, s->ls_w_h.data(), s->ls_w_h.size()));
@@ -2478,8 +2494,7 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
     add_grid(D[0], D[1], D[3], a1, D[4], D[5]);
   }
   std::vector<int32_t> ptr(ns + 1, 0), col;
-  std::vector<double> w, pad(ns, 0.0);
-  s->ls_rest.assign(ns, 0.0);
+  std::vector<double> w, pad(ns, 0.0), rests(ns, 0.0);
   std::vector<double> S6;
   initial_states(m, s->p, &S6);
   // samples are independent: their rows are built by up to eight host threads
@@ -2505,7 +2520,7 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
       if (rx * rx + ry * ry + rz * rz < d->r_thresh) pd += pv[q] * d->f0_pad * pdf(rx, ry, rz);
     }
     pad[i] = pd;
-    s->ls_rest[i] = pd + rest;
+    rests[i] = pd + rest;
   };
   host_parallel(ns, (size_t)ns * (m.N + px.size()) < 100000 ? 1 : 8, sample);
   for (int i = 0; i < ns; ++i) {
@@ -2518,12 +2533,18 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
   s->ls_col_h = col;
   s->ls_w_h = w;
   s->ls_pad_h = pad;
+  s->ls_rest = rests;
   s->ls_version++;
+  // a new scan takes the place of the one before
+  SRS_CUDA(cudaStreamSynchronize(s->st));
+  for (void* p : s->ls_allocs) cudaFree(p);
+  s->ls_allocs.clear();
   LinescanArgs& a = s->ls;
   a.n_samples = ns;
   a.n_state = (int32_t)eng_count(s);
   a.ptr = nullptr;  // uploaded by linescan_csr
   a.tptr = nullptr;
+  LinescanBuffers own(s);
   SRS_TRY(dev_upload(s, (double**)&a.pad, pad.data(), pad.size()));
   if (s->d.precision != SRS_FP64) {
     std::vector<double> rd(eng_count(s), 0.0);
@@ -2632,6 +2653,7 @@ int adjoint_setup(srs_sim* s) {
     SRS_TRY(dev_upload(s, &s->d_ryr_s_cl, scl.data(), scl.size()));
     SRS_TRY(dev_upload(s, &s->d_ryr_s_js, sjs.data(), sjs.size()));
   }
+  LinescanBuffers own(s);
   const int ns = s->ls.n_samples;
   std::vector<int32_t> cnt(NE + 1, 0);
   for (size_t q = 0; q < s->ls_col_h.size(); ++q) cnt[s->ls_col_h[q] + 1]++;
