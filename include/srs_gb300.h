@@ -340,7 +340,7 @@ typedef struct srs_adjoint_desc {
   const double* target;  /* [R][n_steps/tick_every][n_samples] ([n_steps/tick_every]
                             [n_samples] with SRS_ADJ_MEAN_TRACE), or NULL (zero) */
   int flags;
-  int threads_per_cta;   /* reverse-sweep kernel: a multiple of 32 in [64, 512] (0: chosen
+  int threads_per_cta;   /* reverse-sweep kernel: a multiple of 32 in [64, 640] (0: chosen
                             by the library) */
   int cta_partitions;    /* forward partitions per reverse-sweep CTA, a divisor of the
                             cluster size (0: chosen by the library) */

@@ -99,7 +99,7 @@ __device__ __forceinline__ float tick_injection(const AdjArgs& a, const double* 
 // are computed in packed pairs (adj_local) and interior elements' codes are
 // offsets in this CTA (no look-up of the owner's window): 5 % together.
 template <int C>
-__global__ void __launch_bounds__(640, 1) k_adjoint32(AdjArgs a) {
+__global__ void __launch_bounds__(ADJ_MAX_THREADS, 1) k_adjoint32(AdjArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int P = a.P;           // stride of the forward engine's partitions
   const int msub = a.m_sub;    // forward partitions per CTA

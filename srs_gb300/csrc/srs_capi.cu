@@ -3119,8 +3119,9 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
     aa.ak = ak;
     const int n_ent = 2 * NR + NL;
     if (d->threads_per_cta != 0 &&
-        (d->threads_per_cta % 32 || d->threads_per_cta < 64 || d->threads_per_cta > 512))
-      return fail(SRS_ERR_INPUT, "threads_per_cta must be a multiple of 32 in [64, 512]");
+        (d->threads_per_cta % 32 || d->threads_per_cta < 64 || d->threads_per_cta > ADJ_MAX_THREADS))
+      return fail(SRS_ERR_INPUT, "threads_per_cta must be a multiple of 32 in [64, " +
+                                     std::to_string(ADJ_MAX_THREADS) + "]");
     if (d->cta_partitions < 0 || (d->cta_partitions > 0 && s->C % d->cta_partitions))
       return fail(SRS_ERR_INPUT, "cta_partitions must divide the cluster size");
     // CTA grouping: m forward partitions per CTA (clusters of C/m CTAs), the
@@ -3135,7 +3136,7 @@ int srs_adjoint(srs_sim* s, const srs_adjoint_desc* d, srs_adjoint_out* out) {
     bool best_own = false, best_stage = false;
     double best_cost = 1e300;
     const std::vector<int> thr_list =
-        d->threads_per_cta ? std::vector<int>{d->threads_per_cta} : std::vector<int>{256, 512, 640};
+        d->threads_per_cta ? std::vector<int>{d->threads_per_cta} : std::vector<int>{256, 512, ADJ_MAX_THREADS};
     for (int thr : thr_list) {
       for (int m = 1; m <= s->C; ++m) {
         if (s->C % m || (d->cta_partitions && m != d->cta_partitions)) continue;

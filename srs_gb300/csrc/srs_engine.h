@@ -318,6 +318,7 @@ struct AdjConsts {
   float kb_off[3];
 };
 
+constexpr int ADJ_MAX_THREADS = 640;  // of a reverse-sweep CTA, at 96 registers
 struct AdjArgs {
   int32_t R, P, off_bits;  // P: forward partition stride; off_bits of the codes in geo
   int32_t m_sub;           // forward partitions per CTA (CTA slots m_sub * P)
