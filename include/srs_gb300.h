@@ -381,6 +381,13 @@ int srs_grid_write_vtk(const srs_grid* g, const double* states, const int* ryr_s
  * engine's adjoint (packed = 1); every fifth value through the single form.
  * For tests of the device codec against a restatement. */
 int srs_comp_round_trip(const float* in, float* out, int64_t n, int packed);
+/* The FP32 engines' and the logarithm's division without special cases against
+ * the IEEE one, on the device: every significand of the numerator (times 2^ea)
+ * over the n_b significands b_first + i b_step of the denominator (times 2^eb),
+ * exponents in [-60, 59].  wrong[3]: differing quotients, reciprocals (every
+ * significand), and quotients of the logarithm.  All 2^46 pairs: b_first = 0,
+ * b_step = 1, n_b = 2^23. */
+int srs_division_check(int b_first, int b_step, int n_b, int ea, int eb, int64_t* wrong);
 
 /* ---- synthetic meshes (no reference counterpart beyond the file format of
  * mesh/main.cpp:1305-1364): box dyad, see the generator for the geometry. */

@@ -221,6 +221,7 @@ _SIGS = {
     "srs_linescan_setup": (C.c_int, [_P, C.POINTER(LinescanDesc), C.POINTER(C.c_int)]),
     "srs_linescan": (C.c_int, [_P, _P, _P]),
     "srs_sim_total_ca": (C.c_int, [_P, _P]),
+    "srs_division_check": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P]),
     "srs_comp_round_trip": (C.c_int, [_P, _P, C.c_int64, C.c_int]),
     "srs_batch_create": (C.c_int, [_P, C.c_int, C.c_int, C.POINTER(_P)]),
     "srs_batch_destroy": (None, [_P]),
@@ -266,6 +267,14 @@ def library():
 def explicit_step_fp64_noalloc(desc):
     """srs_explicit_step_fp64_noalloc on a filled NoallocStep."""
     _check(_lib.srs_explicit_step_fp64_noalloc(C.byref(desc)))
+
+
+def division_check(b_first, b_step, n_b, ea=0, eb=0):
+    """srs_division_check: quotients, reciprocals and quotients of the logarithm
+    that differ from the correctly rounded ones."""
+    wrong = np.zeros(3, np.int64)
+    _check(_lib.srs_division_check(int(b_first), int(b_step), int(n_b), int(ea), int(eb), _ptr(wrong)))
+    return tuple(int(v) for v in wrong)
 
 
 def comp_round_trip(values, packed=False):

@@ -11,6 +11,7 @@
 // double precision whatever the precision of the state.
 #include "srs_comp.h"
 #include "srs_engine.h"
+#include "srs_math.h"
 
 namespace srs {
 
@@ -148,6 +149,46 @@ __global__ void k_comp_round_trip(const float* in, float* out, int64_t n, int pa
   const float r[5] = {c4.x, c4.y, c4.z, c4.w, comp_load1(comp_store1(v[4]))};
   for (int k = 0; k < 5; ++k)
     if (i + k < n) out[i + k] = r[k];
+}
+
+// srs_div_in_range against the division: all 2^23 significands of a, of both
+// signs in turn, over n_b of b (blockIdx.y; step b_step), a times 2^ea, b 2^eb.
+// wrong: quotients, then reciprocals of every b, then quotients (m - 1) / (m + 1)
+// of srs_logf over every float m from 1/2 to 2 (the last two by blocks of y 0).
+__global__ void __launch_bounds__(256) k_division_check(int32_t b_first, int32_t b_step, int32_t n_b, int32_t ea,
+                                                        int32_t eb, int64_t* wrong) {
+  constexpr uint32_t n = 1u << 23;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  auto scaled = [](uint32_t significand, int e) {
+    return __uint_as_float((uint32_t)(127 + e) << 23 | (significand & (n - 1)));
+  };
+  int64_t q = 0, y = 0, l = 0;
+  for (int32_t i = blockIdx.y; i < n_b; i += gridDim.y) {
+    const float b = scaled((uint32_t)b_first + (uint32_t)i * (uint32_t)b_step, eb);
+    for (uint32_t s = t; s < n; s += nt) {
+      const float a = s & 1 ? -scaled(s, ea) : scaled(s, ea);
+      q += srs_div_in_range(a, b) != __fdiv_rn(a, b);
+    }
+  }
+  if (blockIdx.y == 0) {
+    for (uint32_t s = t; s < n; s += nt) y += srs_rcp_newton(scaled(s, eb)) != __frcp_rn(scaled(s, eb));
+    for (uint32_t s = t; s < 2 * n; s += nt) {
+      const float m = scaled(s, s < n ? -1 : 0);
+      const float a = __fsub_rn(m, 1.0f), b = __fadd_rn(m, 1.0f);
+      l += srs_div_in_range(a, b) != __fdiv_rn(a, b);
+    }
+  }
+  auto add = [&](int k, int64_t v) {
+    if (v) atomicAdd(reinterpret_cast<unsigned long long*>(wrong + k), (unsigned long long)v);
+  };
+  add(0, q);
+  add(1, y);
+  add(2, l);
+}
+int launch_division_check(int32_t b_first, int32_t b_step, int32_t n_b, int32_t ea, int32_t eb, int64_t* wrong,
+                          cudaStream_t st) {
+  k_division_check<<<dim3(128, n_b < 256 ? n_b : 256), 256, 0, st>>>(b_first, b_step, n_b, ea, eb, wrong);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 int launch_comp_round_trip(const float* in, float* out, int64_t n, int packed, cudaStream_t st) {

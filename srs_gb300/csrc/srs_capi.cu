@@ -274,7 +274,7 @@ void fill_protocol_consts(srs_sim* s) {
 }
 
 // |Ca| (uM) below which both divisions of the FP32 element update are in the
-// range of div_in_range, or -1 where the parameters leave it open:
+// range of srs_div_in_range, or -1 where the parameters leave it open:
 //   SERCA: den = sd0 + sd1 Ki + sd2 Ki^2, num = -sn0 + sn1 Ki + 3.2e12 Ki^2,
 //   Ki = (c inv_kdi)^2; sd0 bounds den from below, sn0 keeps num off the
 //   smallest magnitudes (it vanishes only through cancellation, whose
@@ -3527,6 +3527,23 @@ int srs_comp_round_trip(const float* in, float* out, int64_t n, int packed) {
     return fail(SRS_ERR_CUDA, "codec kernel launch failed");
   SRS_CUDA(cudaMemcpy(out, b.d[1], n * sizeof(float), cudaMemcpyDeviceToHost));
   return SRS_OK;
+}
+
+int srs_division_check(int b_first, int b_step, int n_b, int ea, int eb, int64_t* wrong) {
+  if (!wrong || n_b < 1 || n_b > (1 << 23) || ea < -60 || ea > 59 || eb < -60 || eb > 59)
+    return fail(SRS_ERR_INPUT, "bad argument");
+  SRS_TRY(check_device());
+  int64_t* d = nullptr;
+  SRS_CUDA(cudaMalloc(&d, 3 * sizeof(int64_t)));
+  cudaError_t e = cudaMemset(d, 0, 3 * sizeof(int64_t));
+  // launches of at most 4096 significands of b, tens of milliseconds each
+  for (int i = 0; e == cudaSuccess && i < n_b; i += 4096)
+    if (launch_division_check((int32_t)((uint32_t)b_first + (uint32_t)i * (uint32_t)b_step), b_step,
+                              std::min(4096, n_b - i), ea, eb, d, 0))
+      e = cudaErrorLaunchFailure;
+  if (e == cudaSuccess) e = cudaMemcpy(wrong, d, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? SRS_OK : fail(SRS_ERR_CUDA, std::string("division check: ") + cudaGetErrorString(e));
 }
 
 int srs_box_mesh_write(const srs_box_mesh_spec* spec, const char* base, int* rep_i, double* rep_a0) {

@@ -63,7 +63,7 @@ struct Consts32 {
   float dc0;
   float lccA[2], lccE[2], lccB;
   // |Ca| below which the divisions of the element update stay in the range of
-  // div_in_range (srs_fp32_update.cuh); negative: never
+  // srs_div_in_range (srs_math.h); negative: never
   float div_cmax;
 };
 
@@ -300,6 +300,8 @@ struct MassArgs {
 };
 int total_ca_blocks(int n_state, int R, int n_sm);
 int launch_total_ca(const MassArgs& a, int R, int blocks, cudaStream_t st);
+int launch_division_check(int32_t b_first, int32_t b_step, int32_t n_b, int32_t ea, int32_t eb, int64_t* wrong,
+                          cudaStream_t st);
 int launch_comp_round_trip(const float* in, float* out, int64_t n, int packed, cudaStream_t st);
 
 // ---- pathwise adjoint (k_adjoint.cu) ---------------------------------------
