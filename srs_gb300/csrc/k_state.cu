@@ -81,14 +81,18 @@ int launch_export_lambda(const ExportLambdaArgs& a, int R, cudaStream_t st) {
 }
 
 // One state for every realization: dst[r][i] = src[i].
-__global__ void __launch_bounds__(256) k_broadcast_state(const double* src, double* dst, size_t n) {
+template <class T>
+__global__ void __launch_bounds__(256) k_broadcast_state(const T* src, T* dst, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     dst[blockIdx.y * n + i] = src[i];
 }
-int launch_broadcast_state(const double* src, double* dst, size_t n, int R, cudaStream_t st) {
+template <class T>
+int launch_broadcast_state(const T* src, T* dst, size_t n, int R, cudaStream_t st) {
   const size_t most = (n + 255) / 256;
   k_broadcast_state<<<dim3((unsigned)(most < 304 ? most : 304), R), 256, 0, st>>>(src, dst, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
+template int launch_broadcast_state(const double*, double*, size_t, int, cudaStream_t);
+template int launch_broadcast_state(const float*, float*, size_t, int, cudaStream_t);
 
 }  // namespace srs

@@ -104,6 +104,7 @@ struct srs_sim {
   unsigned char* h_pin = nullptr;  // pinned: the timeout flag of the kernels' waits, staging
   size_t h_pin_bytes = 0;
   double* d_S0 = nullptr;          // FP64 engine: the equilibrium state [6][N]
+  float* d_I0 = nullptr;           // FP32 engines: the equilibrium's immobile buffer, where not at rest
   int32_t* d_eng_of_ref = nullptr;  // FP32 engines: [N]
   double* d_export = nullptr;      // a realization's state in the caller's form (large meshes)
   // every realization has finished its run (known for parameter sets without
@@ -1089,8 +1090,22 @@ int upload_state(srs_sim* s, int r, const double* S6) {
   return SRS_OK;
 }
 
+// The FP32 engines' rest is the equilibrium but for the immobile buffer of
+// elements whose troponin indicator is neither 0 nor 1: the equilibrium has
+// troponin times the indicator there (initial_states), the rest has it once.
+int setup_reset32(srs_sim* s) {
+  const size_t NE = eng_count(s);
+  std::vector<double> S6;
+  initial_states(s->m, s->p, &S6);
+  std::vector<float4> M(NE);
+  std::vector<float> I(NE);
+  to_engine_fp32(s, S6.data(), M.data(), I.data());
+  if (std::all_of(I.begin(), I.end(), [](float x) { return x == 0.0f; })) return SRS_OK;
+  return dev_upload(s, &s->d_I0, I.data(), NE);
+}
+
 // The equilibrium state of every realization (ResetDefaultGridStates).  The
-// FP32 engines hold deviations from it: all zero, in every array.
+// FP32 engines hold deviations from rest: zero, but for setup_reset32's.
 int reset_states(srs_sim* s) {
   if (s->d.precision == SRS_FP64) {
     if (launch_broadcast_state(s->d_S0, s->d_S[0], (size_t)6 * s->N, s->R, s->st))
@@ -1099,7 +1114,9 @@ int reset_states(srs_sim* s) {
   }
   const size_t n = (size_t)s->R * eng_count(s);
   SRS_CUDA(cudaMemsetAsync(s->d_M[0], 0, n * sizeof(float4), s->st));
-  SRS_CUDA(cudaMemsetAsync(s->d_I[0], 0, n * sizeof(float), s->st));
+  if (!s->d_I0) SRS_CUDA(cudaMemsetAsync(s->d_I[0], 0, n * sizeof(float), s->st));
+  else if (launch_broadcast_state(s->d_I0, s->d_I[0], eng_count(s), s->R, s->st))
+    return fail(SRS_ERR_CUDA, "state reset launch failed");
   return clear_compensation(s, 0, n);
 }
 
@@ -1694,6 +1711,7 @@ int srs_sim_create(const srs_grid* g, const srs_params* ps, const srs_sim_desc* 
       }
       if (!rc) rc = setup_resident(s, C, threads);
     }
+    if (!rc && d->precision == SRS_FP32) rc = setup_reset32(s);
   }
   if (rc) {
     srs_sim_destroy(s);

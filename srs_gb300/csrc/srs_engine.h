@@ -274,7 +274,8 @@ struct ExportLambdaArgs {
   double* g;                    // [R][6][N]
 };
 int launch_export_lambda(const ExportLambdaArgs& a, int R, cudaStream_t st);
-int launch_broadcast_state(const double* src, double* dst, size_t n, int R, cudaStream_t st);
+template <class T>  // double, float
+int launch_broadcast_state(const T* src, T* dst, size_t n, int R, cudaStream_t st);
 
 // ---- total Ca per compartment (k_mass.cu) ------------------------------------
 struct MassArgs {
