@@ -372,7 +372,7 @@ int launch_plain32_prestep(const Plain32Args& a, int write_initial_row, cudaStre
 // ===========================================================================
 // Resident FP32 engine: kernel in k_resident.cuh, instantiated in k_res_*.cu
 // ===========================================================================
-size_t resident_smem_bytes(int P, int NR, int NL, int n_chtet, int n_entries) {
+size_t resident_smem_bytes(int P, int NR, int NL, int n_chtet, int n_entries, bool gc) {
   // per element: two state buffers, the compact compensation terms of the
   // mobile species, the immobile buffer and its compact compensation term
   size_t b = (size_t)P * (2 * sizeof(float4) + sizeof(ushort4) + sizeof(float) + sizeof(uint16_t));
@@ -385,6 +385,7 @@ size_t resident_smem_bytes(int P, int NR, int NL, int n_chtet, int n_entries) {
   b += (size_t)(n_chtet + 1) * sizeof(int32_t);
   b = (b + 15) & ~(size_t)15;
   b += (size_t)n_entries * sizeof(float2);
+  if (gc) b += 2 * sizeof(srs_gate_consts);
   return b;
 }
 

@@ -24,7 +24,6 @@ namespace srs {
 //   aligned), then the channel block (used by rank 0).
 struct ResidentSmemTail {
   RealCtl ctl;
-  srs_gate_consts gc[2];  // of Protocol, by potential
   int64_t next_ev;        // next step with protocol work
   uint32_t base[2][16];  // cluster addresses of buf[b] in CTA rank q
   int32_t bad;
@@ -222,12 +221,14 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
   double* s_res = reinterpret_cast<double*>(
       (reinterpret_cast<uintptr_t>(s_lrest + NL) + 7) & ~(uintptr_t)7);
   float* s_flux = reinterpret_cast<float*>(s_res + NCH);
-  const ChanSmem cs{s_ccl, s_cjs, s_clc, s_lrest, s_ryr, s_lcc, s_lccv, s_nb, s_res, s_flux, tail->gc};
   // channel-entry CSR of partition 0, staged once per launch: (channel's index
   // in s_flux, +-1 / V0)
   int32_t* s_cptr = reinterpret_cast<int32_t*>(s_flux + NCH);
   float2* s_clist = reinterpret_cast<float2*>(
       (reinterpret_cast<uintptr_t>(s_cptr + a.n_chtet[0] + 1) + 15) & ~(uintptr_t)15);
+  // the gating constants behind them, where they fit (else in global memory)
+  srs_gate_consts* s_gc = reinterpret_cast<srs_gate_consts*>(s_clist + 2 * NR + NL);
+  const ChanSmem cs{s_ccl, s_cjs, s_clc, s_lrest, s_ryr, s_lcc, s_lccv, s_nb, s_res, s_flux, a.gc ? a.gc : s_gc};
 
   uint32_t rank = 0;
   if constexpr (C > 1) {
@@ -240,11 +241,11 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
   const int nthr = blockDim.x;
   const int n_loc = a.n_local[rank];
   const int n_ch = (rank == 0) ? a.n_chtet[0] : 0;  // channel elements: rank 0 only
-  // In partition 0 the channel group (the first resident_group threads) owns
+  // In partition 0 the channel group (the first a.group threads) owns
   // the channel elements, gates the channels right after updating them and runs
   // the protocol; the other warps share the rest.  Elsewhere every thread
   // strides over the whole partition.
-  const int ng = resident_group(nthr);
+  const int ng = a.group;
   const bool split = (rank == 0) && (n_ch > 0) && (nthr > ng);
   const bool chan_group = split && tid < ng;
   const bool chan_warp = (rank == 0) && (warp == 0);
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(Resi
       tail->base[1][q] = (C > 1) ? map_rank(smem_addr(buf1), q) : smem_addr(buf1);
     }
   }
-  if (tid < 2) tail->gc[tid] = P_.gc[tid];
+  if (tid < 2 && !a.gc) s_gc[tid] = P_.gc[tid];
   if (tid == 0) tail->bad = 0;
   // address of rank 0's termination flags, as seen from this CTA
   uint32_t done_addr0 = smem_addr(&tail->done_flag[0]);

@@ -92,6 +92,7 @@ struct srs_sim {
   size_t smem = 0;
   std::vector<int> part_start, part_len, part_nch, part_nint;  // resident partitions
   int ch_interior = 0;
+  srs_gate_consts* d_gc = nullptr;  // [2] Protocol's, where shared memory does not hold them
   int64_t launches = 0;
   cudaGraphExec_t graph_plain = nullptr;      // steps from state buffer 0 ...
   cudaGraphExec_t graph_plain_alt = nullptr;  // ... captured when the buffers were exchanged
@@ -587,12 +588,50 @@ int setup_plain32(srs_sim* s) {
 // ---- FP32 resident engine ----------------------------------------------------
 // Elements of partition 0 (the channels'): every element thread of the
 // cluster gets the same number, the channel group takes the channel elements.
-int partition0_size(int N, int n_ch, int C, int threads) {
+int partition0_size(int N, int n_ch, int C, int threads, int ng) {
   if (C == 1) return N;
-  const int ng = resident_group(threads);
   if (n_ch <= 0 || threads <= ng) return (int)((int64_t)N / C);
   const double lam = (double)(N - n_ch) / ((double)C * threads - ng);
   return std::min(N, std::max(n_ch, n_ch + (int)std::lround(lam * (threads - ng))));
+}
+
+// How a mesh lies in clusters of C CTAs: the channel group, whether the gating
+// constants are staged in shared memory, the longest partition and the shared
+// memory of a CTA.  The first of the forms that fits, the fastest first; ok: it
+// does.
+struct ResidentFit {
+  int group = 0, P = 0;
+  bool gc = true, ok = false;
+  size_t smem = 0;
+};
+ResidentFit resident_fit(const srs_sim* s, int n_ch, int C, int threads) {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  ResidentFit first;
+  for (int form = 0; form < 4; ++form) {
+    ResidentFit f;
+    f.group = resident_group(threads, form < 2);
+    f.gc = form % 2 == 0;
+    const int len0 = partition0_size(s->N, n_ch, C, threads, f.group);
+    f.P = len0;
+    if (C > 1) f.P = std::max(f.P, (s->N - len0 + C - 2) / (C - 1));
+    f.P = (f.P + 3) & ~3;
+    f.smem = resident_smem_bytes(f.P, s->NR, s->NL, n_ch, 2 * s->NR + s->NL, f.gc);
+    int bits = 1, rank_bits = 0;
+    while ((1 << bits) < f.P) ++bits;
+    while ((1 << rank_bits) < C) ++rank_bits;
+    f.ok = f.smem <= (size_t)optin && n_ch <= len0 && bits + rank_bits <= 16;
+    if (f.ok) return f;
+    if (form == 0) first = f;
+  }
+  return first;
+}
+int channel_elements(const Mesh& m) {
+  std::vector<char> ch(m.N, 0);
+  for (int i = 0; i < m.NR; ++i) ch[m.ryr_ele[i]] = ch[m.ryr_jsr[i]] = 1;
+  for (int i = 0; i < m.NL; ++i) ch[m.lcc_ele[i]] = 1;
+  return (int)std::count(ch.begin(), ch.end(), 1);
 }
 
 // Co-resident clusters of C CTAs at one CTA per SM.  It depends on how the
@@ -621,12 +660,7 @@ int clusters_at_one_per_sm(int C, size_t optin) {
 // 1024 realizations (3 x 512) against 100 (5 x 320), and two rounds of 36
 // clusters for 37 realizations.
 int choose_resident(const srs_sim* s, int C_in, int T_in, int* C_out, int* T_out) {
-  const Mesh& m = s->m;
-  std::vector<char> ch(s->N, 0);
-  for (int i = 0; i < m.NR; ++i) ch[m.ryr_ele[i]] = ch[m.ryr_jsr[i]] = 1;
-  for (int i = 0; i < m.NL; ++i) ch[m.lcc_ele[i]] = 1;
-  int n_ch = 0;
-  for (char c : ch) n_ch += c;
+  const int n_ch = channel_elements(s->m);
   int dev = 0, n_sm = 0, optin = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -643,15 +677,10 @@ int choose_resident(const srs_sim* s, int C_in, int T_in, int* C_out, int* T_out
     int one = 0;  // clusters at one CTA per SM
     for (int T : {160, 192, 256, 320, 384, 512, 640}) {
       if (T_in > 0) T = T_in;
-      const int len0 = partition0_size(s->N, n_ch, C, T);
-      int P = len0;
-      if (C > 1) P = std::max(P, (s->N - len0 + C - 2) / (C - 1));
-      P = (P + 3) & ~3;
-      const size_t smem = resident_smem_bytes(P, s->NR, s->NL, n_ch, 2 * s->NR + s->NL);
-      int bits = 1, rank_bits = 0;
-      while ((1 << bits) < P) ++bits;
-      while ((1 << rank_bits) < C) ++rank_bits;
-      if (smem <= (size_t)optin && n_ch <= len0 && bits + rank_bits <= 16) {
+      const ResidentFit f = resident_fit(s, n_ch, C, T);
+      if (f.ok) {
+        const size_t smem = f.smem;
+        const int P = f.P;
         // 96 registers a thread: 20 warps per SM
         const int k = std::max(1, std::min((int)(per_sm / (smem + 1024)), 20 / (T / 32)));
         if (!one) one = std::max(1, clusters_at_one_per_sm(C, (size_t)optin));
@@ -743,14 +772,13 @@ void spread_banks(int* order, int n, int n_int, int bank0, const std::vector<int
   for (int i = 0; i < n; ++i) order[i] = before[id[i]];
 }
 
-int resident_partition(srs_sim* s, int C, int threads) {
+int resident_partition(srs_sim* s, int C, int threads, int group) {
   // Order: the elements that carry channels, then breadth-first layers
   // outward from them over the diffusion faces (so partition 0 holds the
   // channels' neighbourhood and partitions are cut between layers); the
   // sequence is cut into C contiguous partitions that give every element
-  // thread the same number of elements (in partition 0 the channel group,
-  // resident_group threads, takes the channel elements and the gating
-  // instead).  Inside each
+  // thread the same number of elements (in partition 0 the channel group
+  // takes the channel elements and the gating instead).  Inside each
   // partition: channel elements (partition 0 only), then interior elements
   // (every neighbour in the same partition), then boundary elements.
   const int N = s->N;
@@ -796,7 +824,7 @@ int resident_partition(srs_sim* s, int C, int threads) {
   s->part_nch.assign(C, 0);
   s->part_nint.assign(C, 0);
   int Pmax = 0;
-  const int len0 = partition0_size(N, n_ch, C, threads);
+  const int len0 = partition0_size(N, n_ch, C, threads, group);
   s->part_start[0] = 0;
   s->part_len[0] = len0;
   for (int q = 1; q < C; ++q) {
@@ -879,7 +907,8 @@ uint16_t code_of(const srs_sim* s, int eng) {
 
 int setup_resident(srs_sim* s, int C, int threads) {
   SRS_TRY(check_fp32_supported(s, true));
-  SRS_TRY(resident_partition(s, C, threads));
+  const ResidentFit fit = resident_fit(s, channel_elements(s->m), C, threads);
+  SRS_TRY(resident_partition(s, C, threads, fit.group));  // says what is wrong where nothing fits
   const int N = s->N;
   const int NE = C * s->P_stride;
   // rest arrays over the padded engine numbering
@@ -941,6 +970,8 @@ int setup_resident(srs_sim* s, int C, int threads) {
   a.R = s->R;
   a.P = s->P_stride;
   a.off_bits = s->off_bits;
+  a.group = fit.group;
+  if (!fit.gc) SRS_TRY(dev_alloc(s, &s->d_gc, 2));
   SRS_TRY(dev_upload_halves(s, &a.geo_a, &a.geo_b, geo));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_local, s->part_len.data(), s->part_len.size()));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_chtet, s->part_nch.data(), s->part_nch.size()));
@@ -986,7 +1017,7 @@ int setup_resident(srs_sim* s, int C, int threads) {
   if (!resident_cluster_supported(C)) return fail(SRS_ERR_UNSUPPORTED, "unsupported cluster size");
   s->C = C;
   s->threads = threads;
-  s->smem = resident_smem_bytes(s->P_stride, s->NR, s->NL, s->part_nch[0], 2 * s->NR + s->NL);
+  s->smem = resident_smem_bytes(s->P_stride, s->NR, s->NL, s->part_nch[0], 2 * s->NR + s->NL, fit.gc);
   int maxc = resident_max_clusters(C, threads, s->smem);
   if (maxc <= 0) return fail(SRS_ERR_UNSUPPORTED, "resident configuration does not fit on the device");
   s->n_clusters = std::min(maxc, s->R);
@@ -1279,6 +1310,8 @@ void refresh_args(srs_sim* s) {
     s->ar.P_ = s->P;
     s->ar.C = s->ch;
     s->ar.CS = cs;
+    if (s->d_gc) cudaMemcpyAsync(s->d_gc, s->P.gc, sizeof(s->P.gc), cudaMemcpyHostToDevice, s->st);
+    s->ar.gc = s->d_gc;
     s->ar.k = make_consts32(s);
     s->ar.M = s->d_M[0];
     s->ar.I = s->d_I[0];

@@ -172,6 +172,8 @@ struct ResidentArgs {
   int32_t steps;
   const float4* geo_a;  // coefficients
   const float4* geo_b;  // neighbour codes, bsl, flags
+  int32_t group;          // threads of the channel group (resident_group)
+  const srs_gate_consts* gc;  // [2] gating constants by potential; null: staged in shared memory
   int32_t prestep_first;  // run the protocol of the first step before it
   int32_t initial_row;    // ... and write the t = 0 states row
   const int32_t* n_local; // [C] elements in each partition
@@ -435,7 +437,7 @@ void gate_consts(const srs_params& p, double V, srs_gate_consts* g);
 void lcc_flux_consts(const srs_params& p, double V, double* A, double* E, double* Em1, double* B,
                      double* Vg);
 
-size_t resident_smem_bytes(int P, int NR, int NL, int n_chtet, int n_entries);
+size_t resident_smem_bytes(int P, int NR, int NL, int n_chtet, int n_entries, bool gc);
 // per cluster size (k_res_*.cu)
 #define SRS_RESIDENT_DECLARE(CC)                                                            \
   int launch_resident_c##CC(const ResidentArgs& a, int n_clusters, int threads, size_t smem, \
@@ -454,9 +456,11 @@ SRS_RESIDENT_DECLARE(16)
 // three warps, the last one for the LCCs, where the step waits for the
 // channels (large CTAs: 3.81 -> 2.93 us per step of a 16-CTA cluster of 320
 // threads); two where the elements bound it and a third warp is missed there
-// (1024 realizations, 8 x 192 threads: 117 against 126 us).
-__host__ __device__ constexpr int resident_group(int threads) {
-  return threads >= 320 ? 96 : threads >= 128 ? 64 : 32;
+// (1024 realizations, 8 x 192 threads: 117 against 126 us).  A larger group leaves
+// partition 0 fewer elements and the others more: where they do not fit any more
+// the group is of two warps (`wide` false).
+constexpr int resident_group(int threads, bool wide) {
+  return wide && threads >= 320 ? 96 : threads >= 128 ? 64 : 32;
 }
 int launch_resident(const ResidentArgs& a, int C, int n_clusters, int threads, size_t smem,
                     cudaStream_t st);
