@@ -1125,13 +1125,13 @@ int upload_state(srs_sim* s, int r, const double* S6) {
 // elements whose troponin indicator is neither 0 nor 1: the equilibrium has
 // troponin times the indicator there (initial_states), the rest has it once.
 int setup_reset32(srs_sim* s) {
+  if (std::all_of(s->m.tropc.begin(), s->m.tropc.end(), [](int t) { return t == 0 || t == 1; })) return SRS_OK;
   const size_t NE = eng_count(s);
   std::vector<double> S6;
   initial_states(s->m, s->p, &S6);
   std::vector<float4> M(NE);
   std::vector<float> I(NE);
   to_engine_fp32(s, S6.data(), M.data(), I.data());
-  if (std::all_of(I.begin(), I.end(), [](float x) { return x == 0.0f; })) return SRS_OK;
   return dev_upload(s, &s->d_I0, I.data(), NE);
 }
 
