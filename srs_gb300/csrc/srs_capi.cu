@@ -1818,8 +1818,7 @@ int srs_sim_get_config(const srs_sim* s, srs_sim_config* c) {
   c->kernel_launches = s->launches;
   const int64_t NE = (int64_t)eng_count(s);
   c->ctl_bytes = (int64_t)s->R * (int64_t)sizeof(RealCtl);
-  c->reset_h2d_bytes = (int64_t)s->R * ((int64_t)(s->NR + 2 * s->NL) * 4 + (int64_t)s->NCH * 8) +
-                       c->ctl_bytes;
+  c->reset_h2d_bytes = (int64_t)chan_block(s).bytes;
   c->engine_elements = NE;
   return SRS_OK;
 }
