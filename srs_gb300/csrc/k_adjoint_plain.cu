@@ -174,8 +174,9 @@ __global__ void __launch_bounds__(ADJP_THREADS, 4) k_adjp_step(AdjPlainArgs a) {
 
 // Blocks per realization of the reverse-step launches, at most one element per
 // thread: one wave of four blocks per SM while a thread then has at most four
-// elements (69,696 elements of eight realizations: 2.30 ms per gradient of 64
-// steps against 2.35 with two waves), else two waves, which balance better.
+// elements (69,696 elements of eight realizations: 2.33 ms per gradient of 64
+// steps against 2.39 with two waves, and the same gradient to the last digit shown),
+// else two waves, which balance better.
 int adjp_blocks_per_realization(int N, int R, int n_sm) {
   const int by_elem = (N + ADJP_THREADS - 1) / ADJP_THREADS;
   const int wave = std::max(1, 4 * n_sm / R);

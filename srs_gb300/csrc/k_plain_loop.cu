@@ -1,11 +1,12 @@
 // k_plain_loop.cu — the plain engines' steps in one launch, for problems that
 // fit on the chip's threads.
 //
-// With one launch per time step (k_plain64.cu, k_fp32.cu) a small problem waits:
-// 384 elements took 12.4 us a step in FP64 and 7.3 in FP32, whatever their
-// number -- launch, loads, update, a counter of finished blocks, and then the
-// last block's gating, one after the other.  Here a cooperative launch keeps
-// all blocks resident for many steps:
+// With one launch per time step (k_plain64.cu, k_fp32.cu: chained launches,
+// replayed as a graph) a small problem waits: 384 elements take 10.9 us a step in
+// FP64 and 6.4 in FP32, 10,368 take 11.5 and 6.9 -- launch, loads, update, a
+// counter of finished blocks, and then the last block's gating, one after the
+// other.  Here (6.4 and 3.5, 6.9 and 3.4) a cooperative launch keeps all blocks
+// resident for many steps:
 //   * element blocks hold their elements' geometry, immobile buffer and
 //     (FP32) compensation terms in registers; a step reads the neighbours'
 //     values from L2 and writes the mobile species, double buffered as before;
@@ -16,7 +17,7 @@
 //     gate it both: from the same Ca and the same random number they take the
 //     same decision, and neither waits for the other (a flag published by one
 //     gating block, which a first form used, was two more trips through L2 on
-//     the way from one step to the next: 4.3 against 7.5 us before, in FP32);
+//     the way from one step to the next: 4.3 us a step in FP32);
 //   * one more block per realization gates all channels again, off that path,
 //     and runs the protocol: output rows, run's end, final channel states.
 // Results are those of the one-launch-per-step kernels bit for bit: the same

@@ -55,9 +55,10 @@ __device__ __forceinline__ void kadd(float2& s, float2& c, float2 ndt, float2 o)
 }
 
 // Sums of N values over the warp: lane p returns the sum of value p (lanes from N
-// on: anything).  Each exchange halves the values a lane carries, 19 shuffles
-// for 18 values instead of five a value; the sum of each value is taken over the
-// same tree (lanes 16, 8, 4, 2, 1 apart), so it is the same number.
+// on: anything).  Each exchange halves the values a lane carries (of 32, the ones
+// from N on zero), 31 shuffles for 18 values instead of five a value; the sum of
+// each value is taken over the same tree (lanes 16, 8, 4, 2, 1 apart), so it is the
+// same number.
 template <int N>
 __device__ __forceinline__ float warp_sums(const float (&g)[N], int lane) {
   float v[32];
