@@ -79,8 +79,10 @@ __device__ __forceinline__ bool wait_all(const unsigned* bar, unsigned target, i
 // thread of the block calls it.
 template <class Args>
 __device__ __forceinline__ int steps_of(const Args& a, const PlainLoop& l, const RealCtl& c) {
-  if (__syncthreads_or(__ldcg(l.gave_up) != 0) || c.done) return 0;
-  return a.P.run_protocol ? (int)max((int64_t)0, min((int64_t)l.steps, a.P.n_steps - c.step)) : l.steps;
+  const int done = c.done;  // both loads in flight together with the flag's
+  const int64_t step = c.step;
+  if (__syncthreads_or(__ldcg(l.gave_up) != 0) || done) return 0;
+  return a.P.run_protocol ? (int)max((int64_t)0, min((int64_t)l.steps, a.P.n_steps - step)) : l.steps;
 }
 
 // ---- the protocol's block ----------------------------------------------------------
