@@ -8,28 +8,52 @@
 // (samples x elements, engine numbering) and the constant padding sum into an
 // offset; this kernel evaluates the sum from the state in HBM for every
 // realization, accumulating in double precision.
+#include <type_traits>
+
 #include "srs_comp.h"
 #include "srs_engine.h"
 
 namespace srs {
 
-// One block per (sample, realization).
+// One block per (sample, realization).  With few blocks a term's chain of loads
+// and conversions is what a thread waits for, so four terms' are in flight: one
+// realization of 69,696 elements 82 us a call (141 with one term at a time), 256
+// realizations 4.9 ms (7.0).
 __global__ void k_linescan(LinescanArgs a) {
   const int i = blockIdx.x, r = blockIdx.y;
+  const int end = a.ptr[i + 1], stride = blockDim.x;
   double acc = 0.0;
-  for (int q = a.ptr[i] + threadIdx.x; q < a.ptr[i + 1]; q += blockDim.x) {
-    const int e = a.col[q];
-    double dye;
-    if (a.S64) {
-      dye = a.S64[(size_t)r * 6 * a.n_state + 5 * (size_t)a.n_state + e];
-    } else {
-      const size_t o = (size_t)r * a.n_state + e;
-      const float u = a.M[o].w;
-      const float c = a.CMq ? comp_load1(a.CMq[o].w) : a.CM[o].w;
-      dye = a.rest_dye[e] + (widen(u) - widen(c));
+  // adds the terms q, q + stride, ...: N of them, whose loads are in flight together
+  auto terms = [&](int q, auto n) {
+    constexpr int N = decltype(n)::value;
+    int e[N];
+    double w[N], dye[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      e[k] = a.col[q + k * stride];
+      w[k] = a.w[q + k * stride];
     }
-    acc += a.w[q] * dye;
-  }
+    if (a.S64) {
+#pragma unroll
+      for (int k = 0; k < N; ++k) dye[k] = a.S64[(size_t)r * 6 * a.n_state + 5 * (size_t)a.n_state + e[k]];
+    } else {
+      float u[N], c[N];
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        const size_t o = (size_t)r * a.n_state + e[k];
+        u[k] = a.M[o].w;
+        c[k] = a.CMq ? comp_load1(a.CMq[o].w) : a.CM[o].w;
+        dye[k] = a.rest_dye[e[k]];
+      }
+#pragma unroll
+      for (int k = 0; k < N; ++k) dye[k] += widen(u[k]) - widen(c[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) acc += w[k] * dye[k];
+  };
+  int q = a.ptr[i] + threadIdx.x;
+  for (; q + 3 * stride < end; q += 4 * stride) terms(q, std::integral_constant<int, 4>{});
+  for (; q < end; q += stride) terms(q, std::integral_constant<int, 1>{});
   __shared__ double red[256];
   red[threadIdx.x] = acc;
   __syncthreads();
