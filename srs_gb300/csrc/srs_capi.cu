@@ -2386,6 +2386,38 @@ int linescan_csr(srs_sim* s) {
   return SRS_OK;
 }
 
+// Whether the tiled form takes the shorter time, by estimates of both in us:
+//   by sample: a call, the terms at the chip's rate (128 G/s; FP64 states 263 G/s,
+//     which need no conversion), a block's terms one after the other, the blocks;
+//   tiled: a call of two launches, eight multiply-adds an entry and 32 realizations
+//     on the FP64 pipe (0.44 ns), staging each element's dye once per tile, and a
+//     block's entries one after the other.
+// The tiled form is taken where it is shorter by a sixth.  Fitted to 2,736 calls
+// (384 to 69,696 elements, 1 to 1,024 realizations, 2 to 120 samples, thresholds of
+// 0.001 to 1 um^2, both precisions): two of them are then more than 3 % longer than
+// by sample (by 18 % at most), and all together 0.8 % longer than the better form
+// of each.  From 16 realizations on alone, as it was, few samples or a narrow
+// threshold took up to twelve times as long tiled.
+bool linescan_tiled(const srs_sim* s, const std::vector<int32_t>& ptr, const std::vector<int32_t>& col) {
+  const int ns = s->ls.n_samples, N = s->ls.n_state, R = s->R, groups = (ns + 7) / 8;
+  if ((size_t)R * ns >= (size_t)INT32_MAX) return false;
+  std::vector<int32_t> seen(N, -1);
+  double terms = (double)col.size(), entries = 0;
+  for (int i = 0; i < ns; ++i)
+    for (int q = ptr[i]; q < ptr[i + 1]; ++q)
+      if (seen[col[q]] != i / 8) {
+        seen[col[q]] = i / 8;
+        entries += 1;
+      }
+  const bool f64 = s->d.precision == SRS_FP64;
+  const double tiles = (R + 31) / 32, rows = (groups + 7) / 8;
+  const double by_sample = 23 + (f64 ? 3.8e-6 : 7.8e-6) * terms * R + (f64 ? 0.18 : 0.33) * terms / ns / 256 +
+                           4.2e-3 * ns * R;
+  const double tiled = 44 + 4.4e-4 * entries * tiles + (f64 ? 6.8e-6 : 14e-6) * N * tiles * 32 * rows +
+                       0.64 * entries / groups / linescan_splits(ns, N, R, sm_count());
+  return 1.2 * tiled < by_sample;
+}
+
 // The tiled form of the line scan's weights (LinescanArgs): for every group
 // of eight samples, by chunk of engine elements, the elements that any of
 // the eight weighs, with their eight weights and which of them count.
@@ -2606,7 +2638,7 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
   }
   SRS_TRY(dev_alloc(s, &s->d_ls_out, (size_t)s->R * ns));
   a.out = s->d_ls_out;
-  if (s->R >= LINESCAN_TILE_R && (size_t)s->R * ns < (size_t)INT32_MAX) {
+  if (linescan_tiled(s, ptr, col)) {
     SRS_TRY(linescan_tiles(s, ptr, col, w));
   } else {
     a.tptr = nullptr;

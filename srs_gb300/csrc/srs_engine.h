@@ -222,8 +222,8 @@ struct LinescanArgs {
   const ushort4* CMq;    //   (or in compact form, srs_comp.h)
   const double* rest_dye;  // [n_state] resting bound dye per element
   double* out;           // [R][n_samples]
-  // tiled form (LINESCAN_TILE_R realizations and more): per group of eight
-  // samples the elements that any of them weighs, by element chunk
+  // tiled form (linescan_tiled): per group of eight samples the elements that any
+  // of them weighs, by element chunk
   int32_t n_chunk;       // chunks of LINESCAN_CHUNK engine elements
   const int32_t* tptr;   // [groups][n_chunk + 1]
   const uint32_t* tent;  // (sample mask << 24) | offset in the chunk
@@ -233,10 +233,6 @@ struct LinescanArgs {
   double* part;          // [splits][R][n_samples]
 };
 constexpr int LINESCAN_CHUNK = 64;
-// Fewer realizations than this leave most lanes of the tiled form idle: a call
-// for 8 of 69,696 elements took 255 us tiled and 168 untiled, one for 21 of
-// 15,288 elements 108 and 130.
-constexpr int LINESCAN_TILE_R = 16;
 int linescan_splits(int n_samples, int n_state, int R, int n_sm);
 int launch_linescan(const LinescanArgs& a, int R, cudaStream_t st);
 
