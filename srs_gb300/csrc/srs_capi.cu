@@ -92,7 +92,6 @@ struct srs_sim {
   size_t smem = 0;
   std::vector<int> part_start, part_len, part_nch, part_nint;  // resident partitions
   int ch_interior = 0;
-  srs_gate_consts* d_gc = nullptr;  // [2] Protocol's, where shared memory does not hold them
   int64_t launches = 0;
   cudaGraphExec_t graph_plain = nullptr;      // steps from state buffer 0 ...
   cudaGraphExec_t graph_plain_alt = nullptr;  // ... captured when the buffers were exchanged
@@ -971,7 +970,7 @@ int setup_resident(srs_sim* s, int C, int threads) {
   a.P = s->P_stride;
   a.off_bits = s->off_bits;
   a.group = fit.group;
-  if (!fit.gc) SRS_TRY(dev_alloc(s, &s->d_gc, 2));
+  a.stage_gc = fit.gc;
   SRS_TRY(dev_upload_halves(s, &a.geo_a, &a.geo_b, geo));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_local, s->part_len.data(), s->part_len.size()));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_chtet, s->part_nch.data(), s->part_nch.size()));
@@ -1310,8 +1309,6 @@ void refresh_args(srs_sim* s) {
     s->ar.P_ = s->P;
     s->ar.C = s->ch;
     s->ar.CS = cs;
-    if (s->d_gc) cudaMemcpyAsync(s->d_gc, s->P.gc, sizeof(s->P.gc), cudaMemcpyHostToDevice, s->st);
-    s->ar.gc = s->d_gc;
     s->ar.k = make_consts32(s);
     s->ar.M = s->d_M[0];
     s->ar.I = s->d_I[0];
