@@ -93,6 +93,7 @@ struct srs_sim {
   std::vector<int> part_start, part_len, part_nch, part_nint;  // resident partitions
   int ch_interior = 0;
   int64_t launches = 0;
+  int64_t args_version = 0;  // counts refresh_args: graphs hold the arguments of their capture
   cudaGraphExec_t graph_plain = nullptr;      // steps from state buffer 0 ...
   cudaGraphExec_t graph_plain_alt = nullptr;  // ... captured when the buffers were exchanged
   int graph_plain_len = 0;
@@ -1280,6 +1281,7 @@ std::vector<int64_t> ctl_steps(srs_sim* s) {
 
 // ---- launches -----------------------------------------------------------------
 void refresh_args(srs_sim* s) {
+  s->args_version++;
   ChanState cs = chan_state(s);
   if (s->d.precision == SRS_FP64) {
     s->a64.P = s->P;
@@ -2196,7 +2198,7 @@ struct srs_batch {
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> join;
   cudaGraphExec_t graph = nullptr;
-  int graph_mode = -1;  // run_protocol the graph was captured with
+  std::vector<int64_t> graph_args;  // the members' args_version it was captured with
   int64_t replays = 0;
 };
 
@@ -2205,7 +2207,6 @@ namespace {
 void batch_drop_graph(srs_batch* b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   b->graph = nullptr;
-  b->graph_mode = -1;
 }
 
 // One replay: every member advances S steps on its own stream; the members'
@@ -2226,9 +2227,10 @@ int batch_enqueue(srs_batch* b, int steps, int first) {
 }
 
 int batch_graph(srs_batch* b) {
-  const int mode = b->sims[0]->P.run_protocol;
-  if (b->graph && b->graph_mode == mode) return SRS_OK;
-  batch_drop_graph(b);
+  std::vector<int64_t> args;
+  for (const srs_sim* s : b->sims) args.push_back(s->args_version);
+  if (b->graph && b->graph_args == args) return SRS_OK;
+  batch_drop_graph(b);  // replays on their way run to their end
   cudaGraph_t g;
   SRS_CUDA(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
   int rc = batch_enqueue(b, b->S, 0);
@@ -2239,7 +2241,7 @@ int batch_graph(srs_batch* b) {
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return fail(SRS_ERR_CUDA, std::string("batch graph: ") + cudaGetErrorString(e));
   for (srs_sim* s : b->sims) s->launches--;  // counted per replay instead
-  b->graph_mode = mode;
+  b->graph_args = args;
   return SRS_OK;
 }
 

@@ -41,3 +41,18 @@ def test_steps_on_their_way_keep_their_constants(srs, tmp_path, C, T):
     batch.synchronize()
     y.explicit_step(1024)
     _same(x, y)
+
+
+@pytest.mark.parametrize("C,T", CONFIGS)
+@pytest.mark.parametrize("n", [20, 532])  # by one launch; by replays and a launch
+def test_steps_after_take_the_new_constants(srs, tmp_path, C, T, n):
+    x, y = _pair(srs, tmp_path, C, T)
+    batch = srs.Batch([x], steps_per_launch=256)
+    batch.advance_async(n)
+    x.set_globals(60.0, 900.0)
+    batch.advance_async(n)
+    batch.synchronize()
+    y.explicit_step(n)
+    y.set_globals(60.0, 900.0)
+    y.explicit_step(n)
+    _same(x, y)
