@@ -8,6 +8,7 @@
 #include <functional>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -2400,21 +2401,30 @@ int linescan_csr(srs_sim* s) {
 bool linescan_tiled(const srs_sim* s, const std::vector<int32_t>& ptr, const std::vector<int32_t>& col) {
   const int ns = s->ls.n_samples, N = s->ls.n_state, R = s->R, groups = (ns + 7) / 8;
   if ((size_t)R * ns >= (size_t)INT32_MAX) return false;
-  std::vector<int32_t> seen(N, -1);
-  double terms = (double)col.size(), entries = 0;
-  for (int i = 0; i < ns; ++i)
-    for (int q = ptr[i]; q < ptr[i + 1]; ++q)
-      if (seen[col[q]] != i / 8) {
-        seen[col[q]] = i / 8;
-        entries += 1;
-      }
   const bool f64 = s->d.precision == SRS_FP64;
-  const double tiles = (R + 31) / 32, rows = (groups + 7) / 8;
+  const double terms = (double)col.size(), tiles = (R + 31) / 32, rows = (groups + 7) / 8;
+  const int splits = linescan_splits(ns, N, R, sm_count());
   const double by_sample = 23 + (f64 ? 3.8e-6 : 7.8e-6) * terms * R + (f64 ? 0.18 : 0.33) * terms / ns / 256 +
                            4.2e-3 * ns * R;
-  const double tiled = 44 + 4.4e-4 * entries * tiles + (f64 ? 6.8e-6 : 14e-6) * N * tiles * 32 * rows +
-                       0.64 * entries / groups / linescan_splits(ns, N, R, sm_count());
-  return 1.2 * tiled < by_sample;
+  auto shorter = [&](double entries) {
+    const double tiled = 44 + 4.4e-4 * entries * tiles + (f64 ? 6.8e-6 : 14e-6) * N * tiles * 32 * rows +
+                         0.64 * entries / groups / splits;
+    return 1.2 * tiled < by_sample;
+  };
+  // An entry is an element that any of a group's eight samples weighs: an eighth of
+  // the terms at least.  They are counted only where that many would do.
+  if (!shorter(terms / 8)) return false;
+  std::vector<int64_t> entries(groups, 0);
+  host_parallel(groups, terms < 100000 ? 1 : 8, [&](int g) {
+    std::vector<char> seen(N, 0);
+    int64_t n = 0;
+    for (int q = ptr[8 * g]; q < ptr[std::min(ns, 8 * g + 8)]; ++q) {
+      n += !seen[col[q]];
+      seen[col[q]] = 1;
+    }
+    entries[g] = n;
+  });
+  return shorter((double)std::accumulate(entries.begin(), entries.end(), (int64_t)0));
 }
 
 // The tiled form of the line scan's weights (LinescanArgs): for every group
