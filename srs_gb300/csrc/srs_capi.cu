@@ -652,11 +652,14 @@ int clusters_at_one_per_sm(int C, size_t optin) {
 // candidate with the smallest estimated time of a step for all realizations,
 //   rounds * t,  rounds = realizations / co-resident clusters, rounded up,
 //   t = (t_lat^4 + t_thr^4)^(1/4) us,
-//   t_lat = 2.05 + 0.28 elements per thread + 6e-4 threads (the chain of one
-// step: barriers, gating, a thread's elements one after the other) and
+//   t_lat = 2.05 + 0.28 elements per thread + 6e-4 threads, 0.95 less for a single
+// CTA (the chain of one step: barriers, gating, a thread's elements one after the
+// other; a CTA alone needs no cluster barrier and reads all neighbours itself) and
 //   t_thr = 1.2e-3 elements per SM (what an SM issues and moves).
 // Fitted to steps of the 10,368-element dyad: 5 x 320, two CTAs per SM, 5.6 us;
-// 3 x 512, one, 5.3; 8 x 192, three, 5.1; 16 x 320 for two realizations 2.9.
+// 3 x 512, one, 5.3; 8 x 192, three, 5.1; 16 x 320 for two realizations 2.9.  The
+// single CTA's 0.95 to meshes of 384 and 1,296: 1.9 us by one CTA of 384 threads
+// against 3.0 by 16 of 160, and 2.2 (640) against 2.8 (16 x 192).
 // The smallest cluster that fits, which this replaces, took 133 us per step of
 // 1024 realizations (3 x 512) against 100 (5 x 320), and two rounds of 36
 // clusters for 37 realizations.
@@ -688,7 +691,7 @@ int choose_resident(const srs_sim* s, int C_in, int T_in, int* C_out, int* T_out
         const int ncl = std::min(one * k, s->R);
         const int rounds = (s->R + ncl - 1) / ncl;
         const double per = std::max(1.0, std::ceil((double)ncl * C / n_sm)) * P;  // elements per SM
-        const double lat = 2.05 + 0.28 * P / T + 6e-4 * T, thr = 1.2e-3 * per;
+        const double lat = (C > 1 ? 2.05 : 1.1) + 0.28 * P / T + 6e-4 * T, thr = 1.2e-3 * per;
         cand.push_back({rounds * std::sqrt(std::sqrt(lat * lat * lat * lat + thr * thr * thr * thr)), C, T, smem});
       }
       if (T_in > 0) break;
