@@ -391,8 +391,22 @@ size_t resident_smem_bytes(int P, int NR, int NL, int n_chtet, int n_entries, bo
 
 #define SRS_RESIDENT_SIZES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(8) X(16)
 
+// The gating constants of the launch that follows, where its shared memory has no
+// room for them.  By a launch of its own: written or read in the step kernel (its
+// parameters' address, or a store by the first cluster), they make the recording form
+// 1 % longer, staged or not (64 realizations of 10,368 elements, 512 steps of the
+// adjoint 11.6 against 11.45 ms).
+struct GateConsts {
+  srs_gate_consts gc[2];
+};
+__global__ void k_gate_consts(GateConsts in, srs_gate_consts* out) { out[threadIdx.x] = in.gc[threadIdx.x]; }
+
 int launch_resident(const ResidentArgs& a, int C, int n_clusters, int threads, size_t smem,
                     cudaStream_t st) {
+  if (a.gc) {
+    k_gate_consts<<<1, 2, 0, st>>>(GateConsts{{a.P_.gc[0], a.P_.gc[1]}}, a.gc);
+    if (cudaGetLastError() != cudaSuccess) return -1;
+  }
   switch (C) {
 #define SRS_L(CC) \
   case CC:        \

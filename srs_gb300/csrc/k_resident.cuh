@@ -199,7 +199,7 @@ template <int C, bool TRAJ>
 // At most 640 threads per CTA: two CTAs of up to 320 threads share an SM
 // with up to 96 registers per thread (the tuned configurations), and
 // single-CTA configurations keep the same budget.
-__global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(const __grid_constant__ ResidentArgs a) {
+__global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(ResidentArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int P = a.P;
   float4* buf0 = reinterpret_cast<float4*>(smem);
@@ -226,11 +226,9 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(cons
   int32_t* s_cptr = reinterpret_cast<int32_t*>(s_flux + NCH);
   float2* s_clist = reinterpret_cast<float2*>(
       (reinterpret_cast<uintptr_t>(s_cptr + a.n_chtet[0] + 1) + 15) & ~(uintptr_t)15);
-  // the gating constants behind them, where they fit (else read from the launch's
-  // arguments)
+  // the gating constants behind them, where they fit (else in global memory)
   srs_gate_consts* s_gc = reinterpret_cast<srs_gate_consts*>(s_clist + 2 * NR + NL);
-  const ChanSmem cs{s_ccl, s_cjs, s_clc, s_lrest, s_ryr, s_lcc, s_lccv, s_nb, s_res, s_flux,
-                    a.stage_gc ? s_gc : a.P_.gc};
+  const ChanSmem cs{s_ccl, s_cjs, s_clc, s_lrest, s_ryr, s_lcc, s_lccv, s_nb, s_res, s_flux, a.gc ? a.gc : s_gc};
 
   uint32_t rank = 0;
   if constexpr (C > 1) {
@@ -279,7 +277,7 @@ __global__ void __launch_bounds__(SRS_RESIDENT_MAX_THREADS, 1) k_resident32(cons
       tail->base[1][q] = (C > 1) ? map_rank(smem_addr(buf1), q) : smem_addr(buf1);
     }
   }
-  if (tid < 2 && a.stage_gc) s_gc[tid] = P_.gc[tid];
+  if (tid < 2 && !a.gc) s_gc[tid] = P_.gc[tid];
   if (tid == 0) tail->bad = 0;
   // address of rank 0's termination flags, as seen from this CTA
   uint32_t done_addr0 = smem_addr(&tail->done_flag[0]);

@@ -975,7 +975,7 @@ int setup_resident(srs_sim* s, int C, int threads) {
   a.P = s->P_stride;
   a.off_bits = s->off_bits;
   a.group = fit.group;
-  a.stage_gc = fit.gc;
+  if (!fit.gc) SRS_TRY(dev_alloc(s, &a.gc, 2));
   SRS_TRY(dev_upload_halves(s, &a.geo_a, &a.geo_b, geo));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_local, s->part_len.data(), s->part_len.size()));
   SRS_TRY(dev_upload(s, (int32_t**)&a.n_chtet, s->part_nch.data(), s->part_nch.size()));

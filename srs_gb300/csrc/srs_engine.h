@@ -173,7 +173,8 @@ struct ResidentArgs {
   const float4* geo_a;  // coefficients
   const float4* geo_b;  // neighbour codes, bsl, flags
   int32_t group;          // threads of the channel group (resident_group)
-  int32_t stage_gc;       // gating constants staged in shared memory
+  srs_gate_consts* gc;    // [2] gating constants by potential, written before each launch; null: staged in
+                          // shared memory
   int32_t prestep_first;  // run the protocol of the first step before it
   int32_t initial_row;    // ... and write the t = 0 states row
   const int32_t* n_local; // [C] elements in each partition
