@@ -1035,8 +1035,10 @@ size_t eng_count(const srs_sim* s) {
 
 // ---- state conversion ---------------------------------------------------------
 // Staging of export_state with ns state values in it; states beyond
-// kExportDirect bytes are copied without.
-constexpr size_t kExportDirect = (size_t)4 << 20;
+// kExportDirect bytes are copied without: the second copy out of pinned memory
+// takes longer than the driver's own (FP64 states of 10,368 elements, 0.5 MB, 59 us
+// staged and 67 direct; of 15,288, 78 and 72; of 61,000, 255 and 119).
+constexpr size_t kExportDirect = (size_t)640 << 10;
 size_t export_bytes(const srs_sim* s, size_t ns) {
   return (ns + s->NCH) * sizeof(double) + (size_t)(s->NR + 2 * s->NL) * sizeof(int32_t);
 }
@@ -1180,21 +1182,22 @@ int clear_timeout(srs_sim* s) {
 }
 
 // Realization r in the caller's form (any output may be null): the conversion
-// and the gathering run on the device (k_export_state).  Up to a few MB it
-// writes pinned host memory and the caller's arrays are filled from there;
-// larger states go to a device buffer and are copied out of it.
+// and the gathering run on the device (k_export_state).  Small states are written
+// to pinned host memory and the caller's array is filled from there; larger ones
+// are copied to it from a device buffer, the FP64 engine's from the state itself.
 int export_state(srs_sim* s, int r, double* S, int* ryr, int* lcc, int* lccv, double* res) {
   std::lock_guard<std::mutex> lock(s->stage_mtx);
   const size_t N = s->N, NE = eng_count(s), ns = S ? 6 * N : 0;
   const bool direct = export_bytes(s, ns) > kExportDirect;
   double* h = (double*)stage(s, export_bytes(s, direct ? 0 : ns));
   if (!h) return fail(SRS_ERR_NOMEM, "pinned staging allocation failed");
-  if (direct && !s->d_export) SRS_TRY(dev_alloc(s, &s->d_export, 6 * N));
+  const bool f64 = s->d.precision == SRS_FP64;
+  if (direct && !f64 && !s->d_export) SRS_TRY(dev_alloc(s, &s->d_export, 6 * N));
   ExportArgs a{};
   a.N = s->N;
   a.NR = s->NR;
   a.NL = s->NL;
-  if (s->d.precision == SRS_FP64) {
+  if (f64) {
     a.S64 = s->d_S[0] + (size_t)r * 6 * N;
   } else {
     a.M = s->d_M[0] + r * NE;
@@ -1220,13 +1223,14 @@ int export_state(srs_sim* s, int r, double* S, int* ryr, int* lcc, int* lccv, do
   double* hres = h;
   double* hS = hres + s->NCH;
   int32_t* hi = reinterpret_cast<int32_t*>(hS + (direct ? 0 : ns));
-  a.S = S ? (direct ? s->d_export : hS) : nullptr;
+  const double* from = f64 ? a.S64 : s->d_export;
+  a.S = !S || (direct && f64) ? nullptr : direct ? s->d_export : hS;
   a.res_out = res ? hres : nullptr;
   a.ryr_out = ryr ? hi : nullptr;
   a.lcc_out = lcc ? hi + s->NR : nullptr;
   a.lccv_out = lccv ? hi + s->NR + s->NL : nullptr;
   if (launch_export_state(a, s->st)) return fail(SRS_ERR_CUDA, "state export launch failed");
-  if (direct) SRS_CUDA(cudaMemcpyAsync(S, s->d_export, ns * sizeof(double), cudaMemcpyDeviceToHost, s->st));
+  if (direct) SRS_CUDA(cudaMemcpyAsync(S, from, ns * sizeof(double), cudaMemcpyDeviceToHost, s->st));
   SRS_CUDA(cudaStreamSynchronize(s->st));
   SRS_TRY(check_timeout(s));
   if (S && !direct) std::memcpy(S, hS, ns * sizeof(double));
