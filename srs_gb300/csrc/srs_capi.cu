@@ -878,7 +878,7 @@ int resident_partition(srs_sim* s, int C, int threads, int group) {
   std::vector<int> pos(N, -1);  // position in the element's own partition; -1: a channel element
   for (int q = 0; q < C; ++q)
     for (int i = s->part_nch[q]; i < s->part_len[q]; ++i) pos[order[s->part_start[q] + i]] = i - s->part_nch[q];
-  host_parallel(C, N < 3000 ? 1 : 8, [&](int q) {
+  host_parallel(C, host_threads(0.216 * N), [&](int q) {
     const int c0 = s->part_nch[q];
     spread_banks(order.data() + s->part_start[q] + c0, s->part_len[q] - c0, s->part_nint[q], c0, pos,
                  [&](int j, int k) {
@@ -1914,7 +1914,7 @@ int srs_sim_reset(srs_sim* s) {
     for (int i = 0; i < NR; ++i) n_open += ry[i];
     c.n_open_tick = n_open;
   };
-  host_parallel(s->R, (size_t)s->R * NCH < 4096 ? 1 : 8, one);
+  host_parallel(s->R, host_threads(0.02 * s->R * NCH), one);
   SRS_TRY(reset_states(s));
   SRS_CUDA(cudaMemcpyAsync(s->d_ctl, h, blk.bytes, cudaMemcpyHostToDevice, s->st));
   SRS_CUDA(cudaStreamSynchronize(s->st));
