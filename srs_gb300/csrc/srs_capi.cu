@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -115,7 +116,12 @@ struct srs_sim {
   // line scan
   LinescanArgs ls{};
   std::vector<double> ls_rest;  // F at the equilibrium state
-  std::vector<void*> ls_allocs;  // device buffers of this set-up, freed with it
+  struct LsBuffer {
+    void* p;
+    size_t bytes;
+    bool used;
+  };
+  std::vector<LsBuffer> ls_bufs;  // device buffers of this set-up, and unused ones of the one before
   double* d_ls_out = nullptr;
   std::vector<int32_t> ls_ptr_h, ls_col_h;  // host copy of the line-scan CSR
   std::vector<double> ls_w_h;
@@ -153,19 +159,40 @@ int dev_upload(srs_sim* s, T** dst, const T* src, size_t n) {
   *dst = (T*)p;
   return SRS_OK;
 }
-// Device buffers made in its scope belong to the line scan's set-up (the weights
-// in their forms, and the adjoint's map of them) instead of to the simulation.
-struct LinescanBuffers {
-  srs_sim* s;
-  size_t first;
-  explicit LinescanBuffers(srs_sim* sim) : s(sim), first(sim->allocs.size()) {}
-  ~LinescanBuffers() {
-    s->ls_allocs.insert(s->ls_allocs.end(), s->allocs.begin() + first, s->allocs.end());
-    s->allocs.resize(first);
+// Device buffers of the line scan's set-up (the weights in their forms, and the
+// adjoint's map of them): the smallest one of the set-up before that is large enough,
+// else a new one.
+template <class T>
+int ls_alloc(srs_sim* s, T** dst, size_t n) {
+  const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+  srs_sim::LsBuffer* best = nullptr;
+  for (auto& b : s->ls_bufs)
+    if (!b.used && b.bytes >= bytes && (!best || b.bytes < best->bytes)) best = &b;
+  if (!best) {
+    void* p = nullptr;
+    SRS_CUDA(cudaMalloc(&p, bytes));
+    s->ls_bufs.push_back({p, bytes, true});
+    best = &s->ls_bufs.back();
   }
-  LinescanBuffers(const LinescanBuffers&) = delete;
-  LinescanBuffers& operator=(const LinescanBuffers&) = delete;
-};
+  best->used = true;
+  *dst = (T*)best->p;
+  return SRS_OK;
+}
+template <class T>
+int ls_upload(srs_sim* s, T** dst, const T* src, size_t n) {
+  if (int rc = ls_alloc(s, dst, n)) return rc;
+  if (n) SRS_CUDA(cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice));
+  return SRS_OK;
+}
+// A new set-up (the stream idle): the buffers of the one before may be used again,
+// and those that it did not use itself are freed.
+void ls_release(srs_sim* s) {
+  size_t n = 0;
+  for (auto& b : s->ls_bufs)
+    if (b.used) s->ls_bufs[n++] = {b.p, b.bytes, false};
+    else cudaFree(b.p);
+  s->ls_bufs.resize(n);
+}
 // 32-byte records as their first halves, then their second halves.
 template <class Rec>
 std::vector<float4> record_halves(const std::vector<Rec>& rec) {
@@ -1777,7 +1804,7 @@ void srs_sim_destroy(srs_sim* s) {
   if (s->graph_plain_alt) cudaGraphExecDestroy(s->graph_plain_alt);
   if (s->st) cudaStreamSynchronize(s->st);
   for (void* p : s->allocs) cudaFree(p);
-  for (void* p : s->ls_allocs) cudaFree(p);
+  for (auto& b : s->ls_bufs) cudaFree(b.p);
   for (auto& b : s->adj_bufs) cudaFree(b.first);
   if (s->h_stage) cudaFreeHost(s->h_stage);
   if (s->h_pin) cudaFreeHost(s->h_pin);
@@ -2384,11 +2411,10 @@ namespace {
 int linescan_csr(srs_sim* s) {
   LinescanArgs& a = s->ls;
   if (a.ptr) return SRS_OK;
-  LinescanBuffers own(s);
   int32_t* dp;
-  SRS_TRY(dev_upload(s, (int32_t**)&a.col, s->ls_col_h.data(), s->ls_col_h.size()));
-  SRS_TRY(dev_upload(s, (double**)&a.w, s->ls_w_h.data(), s->ls_w_h.size()));
-  SRS_TRY(dev_upload(s, &dp, s->ls_ptr_h.data(), s->ls_ptr_h.size()));
+  SRS_TRY(ls_upload(s, (int32_t**)&a.col, s->ls_col_h.data(), s->ls_col_h.size()));
+  SRS_TRY(ls_upload(s, (double**)&a.w, s->ls_w_h.data(), s->ls_w_h.size()));
+  SRS_TRY(ls_upload(s, &dp, s->ls_ptr_h.data(), s->ls_ptr_h.size()));
   a.ptr = dp;
   return SRS_OK;
 }
@@ -2405,7 +2431,9 @@ int linescan_csr(srs_sim* s) {
 // by sample (by 18 % at most), and all together 0.8 % longer than the better form
 // of each.  From 16 realizations on alone, as it was, few samples or a narrow
 // threshold took up to twelve times as long tiled.
-bool linescan_tiled(const srs_sim* s, const std::vector<int32_t>& ptr, const std::vector<int32_t>& col) {
+// entries: each group's number of them, where the tiled form is taken.
+bool linescan_tiled(const srs_sim* s, std::vector<int64_t>* entries) {
+  const std::vector<int32_t>&ptr = s->ls_ptr_h, &col = s->ls_col_h;
   const int ns = s->ls.n_samples, N = s->ls.n_state, R = s->R, groups = (ns + 7) / 8;
   if ((size_t)R * ns >= (size_t)INT32_MAX) return false;
   const bool f64 = s->d.precision == SRS_FP64;
@@ -2413,60 +2441,62 @@ bool linescan_tiled(const srs_sim* s, const std::vector<int32_t>& ptr, const std
   const int splits = linescan_splits(ns, N, R, sm_count());
   const double by_sample = 23 + (f64 ? 3.8e-6 : 7.8e-6) * terms * R + (f64 ? 0.18 : 0.33) * terms / ns / 256 +
                            4.2e-3 * ns * R;
-  auto shorter = [&](double entries) {
-    const double tiled = 44 + 4.4e-4 * entries * tiles + (f64 ? 6.8e-6 : 14e-6) * N * tiles * 32 * rows +
-                         0.64 * entries / groups / splits;
+  auto shorter = [&](double n) {
+    const double tiled = 44 + 4.4e-4 * n * tiles + (f64 ? 6.8e-6 : 14e-6) * N * tiles * 32 * rows +
+                         0.64 * n / groups / splits;
     return 1.2 * tiled < by_sample;
   };
   // An entry is an element that any of a group's eight samples weighs: an eighth of
   // the terms at least.  They are counted only where that many would do.
   if (!shorter(terms / 8)) return false;
-  std::vector<int64_t> entries(groups, 0);
-  host_parallel(groups, terms < 100000 ? 1 : 8, [&](int g) {
+  entries->assign(groups, 0);
+  host_parallel(groups, host_threads(1e-3 * terms), [&](int g) {
     std::vector<char> seen(N, 0);
     int64_t n = 0;
     for (int q = ptr[8 * g]; q < ptr[std::min(ns, 8 * g + 8)]; ++q) {
       n += !seen[col[q]];
       seen[col[q]] = 1;
     }
-    entries[g] = n;
+    (*entries)[g] = n;
   });
-  return shorter((double)std::accumulate(entries.begin(), entries.end(), (int64_t)0));
+  return shorter((double)std::accumulate(entries->begin(), entries->end(), (int64_t)0));
 }
 
 // The tiled form of the line scan's weights (LinescanArgs): for every group
 // of eight samples, by chunk of engine elements, the elements that any of
 // the eight weighs, with their eight weights and which of them count.
-int linescan_tiles(srs_sim* s, const std::vector<int32_t>& ptr, const std::vector<int32_t>& col,
-                   const std::vector<double>& w) {
+int linescan_tiles(srs_sim* s, const std::vector<int64_t>& entries) {
   LinescanArgs& a = s->ls;
-  a.tptr = nullptr;
+  const std::vector<int32_t>&ptr = s->ls_ptr_h, &col = s->ls_col_h;
   const int ns = a.n_samples, groups = (ns + 7) / 8;
   const int chunks = (a.n_state + LINESCAN_CHUNK - 1) / LINESCAN_CHUNK;
-  std::vector<int32_t> tptr;
-  std::vector<uint32_t> tent;
-  std::vector<double> tw;
-  tptr.reserve((size_t)groups * (chunks + 1));
-  std::vector<int32_t> at(a.n_state);  // entry of an element in this group
-  for (int g = 0; g < groups; ++g) {
+  std::vector<int64_t> first(groups + 1, 0);  // entry of each group
+  std::partial_sum(entries.begin(), entries.end(), first.begin() + 1);
+  const size_t n_ent = (size_t)first[groups];
+  std::vector<int32_t> tptr((size_t)groups * (chunks + 1));
+  std::vector<uint32_t> tent(n_ent);
+  std::unique_ptr<double[]> tw(new double[8 * n_ent]);  // each group clears its own
+  // 3 ns a term: 750 us for 250,000
+  host_parallel(groups, host_threads(3e-3 * (double)col.size()), [&](int g) {
     const int i0 = 8 * g, i1 = std::min(ns, i0 + 8);
-    std::fill(at.begin(), at.end(), -1);
+    std::vector<int32_t> at(a.n_state, -1);  // entry of an element in this group
     for (int q = ptr[i0]; q < ptr[i1]; ++q) at[col[q]] = 0;
+    int32_t n = (int32_t)first[g], *tp = &tptr[(size_t)g * (chunks + 1)];
     for (int e = 0; e < a.n_state; ++e) {
-      if (e % LINESCAN_CHUNK == 0) tptr.push_back((int32_t)tent.size());
+      if (e % LINESCAN_CHUNK == 0) *tp++ = n;
       if (at[e] < 0) continue;
-      at[e] = (int32_t)tent.size();
-      tent.push_back((uint32_t)(e % LINESCAN_CHUNK));
+      at[e] = n;
+      tent[n++] = (uint32_t)(e % LINESCAN_CHUNK);
     }
-    tptr.push_back((int32_t)tent.size());
-    tw.resize(tent.size() * 8, 0.0);
+    *tp = n;
+    std::fill(&tw[8 * (size_t)first[g]], &tw[8 * (size_t)first[g]] + 8 * (size_t)entries[g], 0.0);
     for (int i = i0; i < i1; ++i)
       for (int q = ptr[i]; q < ptr[i + 1]; ++q) {
         const int32_t k = at[col[q]];
-        tw[(size_t)k * 8 + (i - i0)] = w[q];
+        tw[(size_t)k * 8 + (i - i0)] = s->ls_w_h[q];
         tent[k] |= 1u << (24 + (i - i0));
       }
-  }
+  });
   a.n_chunk = chunks;
   a.splits = linescan_splits(ns, a.n_state, s->R, sm_count());
   // The blocks' chunks, by their FP64 instructions (eight an entry; staging a
@@ -2504,12 +2534,12 @@ int linescan_tiles(srs_sim* s, const std::vector<int32_t>& ptr, const std::vecto
   }
   deal(hi);
   split.resize(a.splits + 1, chunks);
-  SRS_TRY(dev_upload(s, (int32_t**)&a.split, split.data(), split.size()));
+  SRS_TRY(ls_upload(s, (int32_t**)&a.split, split.data(), split.size()));
   int32_t* dp;
-  SRS_TRY(dev_upload(s, &dp, tptr.data(), tptr.size()));
-  SRS_TRY(dev_upload(s, (uint32_t**)&a.tent, tent.data(), tent.size()));
-  SRS_TRY(dev_upload(s, (double**)&a.tw, tw.data(), tw.size()));
-  SRS_TRY(dev_alloc(s, &a.part, (size_t)a.splits * s->R * ns));
+  SRS_TRY(ls_upload(s, &dp, tptr.data(), tptr.size()));
+  SRS_TRY(ls_upload(s, (uint32_t**)&a.tent, tent.data(), tent.size()));
+  SRS_TRY(ls_upload(s, (double**)&a.tw, tw.get(), 8 * n_ent));
+  SRS_TRY(ls_alloc(s, &a.part, (size_t)a.splits * s->R * ns));
   a.tptr = dp;
   return SRS_OK;
 }
@@ -2595,11 +2625,9 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
   std::vector<double> w, pad(ns, 0.0), rests(ns, 0.0);
   std::vector<double> S6;
   initial_states(m, s->p, &S6);
-  // samples are independent: their rows are built by up to eight host threads
-  // and joined in order
-  std::vector<std::vector<int32_t>> cols(ns);
-  std::vector<std::vector<double>> ws(ns);
-  auto sample = [&](int i) {
+  // samples are independent: where several host threads build their rows, each
+  // builds its own, and they are joined in order
+  auto sample = [&](int i, std::vector<int32_t>& cols, std::vector<double>& ws) {
     double c[3];
     center(i, c);
     double rest = 0.0;
@@ -2607,8 +2635,8 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
       double rx = cx[j] - c[0], ry = cy[j] - c[1], rz = cz[j] - c[2];
       if (rx * rx + ry * ry + rz * rz < d->r_thresh) {
         double wj = vol[j] * pdf(rx, ry, rz);
-        cols[i].push_back(s->eng_of_ref[j]);
-        ws[i].push_back(wj);
+        cols.push_back(s->eng_of_ref[j]);
+        ws.push_back(wj);
         rest += wj * S6[SP_DYE * (size_t)m.N + j];
       }
     }
@@ -2620,46 +2648,52 @@ int srs_linescan_setup(srs_sim* s, const srs_linescan_desc* d, int* n_samples) {
     pad[i] = pd;
     rests[i] = pd + rest;
   };
-  host_parallel(ns, (size_t)ns * (m.N + px.size()) < 100000 ? 1 : 8, sample);
-  for (int i = 0; i < ns; ++i) {
-    ptr[i] = (int32_t)col.size();
-    col.insert(col.end(), cols[i].begin(), cols[i].end());
-    w.insert(w.end(), ws[i].begin(), ws[i].end());
+  const int threads = host_threads(5.5e-3 * ns * ((double)m.N + px.size()));
+  if (threads == 1) {
+    for (int i = 0; i < ns; ++i) {
+      sample(i, col, w);
+      ptr[i + 1] = (int32_t)col.size();
+    }
+  } else {
+    std::vector<std::vector<int32_t>> cols(ns);
+    std::vector<std::vector<double>> ws(ns);
+    host_parallel(ns, threads, [&](int i) { sample(i, cols[i], ws[i]); });
+    for (int i = 0; i < ns; ++i) ptr[i + 1] = ptr[i] + (int32_t)cols[i].size();
+    col.reserve(ptr[ns]);
+    w.reserve(ptr[ns]);
+    for (int i = 0; i < ns; ++i) {
+      col.insert(col.end(), cols[i].begin(), cols[i].end());
+      w.insert(w.end(), ws[i].begin(), ws[i].end());
+    }
   }
-  ptr[ns] = (int32_t)col.size();
-  s->ls_ptr_h = ptr;
-  s->ls_col_h = col;
-  s->ls_w_h = w;
+  s->ls_ptr_h = std::move(ptr);
+  s->ls_col_h = std::move(col);
+  s->ls_w_h = std::move(w);
   s->ls_pad_h = pad;
-  s->ls_rest = rests;
+  s->ls_rest = std::move(rests);
   s->ls_version++;
   // a new scan takes the place of the one before
   SRS_CUDA(cudaStreamSynchronize(s->st));
-  for (void* p : s->ls_allocs) cudaFree(p);
-  s->ls_allocs.clear();
+  ls_release(s);
   LinescanArgs& a = s->ls;
   a.n_samples = ns;
   a.n_state = (int32_t)eng_count(s);
   a.ptr = nullptr;  // uploaded by linescan_csr
   a.tptr = nullptr;
-  LinescanBuffers own(s);
-  SRS_TRY(dev_upload(s, (double**)&a.pad, pad.data(), pad.size()));
+  SRS_TRY(ls_upload(s, (double**)&a.pad, pad.data(), pad.size()));
   if (s->d.precision != SRS_FP64) {
     std::vector<double> rd(eng_count(s), 0.0);
     for (size_t e = 0; e < rd.size(); ++e) {
       int j = s->ref_of_eng[e];
       if (j >= 0 && s->m.domain[j] == DOMAIN_CYTO) rd[e] = s->rv.dye;
     }
-    SRS_TRY(dev_upload(s, (double**)&a.rest_dye, rd.data(), rd.size()));
+    SRS_TRY(ls_upload(s, (double**)&a.rest_dye, rd.data(), rd.size()));
   }
-  SRS_TRY(dev_alloc(s, &s->d_ls_out, (size_t)s->R * ns));
+  SRS_TRY(ls_alloc(s, &s->d_ls_out, (size_t)s->R * ns));
   a.out = s->d_ls_out;
-  if (linescan_tiled(s, ptr, col)) {
-    SRS_TRY(linescan_tiles(s, ptr, col, w));
-  } else {
-    a.tptr = nullptr;
-    SRS_TRY(linescan_csr(s));
-  }
+  std::vector<int64_t> entries;
+  if (linescan_tiled(s, &entries)) SRS_TRY(linescan_tiles(s, entries));
+  else SRS_TRY(linescan_csr(s));
   if (n_samples) *n_samples = ns;
   return SRS_OK;
 }
@@ -2751,7 +2785,6 @@ int adjoint_setup(srs_sim* s) {
     SRS_TRY(dev_upload(s, &s->d_ryr_s_cl, scl.data(), scl.size()));
     SRS_TRY(dev_upload(s, &s->d_ryr_s_js, sjs.data(), sjs.size()));
   }
-  LinescanBuffers own(s);
   const int ns = s->ls.n_samples;
   std::vector<int32_t> cnt(NE + 1, 0);
   for (size_t q = 0; q < s->ls_col_h.size(); ++q) cnt[s->ls_col_h[q] + 1]++;
@@ -2766,9 +2799,9 @@ int adjoint_setup(srs_sim* s) {
       wv[fill[e]] = s->ls_w_h[q];
       fill[e]++;
     }
-  SRS_TRY(dev_upload(s, &s->d_wt_ptr, cnt.data(), cnt.size()));
-  SRS_TRY(dev_upload(s, &s->d_wt_idx, idx.data(), idx.size()));
-  SRS_TRY(dev_upload(s, &s->d_wt_w, wv.data(), wv.size()));
+  SRS_TRY(ls_upload(s, &s->d_wt_ptr, cnt.data(), cnt.size()));
+  SRS_TRY(ls_upload(s, &s->d_wt_idx, idx.data(), idx.size()));
+  SRS_TRY(ls_upload(s, &s->d_wt_w, wv.data(), wv.size()));
   // the resting part of every sample, pad + sum_q w_q dye_rest(col_q): the
   // tick kernels add the trajectory's dye deviations to it
   std::vector<double> base(ns);
@@ -2780,7 +2813,7 @@ int adjoint_setup(srs_sim* s) {
     }
     base[i] = s->ls_pad_h[i] + acc;
   }
-  SRS_TRY(dev_upload(s, &s->d_ls_base, base.data(), base.size()));
+  SRS_TRY(ls_upload(s, &s->d_ls_base, base.data(), base.size()));
   s->adj_ls_version = s->ls_version;
   return SRS_OK;
 }
