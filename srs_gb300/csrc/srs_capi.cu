@@ -3592,7 +3592,7 @@ int srs_sim_total_ca(srs_sim* s, double* out) {
   }
   SRS_CUDA(cudaStreamSynchronize(s->st));
   if (launch_total_ca(m, s->R, s->mass_blocks, s->st)) return fail(SRS_ERR_CUDA, "total-Ca launch failed");
-  s->launches += 2;
+  s->launches += s->mass_blocks > 1 ? 2 : 1;
   SRS_CUDA(cudaMemcpyAsync(out, m.out, sizeof(double) * 2 * s->R, cudaMemcpyDeviceToHost, s->st));
   SRS_CUDA(cudaStreamSynchronize(s->st));
   return check_timeout(s);
