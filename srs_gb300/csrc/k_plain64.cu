@@ -85,6 +85,8 @@ __device__ __forceinline__ void plain64_tail(const Plain64Args& a, int r, const 
   }
 }
 
+// One thread per element.  64-thread blocks: with 256 the last wave is longer (115,000
+// elements of 300 realizations 53 us a step, 39 so; 236,000 of eight 76 and 72).
 __global__ void __launch_bounds__(256) k_plain64_step(Plain64Args a) {
   pdl_wait();
   pdl_next();
@@ -298,23 +300,25 @@ void plain64_consts(Plain64Args* a) {
 // Tiles of 32 elements up to which the update is dealt to four warps: six blocks
 // per SM.  Beyond, the FP64 pipes are busy anyway and a thread per element
 // avoids passing values between warps.
-static bool split64(const Plain64Args& a) { return (int64_t)((a.N + 31) / 32) * a.R <= 6 * 152; }
-
-static void launch_step64(const Plain64Args& a, cudaStream_t st) {
-  // few realizations: 64-thread blocks spread the element updates (and their
-  // FP64 arithmetic) over more SMs than 256-thread blocks would
-  const int bs = (size_t)((a.N + 255) / 256) * a.R < 304 ? 64 : 256;
-  launch_pdl(k_plain64_step, dim3((a.N + bs - 1) / bs, a.R), bs, 0, st, a);
+static bool small64(const Plain64Args& a) { return (int64_t)((a.N + 31) / 32) * a.R <= 6 * 152; }
+// Dealt to four warps also where the blocks of a thread per element would be a full
+// wave (six of 64 threads per SM) and a small part of another: 62,000 elements take
+// 27.4 us a step so and 39.5 by a thread each, 92,000 35.0 and 39.7, but 104,000 38.8
+// and 40.3, 300 realizations of 384 46.2 and 39.4, 311,000 96.7 and 93.8.
+static bool split64(const Plain64Args& a) {
+  const int64_t blocks = (int64_t)((a.N + 63) / 64) * a.R;
+  return small64(a) || (blocks > 6 * 152 && blocks <= 1600);
 }
 
 int launch_plain64_step(const Plain64Args& a, cudaStream_t st) {
   if (split64(a))
     launch_pdl(k_plain64_split<false>, dim3((a.N + 31) / 32, a.R), 128, 0, st, a, Plain64Keys<false>{});
-  else launch_step64(a, st);
+  else
+    launch_pdl(k_plain64_step, dim3((a.N + 63) / 64, a.R), 64, 0, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-bool plain64_keys_fit(const Plain64Args& a) { return split64(a); }
+bool plain64_keys_fit(const Plain64Args& a) { return small64(a); }
 int launch_plain64_keys(const Plain64Args& a, const Plain64Keys<true>& k, cudaStream_t st) {
   cudaError_t e = launch_pdl(k_plain64_split<true>, dim3((a.N + 31) / 32, a.R), 128, 0, st, a, k);
   if (e == cudaSuccess && !a.P.nogating) e = launch_pdl(k_plain64_gate, a.R, 128, 0, st, a, k);
